@@ -356,15 +356,22 @@ constexpr size_t kPackedSmem = sizeof(PackedTables) + 5 * sizeof(AggEntry);
 constexpr size_t kTabSmem = ((size_t)kAggInts * 4 > kPackedSmem ? (size_t)kAggInts * 4 : kPackedSmem + 15) / 16 * 16;
 constexpr size_t kPairSmem = kTabSmem + (size_t)kTile * kColAccStride * 4;
 
-// copies the run's tables into the block's shared memory (all threads; the caller synchronises)
-__device__ __forceinline__ void load_pair_tables(const PairTables *g, unsigned char *smem, bool packed)
+// copies the run's tables into the block's shared memory (all threads; the caller synchronises); the AVERAGE sums
+// only when the run has a -g test that may need them
+__device__ __forceinline__ void load_pair_tables(const PairTables *g, unsigned char *smem, bool packed, bool fallback)
 {
   if (packed) {
-    const int n0 = (int)(sizeof(PackedTables) / 16), n1 = (int)(5 * sizeof(AggEntry) / 16);
+    const int n0 = (int)((fallback ? sizeof(PackedTables) : offsetof(PackedTables, avg)) / 16);
+    const int n1 = (int)(5 * sizeof(AggEntry) / 16), at1 = (int)(sizeof(PackedTables) / 16);
     const uint4 *src = reinterpret_cast<const uint4 *>(&g->packed);
     const uint4 *src2 = reinterpret_cast<const uint4 *>(&g->agg[kEvEntries]);
     uint4 *dst = reinterpret_cast<uint4 *>(smem);
-    for (int t = threadIdx.x; t < n0 + n1; t += blockDim.x) dst[t] = t < n0 ? src[t] : src2[t - n0];
+    for (int t = threadIdx.x; t < n0 + n1; t += blockDim.x) {
+      if (t < n0)
+        dst[t] = src[t];
+      else
+        dst[at1 + t - n0] = src2[t - n0];
+    }
   } else {
     const uint4 *src = reinterpret_cast<const uint4 *>(g->agg);
     uint4 *dst = reinterpret_cast<uint4 *>(smem);
@@ -400,14 +407,67 @@ __device__ __forceinline__ void store_final(const PairArgs &a, size_t at, const 
   }
 }
 
+// What AVERAGE mode adds to the x16 event sums of one pair (PackedTables::avg words) that the -g test sends there: the
+// events of sequence i against the codes of j, then those of j where i is not a sparse code itself (such a site is
+// counted once, from i's side). Each calling lane walks its own pair's two lists, a dozen to a few hundred table reads,
+// where the site-order walk of the replay kernel visits every word of the alignment with a whole warp. Out of line: few
+// lanes of an ordinary run come here, and its registers stay out of the caller's (the run's arrays come as scalars,
+// since a reference would put the kernel's parameters on every thread's stack).
+__device__ __noinline__ uint4 avg_events(const uint32_t (*tab)[4], bool wplane, const uint32_t *ev_off,
+                                         const uint32_t *ev, const uint8_t *ccT, long Np, int i, int j)
+{
+  uint4 s = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll 1
+  for (int side = 0; side < 2; side++) {
+    const int own = side ? j : i, other = side ? i : j;
+    const uint32_t e1 = ev_off[own + 1];
+    for (uint32_t e = ev_off[own]; e < e1; e++) {
+      const uint32_t v = __ldg(ev + e);
+      const int pc = __ldg(ccT + (size_t)(v >> 5) * Np + other);
+      if (side && sparse_code(pc, wplane)) continue;
+      const uint4 t = *reinterpret_cast<const uint4 *>(tab[((v & 31) - 4) * kCodes + pc]);
+      s.x += t.x;
+      s.y += t.y;
+      s.z += t.z;
+      s.w += t.w;
+    }
+  }
+  return s;
+}
+
+// the same with the unpacked table (a sequence with more than kPackedMaxEvents events): lane q of 0..6
+__device__ __noinline__ int avg_events_lane(const AggEntry *tab, bool wplane, const uint32_t *ev_off,
+                                            const uint32_t *ev, const uint8_t *ccT, long Np, int i, int j, int q)
+{
+  int s = 0;
+#pragma unroll 1
+  for (int side = 0; side < 2; side++) {
+    const int own = side ? j : i, other = side ? i : j;
+    const uint32_t e1 = ev_off[own + 1];
+    for (uint32_t e = ev_off[own]; e < e1; e++) {
+      const uint32_t v = __ldg(ev + e);
+      const int pc = __ldg(ccT + (size_t)(v >> 5) * Np + other);
+      if (side && sparse_code(pc, wplane)) continue;
+      const int32_t *t = tab[((v & 31) - 4) * kCodes + pc].v;
+      s += t[9 + q] - t[q];
+    }
+  }
+  return s;
+}
+
+// the signed low and high 16-bit lanes of a word of sums
+__device__ __forceinline__ int lane_lo(uint32_t w) { return (int)(int16_t)(w & 0xFFFFu); }
+__device__ __forceinline__ int lane_hi(uint32_t w) { return (int)(w - (uint32_t)lane_lo(w)) >> 16; }
+
 // the per-pair epilogue: exact x16 aggregates, tn93's -l / -g / order decisions, formula, certificate (SPLIT: the
-// aggregates go back into the pair's tensor-core record at, and formula_kernel runs the formula)
-template <bool WPLANE, bool SPLIT>
+// aggregates go back into the pair's tensor-core record at, and formula_kernel runs the formula; AVG: the -g test's
+// AVERAGE pairs are finished here)
+template <bool WPLANE, bool SPLIT, bool AVG>
 // cl: the clean-site aggregates of the pair (jointly clean sites, matches, A<->G and C<->T transitions, A, C and G
 // base counts over both sequences), from the popcount loop or the tensor-core count kernel; c: N-plane counts
-__device__ __forceinline__ void pair_epilogue(const PairArgs &a, const AggEntry *EW, const Counts &c, const int cl[7],
-                                              const int acc[9], long i, long j, size_t at, int &namb, int &nund,
-                                              AmbLane &al)
+__device__ __forceinline__ void pair_epilogue(const PairArgs &a, const unsigned char *smem, const AggEntry *EW,
+                                              const Counts &c, const int cl[7], const int acc[9], long i, long j,
+                                              size_t at, int &namb, int &nund, AmbLane &al)
 {
   const RunConsts &rc = a.rc;
   const int base[7] = {16 * (cl[0] + (int)rc.constT), 16 * (cl[1] + (int)rc.constT), 16 * cl[2], 16 * cl[3],
@@ -436,13 +496,45 @@ __device__ __forceinline__ void pair_epilogue(const PairArgs &a, const AggEntry 
   if (acc[8] & 1) {
     to_replay = true;  // order-dependent float sums in the main mode
   } else {
-    const double tng = (double)ag[0] / 16.0;
-    if (tng <= (double)rc.min_overlap) {
+    double tng = (double)ag[0] / 16.0;
+    if (tng > (double)rc.min_overlap && rc.fallback_avg && tng * rc.resolve_fraction <= (double)amb) {
+      // tn93 recomputes the pair with -a average (refkernel.cpp:742-750): with the AVERAGE sums, exact in any order
+      // when they are multiples of 1/16, or else by the site-order path. Only with the N plane on: N runs are what
+      // sends most pairs of a set here (2,000 x 29,900, 1.2 M of 2 M pairs past -g 0.05: 224 ms a run with the walk,
+      // 9.7 ms so); without it few pairs come, and the code costs the kernel at 64 registers more than they do
+      // (6,700 x 1,500: 5.30 ms a run with it, 5.15 ms without).
+      if (!AVG || (acc[8] & 2)) {
+        to_replay = true;
+        qentry = 1ull << 63;
+      } else {
+        if (rc.packed) {
+          const uint4 d = avg_events(reinterpret_cast<const PackedTables *>(smem)->avg, rc.wplane, a.ev_off, a.ev, a.ccT,
+                                     rc.Npad, (int)i, (int)j);
+          ag[0] += lane_lo(d.x);
+          ag[1] += lane_hi(d.x);
+          ag[2] += lane_lo(d.y);
+          ag[3] += lane_hi(d.y);
+          ag[4] += lane_lo(d.z);
+          ag[5] += lane_hi(d.z);
+          ag[6] += (int)d.w;
+        } else {
+          for (int q = 0; q < 7; q++)
+            ag[q] += avg_events_lane(reinterpret_cast<const AggEntry *>(smem), rc.wplane, a.ev_off, a.ev, a.ccT, rc.Npad,
+                                     (int)i, (int)j, q);
+        }
+        if (WPLANE) {
+#pragma unroll
+          for (int q = 0; q < 7; q++)
+            ag[q] += wb[0] * (EW[0].v[9 + q] - EW[0].v[q]) + wb[1] * (EW[1].v[9 + q] - EW[1].v[q]) +
+                     wb[2] * (EW[2].v[9 + q] - EW[2].v[q]) + wb[3] * (EW[3].v[9 + q] - EW[3].v[q]) +
+                     nww * (EW[4].v[9 + q] - EW[4].v[q]);
+        }
+        tng = (double)ag[0] / 16.0;
+      }
+    }
+    if (to_replay) {
+    } else if (tng <= (double)rc.min_overlap) {
       *slot = __longlong_as_double((long long)kSkipBits);
-    } else if (rc.fallback_avg && tng * rc.resolve_fraction <= (double)amb) {
-      // tn93 recomputes the pair with -a average (refkernel.cpp:742-750): the site-order path does that exactly
-      to_replay = true;
-      qentry = 1ull << 63;
     } else if (SPLIT) {
       formula = true;
     } else {
@@ -714,7 +806,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs &a, const unsigned char
       cl[5] = nfC;
       cl[6] = nfG;
     }
-    if (valid) pair_epilogue<WPLANE, SPLIT>(a, EW, c, cl, acc, i, j, at, namb, nund, al);
+    if (valid) pair_epilogue<WPLANE, SPLIT, WPLANE && !GAPMM>(a, smem, EW, c, cl, acc, i, j, at, namb, nund, al);
   }
   if (!SPLIT) {
     count_flags(a.counters, namb, nund);
@@ -730,7 +822,7 @@ __global__ void __launch_bounds__(256, MINB) pair_kernel(PairArgs a)
   const long i0 = a.r0 + blockIdx.y * (long)kTile;
   const long j0 = a.cstart + blockIdx.x * (long)kTile;
   if (i0 >= a.r1 || j0 >= a.rc.N || (!a.rc.cross && j0 + kTile - 1 <= i0)) return;
-  load_pair_tables(a.tab, smem_raw, a.rc.packed);
+  load_pair_tables(a.tab, smem_raw, a.rc.packed, WPLANE && a.rc.fallback_avg);
   __syncthreads();
   pair_tile<WPLANE, GAPMM, SPLIT>(a, smem_raw, colacc, i0, j0, kRowsPerWarp);
 }
@@ -818,7 +910,7 @@ __global__ void __launch_bounds__(256, MINB)
       for (int q = threadIdx.x; q < (int)(sizeof(PairArgs) / 4); q += blockDim.x)
         reinterpret_cast<int32_t *>(sd_raw)[q] = reinterpret_cast<const int32_t *>(&descs[T.k])[q];
       __syncthreads();
-      load_pair_tables(sd.tab, smem_raw, sd.rc.packed);
+      load_pair_tables(sd.tab, smem_raw, sd.rc.packed, WPLANE && sd.rc.fallback_avg);
       cur = T.k;
     }
     __syncthreads();

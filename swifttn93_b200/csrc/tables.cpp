@@ -141,7 +141,7 @@ AggEntry make_agg(int c1, int c2, int mode, const unsigned char *subset)
   const bool da = aggregate(S, a);
   for (int k = 0; k < 7; k++) e.v[k] = m[k];
   e.v[7] = m[7];
-  e.v[8] = dm ? 0 : 1;  // counts entries whose main-mode contribution is not a multiple of 1/16
+  e.v[8] = (dm ? 0 : 1) | (da ? 0 : 2);  // contributions that are not a multiple of 1/16 (main mode, AVERAGE)
   for (int k = 0; k < 7; k++) e.v[9 + k] = a[k];
   return e;
 }
@@ -187,6 +187,12 @@ void pack_tables(const Tables &T, bool w_plane, PackedTables *P)
       }
       P->rowf[k] = (uint32_t)v[8];
       P->colf[k] = partner_sparse ? 0u : (uint32_t)v[8];
+      int32_t d[7];
+      for (int q = 0; q < 7; q++) d[q] = v[9 + q] - v[q];
+      P->avg[k][0] = (uint32_t)d[0] + ((uint32_t)d[1] << 16);
+      P->avg[k][1] = (uint32_t)d[2] + ((uint32_t)d[3] << 16);
+      P->avg[k][2] = (uint32_t)d[4] + ((uint32_t)d[5] << 16);
+      P->avg[k][3] = (uint32_t)d[6];
     }
 }
 

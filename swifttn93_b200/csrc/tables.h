@@ -15,8 +15,9 @@ constexpr int kSparseCodes = 13;  // codes 4..16
 // Lanes of an aggregate entry (x16 integers, exact while every contribution is a multiple of 1/16):
 //   0 T (total), 1 D (diagonal), 2 AG (A<->G), 3 CT (C<->T), 4 nfA, 5 nfC, 6 nfG  -- the main mode
 //   7 ambiguity count (resolved events, for the -g test)
-//   8 1 when the main-mode contribution is not a multiple of 1/16 (a pair with any such site takes the
-//     site-order replay)
+//   8 bit 0 when the main-mode contribution is not a multiple of 1/16 (a pair with any such site takes the
+//     site-order replay), bit 1 when the AVERAGE contribution is not (a pair that the -g test sends to AVERAGE then
+//     takes the replay too)
 //   9..15 lanes 0..6 in AVERAGE mode (the -g fallback)
 constexpr int kLanes = 16;
 struct AggEntry {
@@ -49,10 +50,12 @@ void build_tables(Tables *T, int mode, const unsigned char subset[kCodes]);
 
 // The pair kernel's copy of the event table, packed: per (sparse code c of one sequence, code o of the other) the
 // main-mode x16 lanes two to a 32-bit word, w[0] = T | D << 16, w[1] = AG | CT << 16, w[2] = nfA | nfC << 16,
-// w[3] = nfG | amb << 16, and a separate flag word (1: not a multiple of 1/16). No lane of an entry exceeds 32, so
+// w[3] = nfG | amb << 16, and a separate flag word (AggEntry lane 8). No lane of an entry exceeds 32, so
 // packed sums stay exact for fewer than 2048 events per pair; the engine packs when no sequence has more than
 // kPackedMaxEvents events. col[] is row[] with zeros where o is itself a sparse event code (such a site is counted
-// once, from the row's side), so the column side needs no test.
+// once, from the row's side), so the column side needs no test. avg[] holds what AVERAGE mode adds to lanes 0..6
+// (signed differences, two to a word as low + high * 65536; below 16 each, so their sums stay within 16 bits), for the
+// pairs that the -g test sends there; it comes last so that runs without that test need not load it.
 constexpr int kPackedMaxEvents = 1023;
 constexpr int kEvEntries = kSparseCodes * kCodes;
 struct PackedTables {
@@ -60,7 +63,9 @@ struct PackedTables {
   uint32_t col[kEvEntries][4];
   uint32_t rowf[kEvEntries];
   uint32_t colf[kEvEntries];
+  uint32_t avg[kEvEntries][4];
 };
+static_assert(offsetof(PackedTables, avg) % 16 == 0, "the AVERAGE differences are read as 16-byte words");
 void pack_tables(const Tables &T, bool w_plane, PackedTables *P);
 
 // true if code c is a "sparse event" code: not clean, not a gap, and not N when N has its own plane
