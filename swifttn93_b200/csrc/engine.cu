@@ -3081,111 +3081,125 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   else  // pairs (i, j > i) of rows [row_begin, row_end)
     sum->pairwise = (unsigned long)((row_end - row_begin) * (2 * N - row_begin - row_end - 1) / 2);
   // Band schedule. When the text goes to the host, a band holds about 3 M pairs (at most 16 M pair slots), so
-  // that the copy of one band overlaps the kernels of the next; otherwise up to 64 M slots (512 MB of distances).
+  // that the copy of one band overlaps the kernels of the next; otherwise up to 64 M slots.
   const bool stream_text = !(to_device || hyphy || !rc.emit);
-  static const long band_pairs = [] {
+  static const long forced_band = [] {
     const char *e = getenv("TN93G_BAND_PAIRS");  // tuning knob: pairs per band when streaming text
-    return e && atol(e) > 0 ? atol(e) : (3l << 20);
+    return e ? std::max(atol(e), 0l) : 0l;
   }();
-  const long target_pairs = (stream_text || rc.resolve_all) ? band_pairs : (1l << 62);
-  const long cap_slots = (stream_text || rc.resolve_all) ? (16l << 20) : (64l << 20);
+  const long band_pairs = forced_band ? forced_band : (3l << 20);
   // When the text streams to the host, the bands ramp up from 1/16 of the target, 1.4 times larger each (a band's
   // kernels take about 0.7 of its copy's time, so each band's kernels end before the previous band's copy does and
   // the copies run back to back), and taper at the end (half of what is left, down to 1/8), so that the first copy
-  // starts early and the last one, which nothing overlaps, is short.
+  // starts early and the last one, which nothing overlaps, is short. When the first band shows that little is
+  // reported, there is nothing to overlap and the rest runs as large bands (below).
   std::vector<std::pair<long, long>> bands;
-  long maxrows = 1;
-  long left = 0;
-  for (long r = row_begin; r < upper; r++) left += rc.cross ? ncols : (N - r - 1);
-  for (long r0 = row_begin; r0 < upper;) {
-    long tgt = target_pairs;
-    if (stream_text) {
-      const double ramp = std::pow(1.4, (double)bands.size()) / 16.0;
-      if (ramp < 1.0) tgt = std::max<long>(1, (long)((double)target_pairs * ramp));
-      if (left < 2 * target_pairs) tgt = std::min(tgt, std::max(target_pairs / 8, left / 2));
+  auto plan_bands = [&](long from, long target, long cap, bool ramps) {
+    long left = 0;
+    for (long r = from; r < upper; r++) left += rc.cross ? ncols : (N - r - 1);
+    for (long r0 = from; r0 < upper;) {
+      long tgt = target;
+      if (ramps) {
+        const double ramp = std::pow(1.4, (double)bands.size()) / 16.0;
+        if (ramp < 1.0) tgt = std::max<long>(1, (long)((double)target * ramp));
+        if (left < 2 * target) tgt = std::min(tgt, std::max(target / 8, left / 2));
+      }
+      long r = r0, pairs = 0;
+      while (r < upper && (r == r0 || ((r - r0 + 1) * ncols <= cap && pairs < tgt && r - r0 < 65535l * kTile))) {
+        pairs += rc.cross ? ncols : (N - r - 1);
+        r++;
+      }
+      bands.push_back({r0, r});
+      left -= pairs;
+      r0 = r;
     }
-    long r = r0, pairs = 0;
-    while (r < upper && (r == r0 || ((r - r0 + 1) * ncols <= cap_slots && pairs < tgt && r - r0 < 65535l * kTile))) {
-      pairs += rc.cross ? ncols : (N - r - 1);
-      r++;
-    }
-    bands.push_back({r0, r});
-    maxrows = std::max(maxrows, r - r0);
-    left -= pairs;
-    r0 = r;
-  }
-  const long band = maxrows;
+  };
+  constexpr long kBigSlots = 64l << 20;  // pair slots of a band that need not overlap a copy (512 MB of distances)
+  plan_bands(row_begin, (stream_text || rc.resolve_all) ? band_pairs : (1l << 62),
+             (stream_text || rc.resolve_all) ? (16l << 20) : kBigSlots, stream_text);
   const long maxseg = std::max<long>(1, (ncols + kSeg - 1) / kSeg);
-  const long nseg = band * maxseg;  // per band parity
   if (hyphy) {
     TRY(ensure(ctx, ctx->hy, (size_t)N * N * sizeof(double)));
     fill_nan_kernel<<<1024, 256, 0, st>>>((double *)ctx->hy.p, (size_t)N * N);
     CU(cudaGetLastError());
     ctx->launches++;
   }
-  // per band parity (double-buffered): distances, segment statistics, row sums; the replay queue is per band
-  const size_t dslots = (size_t)band * ncols;
-  TRY(ensure(ctx, ctx->dist, 2 * dslots * sizeof(double)));
-  if (rc.emit && !hyphy) TRY(ensure(ctx, ctx->dcode, 2 * dslots * sizeof(uint32_t)));
+  // per band parity (double-buffered): distances, segment statistics, row sums; the replay queue is per band. Sized for
+  // the largest of the bands from the first one on; called again, with nothing in flight, when the schedule changes.
   const int tc16 = 32 * L < 65536;  // the final x16 aggregates fit 16-bit lanes
-  // the tensor-core path's row chunks per band (boundaries on the count kernel's 32-row tiles)
-  std::vector<std::vector<std::pair<long, long>>> band_chunks(bands.size());
-  size_t chunk_slots = 1;
+  long band = 1, nseg = 1;
+  size_t dslots = 1, stat_stride = 0;
+  std::vector<std::vector<std::pair<long, long>>> band_chunks;  // the tensor-core path's row chunks per band
   int nchunks[2] = {0, 0};
-  if (use_tc) {
-    for (size_t b = 0; b < bands.size(); b++) {
-      const long r0 = bands[b].first, r1 = bands[b].second;
-      long bp = 0;
-      for (long r = r0; r < r1; r++) bp += rc.cross ? ncols : (N - r - 1);
-      static const long chunk_pairs = [] {
-        const char *e = getenv("TN93G_TC_CHUNK_PAIRS");  // tuning knob: pairs per count/pair chunk
-        return e && atol(e) > 0 ? atol(e) : kTcChunkPairs;
-      }();
-      const long target = std::max(chunk_pairs, (bp + kMaxTcChunks - 2) / (kMaxTcChunks - 1));
-      for (long c0 = r0; c0 < r1;) {
-        long c1 = c0, pairs = 0;
-        while (c1 < r1 && (c1 == c0 || pairs < target)) {
-          pairs += rc.cross ? ncols : (N - c1 - 1);
-          c1++;
+  unsigned und_cap_par[2] = {0, 0};  // grown per parity when a band lists more
+  char *d_pstats = nullptr;          // the device's address of the statistics' staging
+  auto size_buffers = [&](size_t first) -> int {
+    band = 1;
+    for (size_t b = first; b < bands.size(); b++) band = std::max(band, bands[b].second - bands[b].first);
+    nseg = band * maxseg;
+    dslots = (size_t)band * ncols;
+    TRY(ensure(ctx, ctx->dist, 2 * dslots * sizeof(double)));
+    if (rc.emit && !hyphy) TRY(ensure(ctx, ctx->dcode, 2 * dslots * sizeof(uint32_t)));
+    // chunk boundaries on the count kernel's 32-row tiles
+    band_chunks.assign(bands.size(), {});
+    size_t chunk_slots = 1;
+    if (use_tc) {
+      for (size_t b = first; b < bands.size(); b++) {
+        const long r0 = bands[b].first, r1 = bands[b].second;
+        long bp = 0;
+        for (long r = r0; r < r1; r++) bp += rc.cross ? ncols : (N - r - 1);
+        static const long chunk_pairs = [] {
+          const char *e = getenv("TN93G_TC_CHUNK_PAIRS");  // tuning knob: pairs per count/pair chunk
+          return e && atol(e) > 0 ? atol(e) : kTcChunkPairs;
+        }();
+        const long target = std::max(chunk_pairs, (bp + kMaxTcChunks - 2) / (kMaxTcChunks - 1));
+        for (long c0 = r0; c0 < r1;) {
+          long c1 = c0, pairs = 0;
+          while (c1 < r1 && (c1 == c0 || pairs < target)) {
+            pairs += rc.cross ? ncols : (N - c1 - 1);
+            c1++;
+          }
+          c1 = std::min(r1, (c1 + kTcRows - 1) / kTcRows * kTcRows);
+          if ((int)band_chunks[b].size() == kMaxTcChunks - 1) c1 = r1;  // never more chunks than events
+          band_chunks[b].push_back({c0, c1});
+          chunk_slots = std::max(chunk_slots, (size_t)(c1 - c0) * ncols);
+          c0 = c1;
         }
-        c1 = std::min(r1, (c1 + kTcRows - 1) / kTcRows * kTcRows);
-        if ((int)band_chunks[b].size() == kMaxTcChunks - 1) c1 = r1;  // never more chunks than events
-        band_chunks[b].push_back({c0, c1});
-        chunk_slots = std::max(chunk_slots, (size_t)(c1 - c0) * ncols);
-        c0 = c1;
       }
+      TRY(ensure(ctx, ctx->tcagg, chunk_slots * (tc16 ? 16 : 32)));
     }
-    TRY(ensure(ctx, ctx->tcagg, chunk_slots * (tc16 ? 16 : 32)));
-  }
-  TRY(ensure(ctx, ctx->rq, dslots * sizeof(unsigned long long)));
+    TRY(ensure(ctx, ctx->rq, dslots * sizeof(unsigned long long)));
+    TRY(ensure(ctx, ctx->rbytes, 2 * nseg * sizeof(unsigned long long)));
+    TRY(ensure(ctx, ctx->roff, 2 * nseg * sizeof(unsigned long long)));
+    TRY(ensure(ctx, ctx->rsum, 2 * band * 3 * sizeof(double)));
+    TRY(ensure(ctx, ctx->rw, 2 * band * 3 * sizeof(double)));
+    TRY(ensure(ctx, ctx->rmax, 2 * nseg * 3 * sizeof(double)));
+    TRY(ensure(ctx, ctx->rlinks, 2 * nseg * sizeof(long long)));
+    TRY(ensure(ctx, ctx->rskip, 2 * nseg * sizeof(long long)));
+    const unsigned und_cap = (unsigned)std::min<size_t>(rc.resolve_all ? dslots : std::max<size_t>(4096, dslots / 64),
+                                                        0xFFFFFFF0u);
+    for (int q = 0; q < 2; q++) {
+      TRY(ensure(ctx, ctx->und[q], (size_t)und_cap * 2 * sizeof(unsigned long long)));
+      und_cap_par[q] = und_cap;
+    }
+    // pinned staging of a band's statistics: row sums and weights (3 each), segment maxima (3 each), segment links
+    // and skips, total bytes, the band's histogram, its undecided count and the count kernel's error word
+    stat_stride = (size_t)band * 6 * sizeof(double) + (size_t)nseg * (3 * sizeof(double) + 2 * sizeof(long long)) +
+                  (3 + 3 * kHistBins) * sizeof(unsigned long long);
+    TRY(ensure_pinned_at(ctx, ctx->pstats, ctx->pstats_n, 2 * stat_stride, cudaHostAllocMapped));
+    CU(cudaHostGetDevicePointer((void **)&d_pstats, ctx->pstats, 0));
+    return TN93G_OK;
+  };
+  TRY(size_buffers(0));
   TRY(ensure(ctx, ctx->rqn, sizeof(unsigned)));
   TRY(ensure(ctx, ctx->counters, 4 * sizeof(unsigned long long)));
-  TRY(ensure(ctx, ctx->rbytes, 2 * nseg * sizeof(unsigned long long)));
-  TRY(ensure(ctx, ctx->roff, 2 * nseg * sizeof(unsigned long long)));
-  TRY(ensure(ctx, ctx->rsum, 2 * band * 3 * sizeof(double)));
-  TRY(ensure(ctx, ctx->rw, 2 * band * 3 * sizeof(double)));
-  TRY(ensure(ctx, ctx->rmax, 2 * nseg * 3 * sizeof(double)));
-  TRY(ensure(ctx, ctx->rlinks, 2 * nseg * sizeof(long long)));
-  TRY(ensure(ctx, ctx->rskip, 2 * nseg * sizeof(long long)));
   // per band parity: its histogram (added on the host, so a band's row stage can run again), its undecided list
   TRY(ensure(ctx, ctx->hist, 2 * 3 * kHistBins * sizeof(unsigned long long)));
   TRY(ensure(ctx, ctx->total, 2 * sizeof(unsigned long long)));
-  const unsigned und_cap = (unsigned)std::min<size_t>(rc.resolve_all ? dslots : std::max<size_t>(4096, dslots / 64),
-                                                      0xFFFFFFF0u);
-  for (int q = 0; q < 2; q++) TRY(ensure(ctx, ctx->und[q], (size_t)und_cap * 2 * sizeof(unsigned long long)));
-  unsigned und_cap_par[2] = {und_cap, und_cap};  // grown per parity when a band lists more
   TRY(ensure(ctx, ctx->undn, 2 * sizeof(unsigned long long)));
   TRY(ensure(ctx, ctx->amb, 3 * 4 * sizeof(unsigned long long)));
   TRY(ensure(ctx, ctx->rdesc, 2 * sizeof(ReplayArgs)));
   CU(cudaMemsetAsync(ctx->amb.p, 0, 3 * 4 * sizeof(unsigned long long), st));
-  // pinned staging of a band's statistics: row sums and weights (3 each), segment maxima (3 each), segment links
-  // and skips, total bytes, the band's histogram, its undecided count and the count kernel's error word
-  const size_t stat_stride = (size_t)band * 6 * sizeof(double) +
-                             (size_t)nseg * (3 * sizeof(double) + 2 * sizeof(long long)) +
-                             (3 + 3 * kHistBins) * sizeof(unsigned long long);
-  TRY(ensure_pinned_at(ctx, ctx->pstats, ctx->pstats_n, 2 * stat_stride, cudaHostAllocMapped));
-  char *d_pstats = nullptr;  // the device's address of the staging
-  CU(cudaHostGetDevicePointer((void **)&d_pstats, ctx->pstats, 0));
   CU(cudaMemsetAsync(ctx->counters.p, 0, 4 * sizeof(unsigned long long), st));
   double max_[3] = {0, 0, 0}, mean[3] = {0, 0, 0}, wc[3] = {0, 0, 0};
   unsigned long long hist_total[3 * kHistBins];
@@ -3442,6 +3456,11 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     if (sink && sink(user, (const char *)ctx->pin2[q], pend_bytes[q])) return TN93G_ESINK;
     return TN93G_OK;
   };
+  auto band_pair_count = [&](int bi) -> long {
+    long p = 0;
+    for (long r = bands[bi].first; r < bands[bi].second; r++) p += rc.cross ? ncols : (N - r - 1);
+    return p;
+  };
   // statistics of band bi in row order, then its text: written on the compute stream (behind the next band's
   // kernels) and copied to the host on the copy stream
   auto finish = [&](int bi) -> int {
@@ -3566,10 +3585,35 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   // Band bi + 1's kernels are queued before band bi is finished, so the device computes while the host takes band
   // bi's statistics; texts reach the sink when their pinned buffer is needed again, or at the end (at most one band
   // per parity waits).
-  const int nb = (int)bands.size();
+  // A streamed run that reports few pairs (the first band gives less than 2 bytes of text a pair, so copying a band takes
+  // less than a sixth of computing it) has nothing to overlap: what is left after the second band runs as large bands,
+  // whose kernels fill the GPU (each kernel's last wave, the row sums' chains and the replays cost a band about as much
+  // whatever its size: 6,700 x 1,500 at -t 0.015 took 17 bands and 7.2 ms of device time, 4.9 ms so). If the larger
+  // buffers do not fit, the small bands go on.
+  const bool may_grow = stream_text && !rc.resolve_all && !forced_band;
+  int nb = (int)bands.size();
   for (int bi = 0; bi <= nb; bi++) {
     if (bi < nb) TRY(enqueue_compute(bi));
     if (bi >= 1) TRY(finish(bi - 1));
+    if (bi == 1 && may_grow && nb > 3 && sum->output_bytes < 2 * (size_t)band_pair_count(0)) {
+      TRY(finish(1));
+      while (pend_n) TRY(deliver_oldest());
+      const std::vector<std::pair<long, long>> small = bands;
+      bands.resize(2);
+      plan_bands(small[2].first, 1l << 62, kBigSlots, false);
+      const int grown = size_buffers(2);
+      if (grown == TN93G_ENOMEM) {
+        ctx->err.clear();
+        cudaGetLastError();
+        bands = small;
+        TRY(size_buffers(2));
+      } else {
+        TRY(grown);
+      }
+      nb = (int)bands.size();
+      bi = 2;
+      TRY(enqueue_compute(2));
+    }
   }
   while (pend_n) TRY(deliver_oldest());
   if (hyphy) {
