@@ -136,6 +136,12 @@ __global__ void wlist_kernel(const uint64_t *planes, long N, long W, int NP, lon
     if (planes[((size_t)w * NP + 3) * Npad + i] != 0) wl[o++] = (uint32_t)w;
 }
 
+__device__ __forceinline__ void put_event(const PackArgs &a, uint32_t at, uint32_t k, int c)
+{
+  a.ev[at] = k << 5 | (uint32_t)c;
+  if (a.ev2) a.ev2[at] = make_uint2(k * a.ev2_Npad, (uint32_t)(c - kSparse0) * (kCodes * 8));
+}
+
 // one warp per sequence: its sparse events in site order (block bx: 8 sequences)
 __device__ __forceinline__ void events_body(const PackArgs &a, long bx)
 {
@@ -144,14 +150,22 @@ __device__ __forceinline__ void events_body(const PackArgs &a, long bx)
   if (i >= a.N) return;
   uint32_t off = a.ev_off[i];
   const uint8_t *row = a.cc + i * a.Lc;
+  bool three = false;
   for (long w = 0; w < a.W; w++) {
     const long k0 = w * 64 + lane, k1 = k0 + 32;
     const int c0 = k0 < a.Lc ? row[k0] : 17, c1 = k1 < a.Lc ? row[k1] : 17;
     const bool s0 = sparse_code(c0, a.wplane), s1 = sparse_code(c1, a.wplane);
     const unsigned b0 = __ballot_sync(0xffffffffu, s0), b1 = __ballot_sync(0xffffffffu, s1);
-    if (s0) a.ev[off + __popc(b0 & lanemask_lt())] = ((uint32_t)k0 << 5) | (uint32_t)c0;
-    if (s1) a.ev[off + __popc(b0) + __popc(b1 & lanemask_lt())] = ((uint32_t)k1 << 5) | (uint32_t)c1;
+    if (s0) put_event(a, off + __popc(b0 & lanemask_lt()), (uint32_t)k0, c0);
+    if (s1) put_event(a, off + __popc(b0) + __popc(b1 & lanemask_lt()), (uint32_t)k1, c1);
     off += __popc(b0) + __popc(b1);
+    three |= (c0 >= 11 && c0 <= 14) || (c1 >= 11 && c1 <= 14);
+  }
+  // null events (no site, the tables' zero row) up to the list's padded end
+  if (lane < (int)(a.ev_off[i + 1] - off)) put_event(a, off + lane, 0, kGap);
+  if (a.three) {
+    three = __any_sync(0xffffffffu, three);
+    if (lane == 0) a.three[i] = three;
   }
 }
 
@@ -391,22 +405,6 @@ struct Counts {
   int nWc, nWh, nWl, nWt, nWW, nGG;
 };
 
-// The final aggregates of a pair for formula_kernel, written over its tensor-core record at: ag[0..6] and a state
-// lane (0: the formula kernel finishes the pair; 1: finished here, skipped or queued for the site-order replay)
-__device__ __forceinline__ void store_final(const PairArgs &a, size_t at, const int ag[7], bool formula)
-{
-  const uint32_t st = formula ? 0u : 1u;
-  if (a.tc16) {
-    reinterpret_cast<uint4 *>(a.tcagg)[at] =
-        make_uint4((uint32_t)ag[0] | (uint32_t)ag[1] << 16, (uint32_t)ag[2] | (uint32_t)ag[3] << 16,
-                   (uint32_t)ag[4] | (uint32_t)ag[5] << 16, (uint32_t)ag[6] | st << 16);
-  } else {
-    uint4 *d = reinterpret_cast<uint4 *>(a.tcagg) + 2 * at;
-    d[0] = make_uint4((uint32_t)ag[0], (uint32_t)ag[1], (uint32_t)ag[2], (uint32_t)ag[3]);
-    d[1] = make_uint4((uint32_t)ag[4], (uint32_t)ag[5], (uint32_t)ag[6], st);
-  }
-}
-
 // What AVERAGE mode adds to the x16 event sums of one pair (PackedTables::avg words) that the -g test sends there: the
 // events of sequence i against the codes of j, then those of j where i is not a sparse code itself (such a site is
 // counted once, from i's side). Each calling lane walks its own pair's two lists, a dozen to a few hundred table reads,
@@ -459,15 +457,14 @@ __device__ __noinline__ int avg_events_lane(const AggEntry *tab, bool wplane, co
 __device__ __forceinline__ int lane_lo(uint32_t w) { return (int)(int16_t)(w & 0xFFFFu); }
 __device__ __forceinline__ int lane_hi(uint32_t w) { return (int)(w - (uint32_t)lane_lo(w)) >> 16; }
 
-// the per-pair epilogue: exact x16 aggregates, tn93's -l / -g / order decisions, formula, certificate (SPLIT: the
-// aggregates go back into the pair's tensor-core record at, and formula_kernel runs the formula; AVG: the -g test's
+// the per-pair epilogue: exact x16 aggregates, tn93's -l / -g / order decisions, formula, certificate (AVG: the -g test's
 // AVERAGE pairs are finished here)
-template <bool WPLANE, bool SPLIT, bool AVG>
+template <bool WPLANE, bool AVG>
 // cl: the clean-site aggregates of the pair (jointly clean sites, matches, A<->G and C<->T transitions, A, C and G
 // base counts over both sequences), from the popcount loop or the tensor-core count kernel; c: N-plane counts
 __device__ __forceinline__ void pair_epilogue(const PairArgs &a, const unsigned char *smem, const AggEntry *EW,
                                               const Counts &c, const int cl[7], const int acc[9], long i, long j,
-                                              size_t at, int &namb, int &nund, AmbLane &al)
+                                              int &namb, int &nund, AmbLane &al)
 {
   const RunConsts &rc = a.rc;
   const int base[7] = {16 * (cl[0] + (int)rc.constT), 16 * (cl[1] + (int)rc.constT), 16 * cl[2], 16 * cl[3],
@@ -492,7 +489,7 @@ __device__ __forceinline__ void pair_epilogue(const PairArgs &a, const unsigned 
   if (WPLANE) amb += wb[0] * EW[0].v[7] + wb[1] * EW[1].v[7] + wb[2] * EW[2].v[7] + wb[3] * EW[3].v[7] + nww * EW[4].v[7];
   double *slot = a.dist + (size_t)(i - a.r0) * a.ncols + (j - a.colbase);
   unsigned long long qentry = 0;
-  bool to_replay = false, formula = false;
+  bool to_replay = false;
   if (acc[8] & 1) {
     to_replay = true;  // order-dependent float sums in the main mode
   } else {
@@ -535,8 +532,6 @@ __device__ __forceinline__ void pair_epilogue(const PairArgs &a, const unsigned 
     if (to_replay) {
     } else if (tng <= (double)rc.min_overlap) {
       *slot = __longlong_as_double((long long)kSkipBits);
-    } else if (SPLIT) {
-      formula = true;
     } else {
       const double nf[4] = {(double)ag[4] / 16.0, (double)ag[5] / 16.0, (double)ag[6] / 16.0,
                             (double)(2 * ag[0] - ag[4] - ag[5] - ag[6]) / 16.0};
@@ -544,7 +539,6 @@ __device__ __forceinline__ void pair_epilogue(const PairArgs &a, const unsigned 
                            j, a.colbase, namb, nund, al);
     }
   }
-  if (SPLIT) store_final(a, at, ag, formula);
   if (to_replay) {
     const unsigned idx = atomicAdd(a.replay_n, 1u);
     if (idx < a.replay_cap) a.replay_q[idx] = qentry | ((unsigned long long)i << 31) | (unsigned long long)j;
@@ -605,7 +599,7 @@ __device__ __forceinline__ void add_events(PackedAcc &p, const uint32_t (*tab)[4
 
 // One tile of pairs: rows [i0, i0 + 8 * rpw) (rpw = rows per warp, 1..4) x columns [j0, j0 + 32). The block's
 // tables must be in smem (load_pair_tables). All threads of the block call it with the same arguments.
-template <bool WPLANE, bool GAPMM, bool SPLIT>
+template <bool WPLANE, bool GAPMM>
 __device__ __forceinline__ void pair_tile(const PairArgs &a, const unsigned char *smem, int *colacc, long i0, long j0,
                                           int rpw)
 {
@@ -765,14 +759,13 @@ __device__ __forceinline__ void pair_tile(const PairArgs &a, const unsigned char
       }
     }
     int cl[7];
-    size_t at = 0;
     if (tc) {
-      // the pair's record from the tensor-core kernel (8 lanes, 7 used); plain loads when SPLIT writes it back
+      // the pair's record from the tensor-core kernel (8 lanes, 7 used)
       const long tn = a.tcncols ? a.tcncols : a.ncols, tb = a.tcncols ? a.tccolbase : a.colbase;
-      at = (size_t)(i - a.r0) * tn + (jj - tb);
+      const size_t at = (size_t)(i - a.r0) * tn + (jj - tb);
       if (a.tc16) {
         const uint4 *gp = reinterpret_cast<const uint4 *>(a.tcagg) + at;
-        const uint4 g = valid ? (SPLIT ? *gp : __ldg(gp)) : make_uint4(0, 0, 0, 0);
+        const uint4 g = valid ? __ldg(gp) : make_uint4(0, 0, 0, 0);
         cl[0] = (int)(g.x & 0xFFFFu);
         cl[1] = (int)(g.x >> 16);
         cl[2] = (int)(g.y & 0xFFFFu);
@@ -782,8 +775,8 @@ __device__ __forceinline__ void pair_tile(const PairArgs &a, const unsigned char
         cl[6] = (int)(g.w & 0xFFFFu);
       } else {
         const uint4 *g = reinterpret_cast<const uint4 *>(a.tcagg) + 2 * at;
-        const uint4 g0 = valid ? (SPLIT ? g[0] : __ldg(g)) : make_uint4(0, 0, 0, 0);
-        const uint4 g1 = valid ? (SPLIT ? g[1] : __ldg(g + 1)) : make_uint4(0, 0, 0, 0);
+        const uint4 g0 = valid ? __ldg(g) : make_uint4(0, 0, 0, 0);
+        const uint4 g1 = valid ? __ldg(g + 1) : make_uint4(0, 0, 0, 0);
         cl[0] = (int)g0.x;
         cl[1] = (int)g0.y;
         cl[2] = (int)g0.z;
@@ -792,10 +785,8 @@ __device__ __forceinline__ void pair_tile(const PairArgs &a, const unsigned char
         cl[5] = (int)g1.y;
         cl[6] = (int)g1.z;
       }
-      // the records are read once; the split form's formula kernel reads them again
-      if (!SPLIT)
-        discard_records(a.tcagg, (size_t)(i - a.r0) * tn + (size_t)(j0 - tb), min((long)kTile, tb + tn - j0),
-                        a.tc16 ? 16 : 32, lane);
+      discard_records(a.tcagg, (size_t)(i - a.r0) * tn + (size_t)(j0 - tb), min((long)kTile, tb + tn - j0),
+                      a.tc16 ? 16 : 32, lane);
     } else {
       const int nfT = c.T1 + c.T2, nfC = c.Y1 + c.Y2 - nfT, nfG = c.L1 + c.L2 - nfT;
       cl[0] = c.T;
@@ -806,15 +797,13 @@ __device__ __forceinline__ void pair_tile(const PairArgs &a, const unsigned char
       cl[5] = nfC;
       cl[6] = nfG;
     }
-    if (valid) pair_epilogue<WPLANE, SPLIT, WPLANE && !GAPMM>(a, smem, EW, c, cl, acc, i, j, at, namb, nund, al);
+    if (valid) pair_epilogue<WPLANE, WPLANE && !GAPMM>(a, smem, EW, c, cl, acc, i, j, namb, nund, al);
   }
-  if (!SPLIT) {
-    count_flags(a.counters, namb, nund);
-    if (a.ex.amb) amb_warp_flush(a.ex.amb, al);
-  }
+  count_flags(a.counters, namb, nund);
+  if (a.ex.amb) amb_warp_flush(a.ex.amb, al);
 }
 
-template <bool WPLANE, bool GAPMM, int MINB, bool SPLIT>
+template <bool WPLANE, bool GAPMM, int MINB>
 __global__ void __launch_bounds__(256, MINB) pair_kernel(PairArgs a)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -824,60 +813,14 @@ __global__ void __launch_bounds__(256, MINB) pair_kernel(PairArgs a)
   if (i0 >= a.r1 || j0 >= a.rc.N || (!a.rc.cross && j0 + kTile - 1 <= i0)) return;
   load_pair_tables(a.tab, smem_raw, a.rc.packed, WPLANE && a.rc.fallback_avg);
   __syncthreads();
-  pair_tile<WPLANE, GAPMM, SPLIT>(a, smem_raw, colacc, i0, j0, kRowsPerWarp);
+  pair_tile<WPLANE, GAPMM>(a, smem_raw, colacc, i0, j0, kRowsPerWarp);
 }
 
-// The formula for the pairs of one split pair-kernel launch (rows [r0, r1), columns [cstart, cstart + ncol)): one
-// thread per pair slot, lanes along a row's columns, reading the final aggregates the pair kernel left in the
-// pair's tensor-core record (state 0) and writing the distance. No shared memory; the registers of the formula
-// alone decide the occupancy (MINB resident blocks per SM).
-template <bool REC16, int MINB>
-__global__ void __launch_bounds__(256, MINB) formula_kernel(PairArgs a, long ncol)
-{
-  const RunConsts &rc = a.rc;
-  const long tn = a.tcncols ? a.tcncols : a.ncols, tb = a.tcncols ? a.tccolbase : a.colbase;
-  const long j = a.cstart + blockIdx.x * 256l + threadIdx.x;
-  int namb = 0, nund = 0;
-  AmbLane al;
-  al.unit = -1;
-  for (long i = a.r0 + blockIdx.y; i < a.r1; i += gridDim.y) {
-    const long lb = rc.cross ? rc.n1 : i + 1;
-    if (j < lb || j >= rc.N || j >= a.cstart + ncol) continue;
-    const size_t at = (size_t)(i - a.r0) * tn + (j - tb);
-    int ag[7];
-    uint32_t st;
-    if (REC16) {
-      const uint4 g = reinterpret_cast<const uint4 *>(a.tcagg)[at];
-      ag[0] = (int)(g.x & 0xFFFFu);
-      ag[1] = (int)(g.x >> 16);
-      ag[2] = (int)(g.y & 0xFFFFu);
-      ag[3] = (int)(g.y >> 16);
-      ag[4] = (int)(g.z & 0xFFFFu);
-      ag[5] = (int)(g.z >> 16);
-      ag[6] = (int)(g.w & 0xFFFFu);
-      st = g.w >> 16;
-    } else {
-      const uint4 *g = reinterpret_cast<const uint4 *>(a.tcagg) + 2 * at;
-      const uint4 g0 = g[0], g1 = g[1];
-      ag[0] = (int)g0.x;
-      ag[1] = (int)g0.y;
-      ag[2] = (int)g0.z;
-      ag[3] = (int)g0.w;
-      ag[4] = (int)g1.x;
-      ag[5] = (int)g1.y;
-      ag[6] = (int)g1.z;
-      st = g1.w;
-    }
-    if (st) continue;
-    const double nf[4] = {(double)ag[4] / 16.0, (double)ag[5] / 16.0, (double)ag[6] / 16.0,
-                          (double)(2 * ag[0] - ag[4] - ag[5] - ag[6]) / 16.0};
-    a.dist[(size_t)(i - a.r0) * a.ncols + (j - a.colbase)] =
-        finish_exact(*a.logt, rc, a.ex, nf, (double)ag[1] / 16.0, (double)ag[2] / 16.0, (double)ag[3] / 16.0, i, j,
-                     a.colbase, namb, nund, al);
-  }
-  count_flags(a.counters, namb, nund);
-  if (a.ex.amb) amb_warp_flush(a.ex.amb, al);
-}
+// Columns per segment of the formula, stats and write kernels: a warp handles one (row, segment), so a band of a few
+// long rows still fills the GPU.
+constexpr int kSeg = 1024;
+
+#include "split_pair.cuh"
 
 static_assert(sizeof(PairArgs) % 4 == 0, "PairArgs is copied as 32-bit words");
 
@@ -914,7 +857,7 @@ __global__ void __launch_bounds__(256, MINB)
       cur = T.k;
     }
     __syncthreads();
-    pair_tile<WPLANE, GAPMM, false>(sd, smem_raw, colacc, T.i0, T.j0, T.rpw);
+    pair_tile<WPLANE, GAPMM>(sd, smem_raw, colacc, T.i0, T.j0, T.rpw);
     __syncthreads();
   }
 }
@@ -1319,10 +1262,6 @@ __device__ __forceinline__ int self_len(const RowArgs &a, long i)
   if (a.rc.format == 1) return 2 * digits_of(i) + 4;
   return 0;
 }
-
-// Columns per segment of the stats and write kernels: a warp handles one (row, segment), so a band of a few
-// long rows still fills the GPU.
-constexpr int kSeg = 1024;
 
 // one warp per (row, segment): histogram, links, skips, maxima and the byte count of the segment's text
 __device__ __forceinline__ void stats_rows(const RowArgs &a, long bx, int sg)
@@ -1891,51 +1830,58 @@ struct PerDevice {
 };
 
 // pair kernel launch (dynamic shared memory above the 48 KB default needs the opt-in attribute once per device).
-// Register budgets: 2 blocks per SM (128 registers, no spills) and 3 (80 registers, some spills) for the fused
-// kernel; 4 (64 registers) for the split kernel, which holds no formula state.
-template <int MINB, bool SPLIT>
+// Register budgets: 2 blocks per SM (128 registers, no spills), 3 (80 registers, some spills) or 4 (64).
+template <int MINB>
 cudaError_t launch_pair_t(const PairArgs &A, dim3 g, cudaStream_t st)
 {
   static PerDevice attr;
   cudaError_t e = attr.once([] {
     cudaError_t r;
-    if ((r = cudaFuncSetAttribute(pair_kernel<false, false, MINB, SPLIT>,
+    if ((r = cudaFuncSetAttribute(pair_kernel<false, false, MINB>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem)) != cudaSuccess)
       return r;
-    if ((r = cudaFuncSetAttribute(pair_kernel<true, false, MINB, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if ((r = cudaFuncSetAttribute(pair_kernel<true, false, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)kPairSmem)) != cudaSuccess)
       return r;
-    return cudaFuncSetAttribute(pair_kernel<true, true, MINB, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(pair_kernel<true, true, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)kPairSmem);
   });
   if (e != cudaSuccess) return e;
   if (A.rc.wplane) {
     if (A.rc.gapmm)
-      pair_kernel<true, true, MINB, SPLIT><<<g, 256, kPairSmem, st>>>(A);
+      pair_kernel<true, true, MINB><<<g, 256, kPairSmem, st>>>(A);
     else
-      pair_kernel<true, false, MINB, SPLIT><<<g, 256, kPairSmem, st>>>(A);
+      pair_kernel<true, false, MINB><<<g, 256, kPairSmem, st>>>(A);
   } else
-    pair_kernel<false, false, MINB, SPLIT><<<g, 256, kPairSmem, st>>>(A);
+    pair_kernel<false, false, MINB><<<g, 256, kPairSmem, st>>>(A);
   return cudaGetLastError();
 }
 
-// Whether the tensor-core path splits the pair stage into the event kernel and formula_kernel. One fused kernel
-// overlaps the formula with the event sums and is the faster form on the 6,700 x 1,500 HIV benchmark set in every
-// mode once the event loads are batched (fused 3.31 / 5.44 ms vs split 3.62 / 6.13 ms per resolve / gapmm pair
-// stage), so it is the default; TN93G_PAIR_SPLIT=1 selects the split form, which gives the same bytes.
-int pair_split(const RunConsts &)
+template <bool WPLANE, bool GAPMM, bool PACK>
+cudaError_t launch_event_t(const PairArgs &A, dim3 g, cudaStream_t st)
 {
-  static const int v = [] {
-    const char *e = getenv("TN93G_PAIR_SPLIT");
-    return e && atoi(e) ? 1 : 0;
-  }();
-  return v;
+  static PerDevice attr;
+  const cudaError_t e = attr.once([] {
+    return cudaFuncSetAttribute(event_kernel<WPLANE, GAPMM, PACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)EvTile<WPLANE>::smem);
+  });
+  if (e != cudaSuccess) return e;
+  event_kernel<WPLANE, GAPMM, PACK><<<g, kEvThreads, EvTile<WPLANE>::smem, st>>>(A);
+  return cudaGetLastError();
 }
 
-// Resident blocks per SM with the tensor-core counts: 4 (64 registers a thread) when the N plane is off, 3 (80) when
-// it is on (6,700 x 1,500 benchmark set, same box: resolve 3.18 ms with 4 vs 3.25 ms with 3 per pair stage, gapmm
-// 3.82 ms with 3 vs 3.89 ms with 4; 2 blocks, 128 registers without spills, 3.60 ms under resolve); 2 with the
-// popcount loop, which needs the registers. TN93G_PAIR_BLOCKS=2|3|4 overrides.
+// Whether a pair launch takes the split form (event_kernel, then formula_kernel): with the tensor-core records, whose
+// slots hold the final aggregates, packed event sums (16-bit lanes), a code matrix that 32-bit offsets reach and, under
+// the N plane, the sequences' N words.
+bool pair_split(const PairArgs &A)
+{
+  if (A.lin) return true;
+  return A.tcagg && A.ev2 && A.rc.packed && A.rc.Lc * A.rc.Npad < (1l << 32) && (!A.rc.wplane || A.wl_off);
+}
+
+// The pair stage of rows [A.r0, A.r1) and the columns from A.cstart (32 ncolblocks of them). Fused kernel: 4 resident
+// blocks per SM (64 registers a thread) with the tensor-core counts and no N plane, 3 (80) with it, 2 with the popcount
+// loop, which needs the registers. TN93G_PAIR_BLOCKS=2|3|4 overrides.
 cudaError_t launch_pair(const PairArgs &A, long ncolblocks, long nrows, cudaStream_t st)
 {
   static const int forced = [] {
@@ -1943,33 +1889,41 @@ cudaError_t launch_pair(const PairArgs &A, long ncolblocks, long nrows, cudaStre
     return e ? (atoi(e) == 4 ? 4 : atoi(e) == 3 ? 3 : 2) : 0;
   }();
   dim3 g((unsigned)ncolblocks, (unsigned)((nrows + kTile - 1) / kTile));
-  if (A.split && A.tcagg) {
-    cudaError_t e = launch_pair_t<4, true>(A, g, st);
+  if (pair_split(A)) {
+    const long jend = std::min<long>(A.rc.N, A.cstart + ncolblocks * kTile), jbeg = A.cstart & ~1l, ibeg = A.r0 & ~1l;
+    const long rows = A.rc.wplane ? EvTile<true>::rows : EvTile<false>::rows;
+    const dim3 ge((unsigned)((jend - jbeg + kEvCols - 1) / kEvCols), (unsigned)((A.r1 - ibeg + rows - 1) / rows));
+    const cudaError_t e = A.lin         ? cudaSuccess
+                          : A.rc.gapmm  ? launch_event_t<true, true, false>(A, ge, st)
+                          : A.rc.wplane ? launch_event_t<true, false, false>(A, ge, st)
+                          : A.tc16      ? launch_event_t<false, false, true>(A, ge, st)
+                                        : launch_event_t<false, false, false>(A, ge, st);
     if (e != cudaSuccess) return e;
-    const long ncol = ncolblocks * kTile;
-    // a few row groups per launch: each thread takes many rows, so that its ambiguity bounds and counters reach the
-    // global atomics once per launch, not once per row
-    const dim3 gf((unsigned)((ncol + 255) / 256), (unsigned)std::min<long>(nrows, 16));
-    static const int fb = [] {
-      const char *v = getenv("TN93G_FORMULA_BLOCKS");  // tuning knob: 2 (128 registers) or 3 (80)
-      return v && atoi(v) == 2 ? 2 : 3;
-    }();
-    if (fb == 2) {
+    // formula: a warp takes one segment of a few rows, or, where each column has a summary unit of its own (a server
+    // batch), a strip of 32 columns down many rows, so that a warp's pairs belong to one or two units. Long segments and
+    // several rows keep the atomics of a warp's totals rare (22.4 M pairs: 0.85 ms with 1,024 columns, 0.90 with 512);
+    // small launches take shorter segments, down to 128 columns, so that the SMs have two waves of warps (1,801 x 1,203 in
+    // bands of 0.2-0.4 M pairs: 0.10 -> 0.05 ms a band), and rows are added up only past four waves.
+    const long jlo = std::max(A.cstart, A.tcncols ? A.tccolbase : A.colbase);
+    int segw = A.ex.colunit ? 32 : kSeg;
+    while (segw > 128 && nrows * ((jend - jlo + segw - 1) / segw) < 148 * 48) segw /= 2;
+    const long nseg = (jend - jlo + segw - 1) / segw;
+    const int rpw = (int)std::max<long>(1, std::min<long>(1024 / std::min<long>(segw, jend - jlo), nrows * nseg / (148 * 128)));
+    const dim3 gf((unsigned)((nrows + kWarps * rpw - 1) / (kWarps * rpw)), (unsigned)nseg);
+    if (A.lin) {
       if (A.tc16)
-        formula_kernel<true, 2><<<gf, 256, 0, st>>>(A, ncol);
+        formula_kernel<true, true><<<gf, 256, 0, st>>>(A, jlo, jend, segw, rpw);
       else
-        formula_kernel<false, 2><<<gf, 256, 0, st>>>(A, ncol);
-    } else {
-      if (A.tc16)
-        formula_kernel<true, 3><<<gf, 256, 0, st>>>(A, ncol);
-      else
-        formula_kernel<false, 3><<<gf, 256, 0, st>>>(A, ncol);
-    }
+        formula_kernel<false, true><<<gf, 256, 0, st>>>(A, jlo, jend, segw, rpw);
+    } else if (A.tc16)
+      formula_kernel<true, false><<<gf, 256, 0, st>>>(A, jlo, jend, segw, rpw);
+    else
+      formula_kernel<false, false><<<gf, 256, 0, st>>>(A, jlo, jend, segw, rpw);
     return cudaGetLastError();
   }
   const int minb = forced ? forced : (A.tcagg ? (A.rc.wplane ? 3 : 4) : 2);
-  if (minb == 4) return launch_pair_t<4, false>(A, g, st);
-  return minb == 3 ? launch_pair_t<3, false>(A, g, st) : launch_pair_t<2, false>(A, g, st);
+  if (minb == 4) return launch_pair_t<4>(A, g, st);
+  return minb == 3 ? launch_pair_t<3>(A, g, st) : launch_pair_t<2>(A, g, st);
 }
 
 // the tensor-core count kernels' opt-in to their dynamic shared memory, once per device
@@ -2061,7 +2015,7 @@ struct tn93g_ctx {
   LogTable *d_logt = nullptr;
   Tables *h_tab = nullptr;
   PairTables *h_ptab = nullptr;  // host staging of the pair stage's tables
-  DevBuf seen, nN, varcol, planes, cc, ccT, evcount, evoff, ev, agg, site, dist, dcode, wcount, wloff, wl, rq, rqn, counters,
+  DevBuf seen, nN, varcol, planes, cc, ccT, evcount, evoff, ev, ev2, three, agg, site, dist, dcode, wcount, wloff, wl, rq, rqn, counters,
       rbytes, rsum, rw, fraw, fspan, flen, fcode,
       rmax, rlinks, rskip, hist, roff, out, hy;
   void *pinned = nullptr;
@@ -2105,6 +2059,9 @@ namespace {
       return e_ == cudaErrorMemoryAllocation ? TN93G_ENOMEM : TN93G_ECUDA;            \
     }                                                                                 \
   } while (0)
+
+// length of an event list with its null events
+uint32_t pad_events(uint32_t n) { return (n + kEvPad - 1) / kEvPad * kEvPad; }
 
 int ensure(tn93g_ctx *ctx, DevBuf &b, size_t bytes)
 {
@@ -2234,6 +2191,17 @@ void fill_pair_tables(const Tables &T, bool wplane, PairTables *out)
 {
   memcpy(out->agg, T.ev, sizeof out->agg);
   pack_tables(T, wplane, &out->packed);
+  event_tables(T, wplane, &out->events);
+}
+
+// Whether a run's records hold whole pairs (TcClasses weights): the modes without resolution, on the tensor cores
+bool weighted_mode(int mode) { return mode == TN93G_AVERAGE || mode == TN93G_GAPMM || mode == TN93G_SKIP; }
+
+TcClasses tc_classes(int mode, bool weighted)
+{
+  TcClasses C;
+  class_weights(mode, weighted, C.w);
+  return C;
 }
 
 // the summary units' bounds (ExactSink::amb words) as doubles: {largest low, largest high, spread, count}
@@ -2491,7 +2459,7 @@ void tn93g_destroy(tn93g_ctx *ctx)
   if (!ctx) return;
   cudaSetDevice(ctx->device);
   DevBuf *bufs[] = {&ctx->seen, &ctx->nN, &ctx->varcol, &ctx->planes, &ctx->cc, &ctx->ccT, &ctx->evcount,
-                    &ctx->evoff, &ctx->ev, &ctx->agg, &ctx->site, &ctx->dist, &ctx->dcode, &ctx->wcount, &ctx->wloff, &ctx->wl, &ctx->fraw, &ctx->fspan, &ctx->flen, &ctx->fcode, &ctx->rq, &ctx->rqn, &ctx->counters,
+                    &ctx->evoff, &ctx->ev, &ctx->ev2, &ctx->three, &ctx->agg, &ctx->site, &ctx->dist, &ctx->dcode, &ctx->wcount, &ctx->wloff, &ctx->wl, &ctx->fraw, &ctx->fspan, &ctx->flen, &ctx->fcode, &ctx->rq, &ctx->rqn, &ctx->counters,
                     &ctx->rbytes, &ctx->rsum, &ctx->rw, &ctx->rmax, &ctx->rlinks, &ctx->rskip, &ctx->hist,
                     &ctx->roff, &ctx->out, &ctx->hy};
   for (DevBuf *b : bufs)
@@ -2941,8 +2909,10 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   // a column is constant when every sequence has the same clean base there: each pair gets (b, b)
   std::vector<int32_t> varcol;
   varcol.reserve(L);
+  bool three = false;
   for (long p = 0; p < L; p++) {
     const uint32_t m = seen[p];
+    three |= (m & 0x7800u) != 0;
     if (m && !(m & (m - 1)) && m < 16) {
       const int b = __builtin_ctz(m);
       rc.constT++;
@@ -2966,6 +2936,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   TRY(ensure(ctx, ctx->ccT, (size_t)std::max<long>(Lc, 1) * Npad));
   TRY(ensure(ctx, ctx->evcount, N * sizeof(uint32_t)));
   TRY(ensure(ctx, ctx->evoff, (N + 1) * sizeof(uint32_t)));
+  TRY(ensure(ctx, ctx->three, N));
   if (Lc) CU(cudaMemcpyAsync(ctx->varcol.p, varcol.data(), Lc * sizeof(int32_t), cudaMemcpyHostToDevice, st));
   CU(cudaMemsetAsync(ctx->planes.p, 0, (size_t)std::max<long>(W, 1) * rc.NP * Npad * sizeof(uint64_t), st));
   CU(cudaMemsetAsync(ctx->evcount.p, 0, N * sizeof(uint32_t), st));
@@ -2984,6 +2955,8 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   pa.cc = (uint8_t *)ctx->cc.p;
   pa.evcount = (uint32_t *)ctx->evcount.p;
   pa.ev_off = (const uint32_t *)ctx->evoff.p;
+  // three-fold codes anywhere: the events kernel then marks their sequences
+  pa.three = three && opts->mode != TN93G_SKIP ? (uint8_t *)ctx->three.p : nullptr;
   if (W) {
     pack_kernel<<<dim3((unsigned)((N + kWarps - 1) / kWarps), (unsigned)std::min<long>(W, 65535)), 256, 0, st>>>(pa);
     CU(cudaGetLastError());
@@ -2993,8 +2966,11 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     CU(cudaGetLastError());
     ctx->launches++;
   }
+  const bool use_tc = ctx->count_path == 1 && Lc > 0;
+  const bool lin = use_tc && weighted_mode(opts->mode);  // the records will hold the ambiguity codes
+  const bool use_ev = !lin || (three && opts->mode != TN93G_SKIP);  // events are needed: all, or for three-fold codes
   // per sequence, its nonzero N-plane words (the pair kernel's sparse N-plane pass); counted here, listed below
-  bool sparse_w = rc.wplane && W > 0;
+  bool sparse_w = rc.wplane && W > 0 && (!lin || rc.gapmm);
   std::vector<uint32_t> wcnt;
   if (sparse_w) {
     TRY(ensure(ctx, ctx->wcount, N * sizeof(uint32_t)));
@@ -3006,8 +2982,8 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     CU(cudaMemcpyAsync(wcnt.data(), ctx->wcount.p, N * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   }
   std::vector<uint32_t> evc(N), evoff(N + 1);
-  CU(cudaMemcpyAsync(evc.data(), ctx->evcount.p, N * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  CU(cudaStreamSynchronize(st));
+  if (use_ev) CU(cudaMemcpyAsync(evc.data(), ctx->evcount.p, N * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  if (use_ev || sparse_w) CU(cudaStreamSynchronize(st));
   if (sparse_w) {
     std::vector<uint32_t> woff(N + 1);
     unsigned long long t = 0;
@@ -3032,14 +3008,18 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   evoff[0] = 0;
   uint32_t max_ev = 0;
   for (long i = 0; i < N; i++) {
-    evoff[i + 1] = evoff[i] + evc[i];
-    max_ev = std::max(max_ev, evc[i]);
+    const uint32_t n = pad_events(evc[i]);
+    evoff[i + 1] = evoff[i] + n;
+    max_ev = std::max(max_ev, n);
   }
   rc.packed = max_ev <= (uint32_t)kPackedMaxEvents;
   TRY(ensure(ctx, ctx->ev, std::max<size_t>(evoff[N], 1) * sizeof(uint32_t)));
+  TRY(ensure(ctx, ctx->ev2, std::max<size_t>(evoff[N], 1) * sizeof(uint2)));
   CU(cudaMemcpyAsync(ctx->evoff.p, evoff.data(), (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
   pa.ev = (uint32_t *)ctx->ev.p;
-  if (W && evoff[N]) {
+  pa.ev2 = (uint2 *)ctx->ev2.p;
+  pa.ev2_Npad = (uint32_t)Npad;
+  if (W && evoff[N]) {  // no list: nothing reads one
     events_kernel<<<(unsigned)((N + kWarps - 1) / kWarps), 256, 0, st>>>(pa);
     CU(cudaGetLastError());
     ctx->launches++;
@@ -3053,7 +3033,6 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   CU(cudaMemcpyAsync(ctx->site.p, ctx->h_tab->site, sizeof(ctx->h_tab->site), cudaMemcpyHostToDevice, st));
   // tensor-core count path: the one-hot operand image of every sequence (an extra 32-sequence block at the end,
   // which the last 64-column tile reads)
-  const bool use_tc = ctx->count_path == 1 && Lc > 0;
   const long tc_NB = (N + 31) / 32 + 1, tc_KS = (Lc + kTcStageK - 1) / kTcStageK;
   if (use_tc) {
     TRY(ensure(ctx, ctx->ohimg, (size_t)tc_KS * tc_NB * kTcBlockBytes));
@@ -3061,7 +3040,8 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     CU(cudaMemsetAsync(ctx->tcerr.p, 0, sizeof(unsigned long long), st));
     const long nthr = tc_NB * 32 * tc_KS * (kTcStageK / 16);
     onehot_kernel<<<(unsigned)((nthr + 255) / 256), 256, 0, st>>>((const uint8_t *)ctx->cc.p, N, Lc, tc_NB, tc_KS,
-                                                                  (uint8_t *)ctx->ohimg.p, 0, tc_NB * 32);
+                                                                  (uint8_t *)ctx->ohimg.p, 0, tc_NB * 32,
+                                                                  tc_classes(opts->mode, lin));
     CU(cudaGetLastError());
     ctx->launches++;
     CU(tc_attr_once());
@@ -3329,6 +3309,9 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     A.ccT = (const uint8_t *)ctx->ccT.p;
     A.ev_off = (const uint32_t *)ctx->evoff.p;
     A.ev = (const uint32_t *)ctx->ev.p;
+    A.ev2 = pa.ev2;
+    A.three = pa.three;
+    A.lin = lin;
     A.tab = (const PairTables *)ctx->agg.p;
     A.r0 = r0;
     A.r1 = r1;
@@ -3385,12 +3368,11 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
         AC.dist = A.dist + (size_t)(c0 - r0) * ncols;
         AC.tcagg = ctx->tcagg.p;
         AC.tc16 = tc16;
-        AC.split = pair_split(AC.rc);
         const long cb0 = (ccs - colbase) / 32, cbs = (ncols + 31) / 32 - cb0;
         if (cbs > 0) {
           AC.cstart = colbase + cb0 * 32;
           CU(launch_pair(AC, cbs, c1 - c0, st));
-          ctx->launches += AC.split ? 2 : 1;
+          ctx->launches += pair_split(AC) && !AC.lin ? 2 : 1;
         }
       }
       nchunks[par] = (int)chunks.size();
@@ -4170,13 +4152,14 @@ struct tn93g_server {
   long Nref = 0, L = 0, W = 0, Npad = 0, cap_q = 0;
   int cap_nq = 0;
   size_t ev_ref = 0, ev_cap = 0, names_ref = 0;
-  DevBuf planes, cc, ccT, evcount, evoff, ev, agg, site, varcol, qcodes, counts, names, name_off, name_len, dist, rq,
+  DevBuf planes, cc, ccT, evcount, evoff, ev, ev2, three, agg, site, varcol, qcodes, counts, names, name_off, name_len, dist, rq,
       rqn, counters, segcols, sbytes, soff, slinks, sskip, smax, rsum, rw, hist, total, out, qout, qlinks, scantmp;
   void *pin = nullptr;
   size_t pin_n = 0;
   // tensor-core counts: the one-hot image of the reference and the batch's queries, and the aggregates of one
   // chunk of query columns at a time
   bool tc = false;
+  bool lin = false;  // the records hold the ambiguity codes (average, gapmm, skip)
   int tc16 = 0;
   long tc_NB = 0, tc_KS = 0;
   DevBuf ohimg, tcagg, tcerr;
@@ -4206,7 +4189,7 @@ void tn93g_server_destroy(tn93g_server *srv)
   if (!srv) return;
   tn93g_ctx *ctx = srv->ctx;
   if (ctx) cudaSetDevice(ctx->device);
-  DevBuf *bufs[] = {&srv->planes, &srv->cc, &srv->ccT, &srv->evcount, &srv->evoff, &srv->ev, &srv->agg, &srv->site,
+  DevBuf *bufs[] = {&srv->planes, &srv->cc, &srv->ccT, &srv->evcount, &srv->evoff, &srv->ev, &srv->ev2, &srv->three, &srv->agg, &srv->site,
                     &srv->varcol, &srv->qcodes, &srv->counts, &srv->names, &srv->name_off, &srv->name_len,
                     &srv->dist, &srv->rq, &srv->rqn, &srv->counters, &srv->segcols, &srv->sbytes, &srv->soff,
                     &srv->slinks, &srv->sskip, &srv->smax, &srv->rsum, &srv->rw, &srv->hist, &srv->total,
@@ -4301,9 +4284,12 @@ int tn93g_server_create(tn93g_ctx *ctx, tn93g_server **out, const uint8_t *codes
   SV(ensure(ctx, srv->ccT, (size_t)L * Np));
   SV(ensure(ctx, srv->evcount, cap_n * sizeof(uint32_t)));
   SV(ensure(ctx, srv->evoff, (cap_n + 1) * sizeof(uint32_t)));
+  SV(ensure(ctx, srv->three, cap_n));
   SV(ensure(ctx, srv->varcol, L * sizeof(int32_t)));
   SVC(cudaMemsetAsync(srv->planes.p, 0, (size_t)W * rc.NP * Np * sizeof(uint64_t), st));
   SVC(cudaMemsetAsync(srv->evcount.p, 0, cap_n * sizeof(uint32_t), st));
+  SVC(cudaMemsetAsync(srv->three.p, 0, cap_n, st));
+  SVC(cudaMemsetAsync(srv->ccT.p, kGap, (size_t)L * Np, st));  // slots past the batch read as gaps
   {
     std::vector<int32_t> id(L);
     for (long p = 0; p < L; p++) id[p] = (int32_t)p;
@@ -4333,15 +4319,19 @@ int tn93g_server_create(tn93g_ctx *ctx, tn93g_server **out, const uint8_t *codes
   SVC(cudaStreamSynchronize(st));
   evo[0] = 0;
   for (long i = 0; i < N; i++) {
-    evo[i + 1] = evo[i] + evc[i];
-    srv->ref_max_ev = std::max(srv->ref_max_ev, evc[i]);
+    evo[i + 1] = evo[i] + pad_events(evc[i]);
+    srv->ref_max_ev = std::max(srv->ref_max_ev, pad_events(evc[i]));
   }
   srv->ev_ref = evo[N];
-  srv->ev_cap = srv->ev_ref + (size_t)max_batch_sequences * L;
+  srv->ev_cap = srv->ev_ref + (size_t)max_batch_sequences * ((L + kEvPad - 1) / kEvPad * kEvPad);
   SV(ensure(ctx, srv->ev, std::max<size_t>(srv->ev_cap, 1) * sizeof(uint32_t)));
+  SV(ensure(ctx, srv->ev2, std::max<size_t>(srv->ev_cap, 1) * sizeof(uint2)));
   SVC(cudaMemcpyAsync(srv->evoff.p, evo.data(), (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
   pa.ev_off = (const uint32_t *)srv->evoff.p;
   pa.ev = (uint32_t *)srv->ev.p;
+  pa.ev2 = (uint2 *)srv->ev2.p;
+  pa.ev2_Npad = (uint32_t)Np;
+  pa.three = (uint8_t *)srv->three.p;
   if (srv->ev_ref) {
     events_kernel<<<(unsigned)((N + kWarps - 1) / kWarps), 256, 0, st>>>(pa);
     SVC(cudaGetLastError());
@@ -4414,12 +4404,14 @@ int tn93g_server_create(tn93g_ctx *ctx, tn93g_server **out, const uint8_t *codes
     if (ensure(ctx, srv->ohimg, img) == TN93G_OK && ensure(ctx, srv->tcagg, agg) == TN93G_OK &&
         ensure(ctx, srv->tcerr, sizeof(unsigned long long)) == TN93G_OK) {
       srv->tc = true;
+      srv->lin = weighted_mode(opts->mode);
       SV(tc_attr(ctx));
       const long nfull = N / 32 * 32;  // whole reference blocks (the block shared with queries is built per batch)
       if (nfull) {
         const long nthr = nfull * srv->tc_KS * (kTcStageK / 16);
         onehot_kernel<<<(unsigned)((nthr + 255) / 256), 256, 0, st>>>((const uint8_t *)srv->cc.p, N, L, srv->tc_NB,
-                                                                      srv->tc_KS, (uint8_t *)srv->ohimg.p, 0, nfull);
+                                                                      srv->tc_KS, (uint8_t *)srv->ohimg.p, 0, nfull,
+                                                                      tc_classes(opts->mode, srv->lin));
         SVC(cudaGetLastError());
       }
     } else {
@@ -4529,14 +4521,17 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
   evo[0] = (uint32_t)srv->ev_ref;
   uint32_t max_ev = srv->ref_max_ev;
   for (long k = 0; k < Q; k++) {
-    evo[k + 1] = evo[k] + evc[k];
-    max_ev = std::max(max_ev, evc[k]);
+    evo[k + 1] = evo[k] + pad_events(evc[k]);
+    max_ev = std::max(max_ev, pad_events(evc[k]));
   }
   rc.packed = max_ev <= (uint32_t)kPackedMaxEvents;
   CU(cudaMemcpyAsync((uint32_t *)srv->evoff.p + Nref, evo.data(), (Q + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice,
                      st));
   pa.ev_off = (const uint32_t *)srv->evoff.p + Nref;
   pa.ev = (uint32_t *)srv->ev.p;
+  pa.ev2 = (uint2 *)srv->ev2.p;
+  pa.ev2_Npad = (uint32_t)Np;
+  pa.three = (uint8_t *)srv->three.p + Nref;
   if (evo[Q] > evo[0]) {
     events_kernel<<<(unsigned)((Q + kWarps - 1) / kWarps), 256, 0, st>>>(pa);
     CU(cudaGetLastError());
@@ -4565,7 +4560,7 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
     CU(cudaMemsetAsync(srv->tcerr.p, 0, sizeof(unsigned long long), st));
     onehot_kernel<<<(unsigned)((nthr + 255) / 256), 256, 0, st>>>((const uint8_t *)srv->cc.p, Nref + Q, L, srv->tc_NB,
                                                                   srv->tc_KS, (uint8_t *)srv->ohimg.p, b0 * 32,
-                                                                  (b1 - b0) * 32);
+                                                                  (b1 - b0) * 32, tc_classes(rc.mode, srv->lin));
     CU(cudaGetLastError());
     ctx->launches++;
   }
@@ -4591,6 +4586,9 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
     A.ccT = (const uint8_t *)srv->ccT.p;
     A.ev_off = (const uint32_t *)srv->evoff.p;
     A.ev = (const uint32_t *)srv->ev.p;
+    A.ev2 = (const uint2 *)srv->ev2.p;
+    A.three = rc.mode != TN93G_SKIP ? (const uint8_t *)srv->three.p : nullptr;
+    A.lin = srv->tc && srv->lin;
     A.tab = (const PairTables *)srv->agg.p;
     A.r0 = 0;
     A.r1 = Nref;
@@ -4631,12 +4629,11 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
         PairArgs AC = A;
         AC.tcagg = srv->tcagg.p;
         AC.tc16 = srv->tc16;
-        AC.split = pair_split(AC.rc);
         AC.tcncols = kServerTcChunk;
         AC.tccolbase = c0;
         AC.cstart = c0;
         CU(launch_pair(AC, (c1 - c0 + 31) / 32, Nref, st));
-        ctx->launches += AC.split ? 3 : 2;
+        ctx->launches += pair_split(AC) && !AC.lin ? 3 : 2;
       }
     } else {
       CU(launch_pair(A, (Q + 31) / 32, Nref, st));
@@ -4906,6 +4903,7 @@ struct OneHotDesc {
   const uint8_t *cc;
   long N, Lc, NB, KS;
   uint8_t *img;
+  TcClasses C;
 };
 
 __global__ void __launch_bounds__(256) colscan_batch_kernel(const ScanDesc *d, const int *off, int K)
@@ -4946,7 +4944,7 @@ __global__ void __launch_bounds__(256) onehot_batch_kernel(const OneHotDesc *d, 
 {
   const int k = batch_owner(off, K, blockIdx.x);
   const OneHotDesc &a = d[k];
-  onehot_body(a.cc, a.N, a.Lc, a.NB, a.KS, a.img, 0, a.NB * 32, (long)blockIdx.x - off[k]);
+  onehot_body(a.cc, a.N, a.Lc, a.NB, a.KS, a.img, 0, a.NB * 32, (long)blockIdx.x - off[k], a.C);
 }
 
 // the prefix sum of per-alignment block counts, uploaded to slot q of the offsets buffer; returns the total
@@ -5206,8 +5204,8 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
     uint32_t max_ev = 0;
     for (long i = 0; i < alns[k].n; i++) {
       evo[evo_off[k] + i] = (uint32_t)nev;
-      nev += evc[row_base[k] + i];
-      max_ev = std::max(max_ev, evc[row_base[k] + i]);
+      nev += pad_events(evc[row_base[k] + i]);
+      max_ev = std::max(max_ev, pad_events(evc[row_base[k] + i]));
     }
     evo[evo_off[k] + alns[k].n] = (uint32_t)nev;
     RC[k].packed = max_ev <= (uint32_t)kPackedMaxEvents;
@@ -5385,7 +5383,7 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
       T.err = (unsigned long long *)bb[BB_TCERR].p;
       T.wait_ns = ctx->wait_ns;
       T.skip_fill_block = -1;
-      ohd[k] = OneHotDesc{PA[k].cc, T.N, RC[k].Lc, T.NB, T.KS, (uint8_t *)bb[BB_OH].p + oh_off[k]};
+      ohd[k] = OneHotDesc{PA[k].cc, T.N, RC[k].Lc, T.NB, T.KS, (uint8_t *)bb[BB_OH].p + oh_off[k], tc_classes(opts[k].mode, false)};
       nbo[k] = (T.NB * 32 * T.KS * (kTcStageK / 16) + 255) / 256;
       for (long i0 = 0; i0 < T.N - 1; i0 += kTcRows)
         for (long j0 = (i0 + 1) / kTcCols * kTcCols; j0 < T.N; j0 += kTcCols) tct.push_back(make_int4(k, (int)i0, (int)j0, 0));

@@ -31,6 +31,9 @@ struct PackArgs {
   uint32_t *evcount;  // [N]
   const uint32_t *ev_off;
   uint32_t *ev;
+  uint2 *ev2 = nullptr;      // the events again as event_kernel reads them: {k * ev2_Npad, (code - 4) * kCodes * 8}
+  uint32_t ev2_Npad = 0;
+  uint8_t *three = nullptr;  // [N]: whether the sequence has a three-fold event (written with the events; nullptr: not)
 };
 
 struct RunConsts {
@@ -54,7 +57,10 @@ struct RunConsts {
 struct PairTables {
   AggEntry agg[kEvEntries + 5];
   PackedTables packed;
+  EventTables events;
 };
+static_assert(offsetof(PairTables, packed) % 16 == 0 && offsetof(PairTables, events) % 16 == 0 && sizeof(PairTables) % 16 == 0,
+              "the tables are copied as 16-byte words");
 
 // Where the pair stage reports exactness problems:
 //   * the undecided list: pairs whose printed bytes, histogram bin or link decision depend on which candidate the
@@ -91,11 +97,12 @@ struct PairArgs {
   const LogTable *logt;
   ExactSink ex;
   void *tcagg = nullptr;  // clean-site aggregates from the tensor-core kernel: one record per pair slot of
-                          // [band rows][ncols], 8 uint16 (16 bytes) or 8 int32 (32 bytes), 7 used; with split, the
-                          // pair kernel writes the pair's final x16 aggregates back into it
+                          // [band rows][ncols], 8 uint16 (16 bytes) or 8 int32 (32 bytes), 7 used; event_kernel writes
+                          // the pair's final x16 aggregates and its state back into it
   int tc16 = 0;           // the records are uint16 (every final aggregate fits: 32 L < 65536), else int32
-  int split = 0;          // tensor-core path only: the pair kernel stops before the formula, which formula_kernel
-                          // finishes from the records
+  bool lin = false;  // the records are sixteenths with the ambiguity codes in them (average, gapmm, skip): no events to add
+  const uint2 *ev2 = nullptr;      // the events as offsets (PackArgs::ev2); nullptr: the fused kernel runs
+  const uint8_t *three = nullptr;  // per sequence: it has a three-fold event (nullptr: none has)
   // The nonzero words of each sequence's N plane (N sites, or N and gap sites under gapmm): sequence s owns
   // wl[wl_off[s] .. wl_off[s + 1]). With the tensor-core counts and packed events, the pair kernel's N-plane
   // cross terms visit only these words; nullptr: every word.

@@ -22,9 +22,10 @@ void build_log_table(LogTable *T)
       c = (257.0 + 2.0 * i) / 256.0;  // centre of [1 + i/128, 1 + (i+1)/128)
     else
       c = (257.0 + 2.0 * i) / 512.0;  // centre of the folded interval [(128+i)/256, (129+i)/256)
-    T->c[i] = c;
-    split((__float128)1 / (__float128)c, T->invc_hi[i], T->invc_lo[i]);
-    split(logq((__float128)c), T->logc_hi[i], T->logc_lo[i]);
+    T->e[i].c = c;
+    T->e[i].pad = 0.0;
+    split((__float128)1 / (__float128)c, T->e[i].invc_hi, T->e[i].invc_lo);
+    split(logq((__float128)c), T->e[i].logc_hi, T->e[i].logc_lo);
   }
   const __float128 ln2 = logq((__float128)2);
   double h = (double)ln2;

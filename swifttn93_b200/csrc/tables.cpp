@@ -196,4 +196,47 @@ void pack_tables(const Tables &T, bool w_plane, PackedTables *P)
     }
 }
 
+void event_tables(const Tables &T, bool w_plane, EventTables *E)
+{
+  memset(E, 0, sizeof *E);
+  uint32_t bits = 0;
+  for (int k = 0; k < kEvEntries; k++)
+    for (int q = 0; q < 7; q++) bits |= (uint32_t)T.ev[k].v[q];
+  E->shift = bits ? __builtin_ctz(bits) : 0;
+  uint32_t most = 1;  // of any lane, the ambiguities' included
+  for (int c = kSparse0; c < kGap; c++)
+    for (int o = 0; o < kCodes; o++) {
+      const int k = (c - kSparse0) * kCodes + o;
+      const int32_t *v = T.ev[k].v;
+      uint32_t u[8];
+      for (int q = 0; q < 8; q++) {
+        u[q] = q < 7 ? (uint32_t)v[q] >> E->shift : (uint32_t)v[q];
+        if (u[q] > most) most = u[q];
+      }
+      const uint32_t w[2] = {u[0] | u[2] << 8 | u[1] << 16 | u[3] << 24, u[4] | u[6] << 8 | u[5] << 16 | u[7] << 24};
+      const bool partner_sparse = is_sparse_code(o, w_plane);
+      for (int q = 0; q < 2; q++) {
+        E->row[k][q] = w[q];
+        E->col[k][q] = partner_sparse ? 0u : w[q];
+      }
+      E->flag[k] = (uint8_t)v[8];
+    }
+  E->group = (int32_t)(255 / most / 4 * 4);
+}
+
+void class_weights(int mode, bool weighted, uint32_t w[kCodes])
+{
+  for (int c = 0; c < kCodes; c++) {
+    w[c] = 0;
+    if (!weighted || mode == 2) {
+      if (c < 4) w[c] = (weighted ? 4u : 1u) << (8 * c);
+      continue;
+    }
+    const int set = kSet[c == kGap && mode == 3 ? kN : c], n = __builtin_popcount(set);
+    if (n == 0 || n == 3) continue;
+    for (int x = 0; x < 4; x++)
+      if (set >> x & 1) w[c] |= (uint32_t)(4 / n) << (8 * x);
+  }
+}
+
 }  // namespace tn93

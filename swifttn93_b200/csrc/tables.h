@@ -10,7 +10,8 @@ constexpr int kCodes = 18;   // "ACGTURYSWKMBDHVN?-"
 constexpr int kGap = 17;
 constexpr int kN = 15;
 constexpr int kSparse0 = 4;  // first non-clean code
-constexpr int kSparseCodes = 13;  // codes 4..16
+constexpr int kSparseCodes = 14;  // codes 4..16, and a row of zeros for the null events that pad a list (code 17)
+constexpr int kEvPad = 4;         // event lists are padded to a multiple of this, so that kernels read four at a time
 
 // Lanes of an aggregate entry (x16 integers, exact while every contribution is a multiple of 1/16):
 //   0 T (total), 1 D (diagonal), 2 AG (A<->G), 3 CT (C<->T), 4 nfA, 5 nfC, 6 nfG  -- the main mode
@@ -67,6 +68,24 @@ struct PackedTables {
 };
 static_assert(offsetof(PackedTables, avg) % 16 == 0, "the AVERAGE differences are read as 16-byte words");
 void pack_tables(const Tables &T, bool w_plane, PackedTables *P);
+
+// The event kernel's copy of the event table: an entry is 8 bytes of 8-bit lanes, {T, AG, D, CT} and {nfA, nfG, nfC,
+// ambiguities}, every lane but the last in units of 2^shift sixteenths (the largest power of two that divides the whole
+// table: 1/4 under resolve, where no site contributes less, 1/16 under average). The byte lanes of `group` events add
+// without overflow (a multiple of 4), and masking a word with 0x00FF00FF gives the 16-bit lanes of PackedTables. col[]
+// is row[] with zeros where o is itself a sparse event code; flag[] is AggEntry lane 8.
+struct EventTables {
+  uint32_t row[kEvEntries][2];
+  uint32_t col[kEvEntries][2];
+  uint8_t flag[256];
+  int32_t shift, group, pad[2];
+};
+static_assert(sizeof(EventTables) % 16 == 0, "the event tables are copied as 16-byte words");
+void event_tables(const Tables &T, bool w_plane, EventTables *E);
+
+// The four class bytes of each code in the tensor cores' operand image (tc_count.cuh, TcClasses): weights in quarters of a
+// site under average, gapmm and skip (weighted), else a 1 for each clean base.
+void class_weights(int mode, bool weighted, uint32_t w[kCodes]);
 
 // true if code c is a "sparse event" code: not clean, not a gap, and not N when N has its own plane
 inline bool is_sparse_code(int c, bool w_plane) { return c >= kSparse0 && c < kGap && !(w_plane && c == kN); }

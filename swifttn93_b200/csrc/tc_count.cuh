@@ -11,6 +11,8 @@
 // so that the pair kernel can write the final x16 aggregates, at most 32 L, back into the same slot), else eight
 // int32 (32 bytes). The pair kernel reads a record with one vector load.
 //
+// (A pair's record holds whole counts when the image is one-hot, sixteenths of a site when it holds weights: TcClasses.)
+//
 // Operand image in HBM (built by onehot_kernel from the compressed codes): per 128-column stage s and 32-sequence
 // block b a 16 KB block at (s * NB + b) * 16 KB, in the canonical K-major layout without swizzle: row r =
 // 4 * sequence + class, row group g = r / 8 at g * 1024 B, 16-byte column chunk c at + c * 128 B, row r % 8 at
@@ -147,38 +149,59 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16])
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Per code, its four class bytes in the operand image (low byte: class A). Counting clean sites, a clean base has a 1 in
+// its own class. Under average, gapmm and skip a pair's whole contribution is the outer product of its codes' weights,
+// so the image holds 4 / |bases| in each base of the code's set (4, 2 or 1; gapmm reads a gap as N) and the product
+// matrix is the pair's 4 x 4 table in sixteenths, ambiguity codes included. Three-fold codes (weight 1/3) stay 0: their
+// pairs take the site-order walk.
+struct TcClasses {
+  uint32_t w[18];
+};
+
 // one thread per (sequence, 16 columns): the four class rows' 16 bytes of the operand image, for the sequences
 // [seq0, seq0 + nseq) (seq0 and nseq multiples of 32; sequences at or past N get zero rows)
 __device__ __forceinline__ void onehot_body(const uint8_t *__restrict__ cc, long N, long Lc, long NB, long KS,
-                                            uint8_t *img, long seq0, long nseq, long bx)
+                                            uint8_t *img, long seq0, long nseq, long bx, const TcClasses &C)
 {
+  __shared__ uint32_t sw[32];
+  if (threadIdx.x < 32) sw[threadIdx.x] = threadIdx.x < 18 ? C.w[threadIdx.x] : 0u;
+  __syncthreads();
   const long t = bx * 256l + threadIdx.x;
   const long nchunk = KS * (kTcStageK / 16);
   if (t >= nseq * nchunk) return;
   const long seq = seq0 + t / nchunk, ch = t % nchunk;
   const long s = ch / (kTcStageK / 16), c = ch % (kTcStageK / 16);
   const long k0 = ch * 16;
-  uint8_t code[16];
+  uint32_t code[16];
 #pragma unroll
-  for (int q = 0; q < 16; q++) code[q] = (seq < N && k0 + q < Lc) ? cc[seq * Lc + k0 + q] : (uint8_t)17;
+  for (int q = 0; q < 16; q++) code[q] = (seq < N && k0 + q < Lc) ? sw[cc[seq * Lc + k0 + q] & 31] : 0u;
   const long b = seq / 32, sl = seq % 32;
   uint8_t *blk = img + ((size_t)s * NB + b) * kTcBlockBytes;
+  // 4 x 4 byte transposes: class cls of four columns to a word
+  uint32_t w[4][4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const uint32_t a0 = code[4 * q], a1 = code[4 * q + 1], a2 = code[4 * q + 2], a3 = code[4 * q + 3];
+    const uint32_t x0 = __byte_perm(a0, a1, 0x5140), x1 = __byte_perm(a2, a3, 0x5140);
+    const uint32_t y0 = __byte_perm(a0, a1, 0x7362), y1 = __byte_perm(a2, a3, 0x7362);
+    w[0][q] = __byte_perm(x0, x1, 0x5410);
+    w[1][q] = __byte_perm(x0, x1, 0x7632);
+    w[2][q] = __byte_perm(y0, y1, 0x5410);
+    w[3][q] = __byte_perm(y0, y1, 0x7632);
+  }
 #pragma unroll
   for (int cls = 0; cls < 4; cls++) {
     const int r = (int)sl * 4 + cls;
-    uint32_t w[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      w[q] = (uint32_t)(code[4 * q] == cls) | ((uint32_t)(code[4 * q + 1] == cls) << 8) |
-             ((uint32_t)(code[4 * q + 2] == cls) << 16) | ((uint32_t)(code[4 * q + 3] == cls) << 24);
-    *reinterpret_cast<uint4 *>(blk + (r / 8) * 1024 + c * 128 + (r % 8) * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+    *reinterpret_cast<uint4 *>(blk + (r / 8) * 1024 + c * 128 + (r % 8) * 16) =
+        make_uint4(w[cls][0], w[cls][1], w[cls][2], w[cls][3]);
   }
 }
 
-__global__ void onehot_kernel(const uint8_t *__restrict__ cc, long N, long Lc, long NB, long KS, uint8_t *img,
-                              long seq0, long nseq)
+__global__ void __launch_bounds__(256) onehot_kernel(const uint8_t *__restrict__ cc, long N, long Lc, long NB, long KS,
+                                                     uint8_t *img, long seq0, long nseq,
+                                                     const __grid_constant__ TcClasses C)
 {
-  onehot_body(cc, N, Lc, NB, KS, img, seq0, nseq, blockIdx.x);
+  onehot_body(cc, N, Lc, NB, KS, img, seq0, nseq, blockIdx.x, C);
 }
 
 // Reads the accumulator of tile (i0, j0) (tensor memory from tacc, lane quarter q = 32 rows: sequences

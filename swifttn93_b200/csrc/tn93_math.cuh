@@ -29,6 +29,7 @@
 #define TSUB(a, b) __dsub_rn((a), (b))
 #define TMUL(a, b) __dmul_rn((a), (b))
 #define TDIV(a, b) __ddiv_rn((a), (b))
+#define TRCP(a) __drcp_rn(a)
 #define TFMA(a, b, c) __fma_rn((a), (b), (c))
 #define TFLOOR(a) floor(a)
 #define TBITS(x) ((uint64_t)__double_as_longlong(x))
@@ -41,6 +42,7 @@
 #define TSUB(a, b) ((a) - (b))
 #define TMUL(a, b) ((a) * (b))
 #define TDIV(a, b) ((a) / (b))
+#define TRCP(a) (1.0 / (a))
 #define TFMA(a, b, c) fma((a), (b), (c))
 #define TFLOOR(a) floor(a)
 static inline uint64_t tn_bits_host(double x) { uint64_t u; memcpy(&u, &x, 8); return u; }
@@ -62,10 +64,13 @@ constexpr double kMaxDist = 1000.0;
 // fills it once with quadruple-precision arithmetic (libquadmath) and uploads it.
 constexpr int kLogTab = 128;
 constexpr int kLogFold = 53;
-struct LogTable {
-  double c[kLogTab];
-  double invc_hi[kLogTab], invc_lo[kLogTab];
-  double logc_hi[kLogTab], logc_lo[kLogTab];
+struct LogEntry {  // one interval: read with 16-byte loads
+  double c, invc_hi;
+  double invc_lo, logc_hi;
+  double logc_lo, pad;
+};
+struct alignas(16) LogTable {
+  LogEntry e[kLogTab];
   double ln2_hi, ln2_lo;  // ln2_hi has 42 significant bits, so k * ln2_hi is exact for |k| < 2048
 };
 
@@ -118,11 +123,18 @@ TN_HD LogR tlog(const LogTable &T, double x, double band = kLogBand, double spre
     m = TMUL(m, 0.5);
     k += 1;
   }
-  const double c = T.c[idx];
+#if defined(__CUDA_ARCH__)
+  const double2 *te = reinterpret_cast<const double2 *>(&T.e[idx]);
+  const double2 e0 = __ldg(te), e1 = __ldg(te + 1);
+  const double c = e0.x, invc_hi = e0.y, invc_lo = e1.x, logc_hi = e1.y, logc_lo = __ldg(&T.e[idx].logc_lo);
+#else
+  const double c = T.e[idx].c, invc_hi = T.e[idx].invc_hi, invc_lo = T.e[idx].invc_lo, logc_hi = T.e[idx].logc_hi,
+               logc_lo = T.e[idx].logc_lo;
+#endif
   const double f = TSUB(m, c);  // exact (Sterbenz)
   // r = f / c as a double-double
-  const double r_hi = TMUL(f, T.invc_hi[idx]);
-  const double r_lo = TADD(TFMA(f, T.invc_hi[idx], -r_hi), TMUL(f, T.invc_lo[idx]));
+  const double r_hi = TMUL(f, invc_hi);
+  const double r_lo = TADD(TFMA(f, invc_hi, -r_hi), TMUL(f, invc_lo));
   // log1p(r) = r - r^2/2 + r^3 P(r), P(r) = 1/3 - r/4 + ... + r^8/11 (|r| < 2^-7: the tail is below 2^-70 r)
   const double q = r_hi;
   const double t2h = TMUL(q, q), t2l = TFMA(q, q, -t2h);
@@ -140,32 +152,30 @@ TN_HD LogR tlog(const LogTable &T, double x, double band = kLogBand, double spre
   two_sum(q, TMUL(-0.5, t2h), s_hi, s_lo);
   // remaining small terms: -t2l/2 + tail + r_lo / (1 + q)
   s_lo = TADD(s_lo, TADD(TADD(TMUL(-0.5, t2l), tail), TSUB(r_lo, TMUL(r_lo, q))));
-  // k ln2 + log c + (s_hi + s_lo)
-  const double kd = (double)k;
-  double u_hi, u_lo, v_hi, v_lo;
-  two_sum(TMUL(kd, T.ln2_hi), T.logc_hi[idx], u_hi, u_lo);
+  // k ln2 + log c + (s_hi + s_lo); with k = 0 (the arguments of close pairs) the ln2 terms are zero
+  double u_hi = logc_hi, u_lo = 0., kl = 0., v_hi, v_lo;
+  if (k != 0) {
+    const double kd = (double)k;
+    two_sum(TMUL(kd, T.ln2_hi), logc_hi, u_hi, u_lo);
+    kl = TMUL(kd, T.ln2_lo);
+  }
   two_sum(u_hi, s_hi, v_hi, v_lo);
-  const double lo = TADD(TADD(TADD(u_lo, v_lo), TADD(s_lo, T.logc_lo[idx])), TMUL(kd, T.ln2_lo));
+  const double lo = TADD(TADD(TADD(u_lo, v_lo), TADD(s_lo, logc_lo)), kl);
   double hi, lo2;
   fast_two_sum(v_hi, lo, hi, lo2);
-  // hi is the rounding of the double-double (hi + lo2); |exact - (hi + lo2)| <= 2^-69 |hi|
+  // hi is the rounding of the double-double (hi + lo2); |exact - (hi + lo2)| <= 2^-69 |hi|. The exact value lies
+  // within the band of a rounding midpoint exactly when moving the remainder away from zero by the band (and that
+  // error) makes the rounding change; the value it changes to is the other candidate.
   R.y = hi;
-  R.alt = hi;
   const uint64_t hb = TBITS(hi);
-  const int hexp = (int)((hb >> 52) & 0x7ff);
-  const double ulp = TDBL((uint64_t)(hexp > 52 ? hexp - 52 : 1) << 52);  // 2^(e-52)
-  const bool pow2 = (hb & 0x000FFFFFFFFFFFFFull) == 0;
-  const double E = TMUL(hi < 0 ? -hi : hi, 1.6940658945086007e-21);  // 2^-69 |hi|
-  // e_away > 0: the remainder points away from zero
-  const double e_away = hi < 0 ? -lo2 : lo2;
-  const double half = (e_away >= 0 || !pow2) ? TMUL(0.5, ulp) : TMUL(0.25, ulp);
-  const double margin = TSUB(TSUB(half, e_away < 0 ? -e_away : e_away), E);
-  if (margin <= TMUL(band, ulp)) {
-    R.amb = 1;
-    // neighbour of hi on the side of the remainder (spread ulps away; 1 unless a test widens it)
-    const bool away = e_away >= 0;
+  const double ulp = TDBL((hb & 0x7FF0000000000000ull) - (52ull << 52));  // 2^(e-52); |hi| >= 2^-53 here
+  const double d = TADD(TMUL(band, ulp), TMUL(TDBL(hb & 0x7FFFFFFFFFFFFFFFull), 1.6940658945086007e-21));
+  const bool up = lo2 >= 0;
+  R.alt = TADD(hi, up ? TADD(lo2, d) : TSUB(lo2, d));
+  R.amb = R.alt != hi;
+  if (spread != 1.0 && R.amb) {  // a test's wider candidate: spread ulps away on the side of the remainder
     const uint64_t sp = (uint64_t)spread;
-    R.alt = TDBL(away ? hb + sp : hb - sp);
+    R.alt = TDBL(up == (hi >= 0) ? hb + sp : hb - sp);
   }
   return R;
 }
@@ -219,7 +229,7 @@ TN_HD Prep tn93_prep(const double nf[4], double diag, double ag_in, double ct_in
   Prep P;
   const double s = TADD(TADD(TADD(nf[0], nf[1]), nf[2]), nf[3]);
   // tn93 divides 2 by s and 1 by s; scaling by 2 commutes with rounding, so 2 x (1 / s) is the same double
-  const double auxd = TDIV(1.0, s);
+  const double auxd = TRCP(s);
   const double tng = TMUL(2.0, auxd);
   double f0 = TMUL(nf[0], auxd), f1 = TMUL(nf[1], auxd), f2 = TMUL(nf[2], auxd), f3 = TMUL(nf[3], auxd);
   const double fR = TADD(f0, f2), fY = TADD(f1, f3);
@@ -227,8 +237,8 @@ TN_HD Prep tn93_prep(const double nf[4], double diag, double ag_in, double ct_in
   P.K1 = P.K2 = P.K3 = 0;
   double rR = 0, rY = 0;  // RN(1 / fR), RN(1 / fY)
   if (!P.k2p) {
-    rR = TDIV(1.0, fR);
-    rY = TDIV(1.0, fY);
+    rR = TRCP(fR);
+    rY = TRCP(fY);
     P.K1 = div_by(TMUL(TMUL(2.0, f0), f2), fR, rR);
     P.K2 = div_by(TMUL(TMUL(2.0, f1), f3), fY, rY);
     P.K3 = TMUL(2.0, TSUB(TSUB(TMUL(fR, fY), div_by(TMUL(TMUL(f0, f2), fY), fR, rR)),
