@@ -23,7 +23,7 @@ HOSTCXX = "g++"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 DEVICE_SOURCES = ["engine.cu"]
 HOST_SOURCES = ["tables.cpp", "logtable.cpp", "summary_json.cpp", "fasta.cpp"]
-HEADERS = ["kernels.cuh", "tn93_math.cuh", "tables.h", "tc_count.cuh", "split_pair.cuh"]
+HEADERS = ["kernels.cuh", "tn93_math.cuh", "tables.h", "tc_count.cuh", "split_pair.cuh", "chain_sum.cuh"]
 
 
 def _newer(out: Path, deps) -> bool:

@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "kernels.cuh"
+#include "chain_sum.cuh"
 #include "tc_count.cuh"
 #include "tn93g.h"
 
@@ -115,25 +116,53 @@ __device__ __forceinline__ void pack_body(const PackArgs &a, long bx, long w0, l
 
 __global__ void pack_kernel(PackArgs a) { pack_body(a, blockIdx.x, blockIdx.y, gridDim.y); }
 
-// one thread per sequence: how many of its N-plane words (plane 3 of each word) are nonzero
-__global__ void wcount_kernel(const uint64_t *planes, long N, long W, int NP, long Npad, uint32_t *wcount)
+// The nonzero N-plane words (plane 3 of each word) of 32 sequences by a block of 16 warps: lanes over the sequences, so
+// that loads coalesce, warps over 16 stretches of the words (one thread a sequence walked 468 words alone: 2,000 x 29,900
+// 91 us to count and 226 us to list, 8 and 21 us so).
+constexpr int kWlWarps = 16;
+
+__device__ __forceinline__ bool w_word(const uint64_t *planes, long w, int NP, long Npad, long i)
 {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  uint32_t n = 0;
-  for (long w = 0; w < W; w++) n += planes[((size_t)w * NP + 3) * Npad + i] != 0;
-  wcount[i] = n;
+  return planes[((size_t)w * NP + 3) * Npad + i] != 0;
 }
 
-// one thread per sequence: the indices of its nonzero N-plane words, in order, from wl_off[i]
-__global__ void wlist_kernel(const uint64_t *planes, long N, long W, int NP, long Npad, const uint32_t *wl_off,
-                             uint32_t *wl)
+// wcount[i]: how many of sequence i's words are nonzero
+__global__ void __launch_bounds__(32 * kWlWarps) wcount_kernel(const uint64_t *planes, long N, long W, int NP, long Npad,
+                                                               uint32_t *wcount)
 {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= N) return;
+  __shared__ uint32_t part[kWlWarps][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long i = blockIdx.x * 32l + lane;  // below Npad, a multiple of 32
+  uint32_t n = 0;
+#pragma unroll 4
+  for (long w = W * warp / kWlWarps; w < W * (warp + 1) / kWlWarps; w++) n += w_word(planes, w, NP, Npad, i);
+  part[warp][lane] = n;
+  __syncthreads();
+  if (warp == 0 && i < N) {
+    for (int k = 1; k < kWlWarps; k++) n += part[k][lane];
+    wcount[i] = n;
+  }
+}
+
+// wl: the indices of sequence i's nonzero words, in order, from wl_off[i]
+__global__ void __launch_bounds__(32 * kWlWarps) wlist_kernel(const uint64_t *planes, long N, long W, int NP, long Npad,
+                                                              const uint32_t *wl_off, uint32_t *wl)
+{
+  __shared__ uint32_t part[kWlWarps][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long i = blockIdx.x * 32l + lane;
+  const long w0 = W * warp / kWlWarps, w1 = W * (warp + 1) / kWlWarps;
+  uint32_t n = 0;
+#pragma unroll 4
+  for (long w = w0; w < w1; w++) n += w_word(planes, w, NP, Npad, i);
+  part[warp][lane] = n;
+  __syncthreads();
+  if (i >= N || n == 0) return;
   uint32_t o = wl_off[i];
-  for (long w = 0; w < W; w++)
-    if (planes[((size_t)w * NP + 3) * Npad + i] != 0) wl[o++] = (uint32_t)w;
+  for (int k = 0; k < warp; k++) o += part[k][lane];
+#pragma unroll 4
+  for (long w = w0; w < w1; w++)
+    if (w_word(planes, w, NP, Npad, i)) wl[o++] = (uint32_t)w;
 }
 
 __device__ __forceinline__ void put_event(const PackArgs &a, uint32_t at, uint32_t k, int c)
@@ -1072,29 +1101,47 @@ __global__ void __launch_bounds__(256) replay_batch_kernel(const ReplayArgs *des
     if (*descs[k].qn) replay_run(descs[k]);
 }
 
-// exclusive scan of a band's segment byte counts (one block), and the band total
+// exclusive scan of a band's segment byte counts (one block), and the band total: 4,096 counts at a time, four to a
+// thread, the next ones loaded while these are scanned. (46,900 counts: 58 us with a stretch of 46 to each thread, whose
+// loads do not coalesce, 35 us so.)
 __global__ void __launch_bounds__(1024) scan_kernel(const unsigned long long *in, unsigned long long *out, long n,
                                                    unsigned long long *total)
 {
-  __shared__ unsigned long long part[1024];
-  const long per = (n + 1023) / 1024;
-  const long b = threadIdx.x * per, e = min(n, b + per);
-  unsigned long long s = 0;
-  for (long k = b; k < e; k++) s += in[k];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    const unsigned long long v = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
-    __syncthreads();
-    part[threadIdx.x] += v;
-    __syncthreads();
+  __shared__ unsigned long long part[2][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long v[4], carry = 0;
+  auto load = [&](long b) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[k] = b + k < n ? in[b + k] : 0;
+  };
+  long b = threadIdx.x * 4l;
+  load(b);
+  for (long b0 = 0, t = 0; b0 < n; b0 += 4096, b += 4096, t++) {
+    const unsigned long long x[4] = {v[0], v[1], v[2], v[3]}, own = x[0] + x[1] + x[2] + x[3];
+    load(b + 4096);
+    unsigned long long inc = own;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += y;
+    }
+    if (lane == 31) part[t & 1][warp] = inc;
+    __syncthreads();  // the other buffer is free: every warp has passed the barrier after it read that one
+    unsigned long long w = part[t & 1][lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
+    }
+    unsigned long long run = carry + inc - own;
+    const unsigned long long before = __shfl_sync(0xffffffffu, w, (warp + 31) & 31);
+    if (warp) run += before;
+    carry += __shfl_sync(0xffffffffu, w, 31);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (b + k < n) out[b + k] = run;
+      run += x[k];
+    }
   }
-  unsigned long long run = threadIdx.x ? part[threadIdx.x - 1] : 0;
-  for (long k = b; k < e; k++) {
-    out[k] = run;
-    run += in[k];
-  }
-  if (threadIdx.x == 1023) *total = part[1023];
+  if (threadIdx.x == 0) *total = carry;
 }
 
 // Large exclusive scans in three coalesced passes: tile sums, a scan of the tile sums (scan_kernel), then each
@@ -1355,8 +1402,105 @@ __device__ __forceinline__ void stats_rows(const RowArgs &a, long bx, int sg)
 __global__ void __launch_bounds__(256, 6) stats_kernel(RowArgs a) { stats_rows(a, blockIdx.x, blockIdx.y); }
 
 
-// one warp per row: tn93's row sums in column order (swifttn93.cpp:2594-2602); lane 0 adds each chunk's terms in
-// order. The self-pair weights come first, as tn93 adds them when the row starts (swifttn93.cpp:2405-2415).
+// Sums in order by a warp (chain_sum.cuh): s and the result are the same in every lane.
+__device__ __forceinline__ double warp_total(double x)
+{
+  for (int o = 16; o; o >>= 1) x = __dadd_rn(x, __shfl_xor_sync(0xffffffffu, x, o));
+  return x;
+}
+
+// s plus the 32 lanes' terms, lane 0's first
+__device__ __forceinline__ double chain_add32(double s, double t)
+{
+  ChainBinade c;
+  bool ok = chain_binade(s, c);
+  const double s1 = __dadd_rn(s, warp_total(chain_round(c, t, ok)));
+  if (__all_sync(0xffffffffu, (ok && s1 < c.end) || t == 0.)) return __any_sync(0xffffffffu, t != 0.) ? s1 : s;
+#pragma unroll
+  for (int l = 0; l < 32; l++) s = __dadd_rn(s, __shfl_sync(0xffffffffu, t, l));
+  return s;
+}
+
+// s plus 128 terms: the lanes' t[0], then their t[1], ...
+__device__ __forceinline__ double chain_add128(double s, const double (&t)[4])
+{
+  ChainBinade c;
+  bool ok = chain_binade(s, c);
+  double x = 0.;
+#pragma unroll
+  for (int q = 0; q < 4; q++) x = __dadd_rn(x, chain_round(c, t[q], ok));
+  const double s1 = __dadd_rn(s, warp_total(x));
+  if (__all_sync(0xffffffffu, ok && s1 < c.end)) return s1;
+#pragma unroll 1
+  for (int q = 0; q < 4; q++) s = chain_add32(s, q == 0 ? t[0] : q == 1 ? t[1] : q == 2 ? t[2] : t[3]);
+  return s;
+}
+
+// s plus x[0], x[1], ... x[n - 1] (shared memory), in groups that grow to 1,024 while they succeed
+__device__ __forceinline__ double chain_shared(const double *x, int n, double s)
+{
+  const int lane = threadIdx.x & 31;
+  int len = 32;
+  for (int at = 0; at < n;) {
+    const int m = min(len, n - at);
+    ChainBinade c;
+    bool ok = chain_binade(s, c);
+    double y = 0.;
+    for (int k = lane; k < m; k += 32) y = __dadd_rn(y, chain_round(c, x[at + k], ok));
+    const double s1 = __dadd_rn(s, warp_total(y));
+    if (__all_sync(0xffffffffu, ok && s1 < c.end)) {
+      s = s1;
+      at += m;
+      len = min(2 * len, 1024);
+    } else if (m <= 32) {
+#pragma unroll 8
+      for (int k = 0; k < m; k++) s = __dadd_rn(s, x[at + k]);
+      at += m;
+    } else {
+      len = max(32, len / 4);
+    }
+  }
+  return s;
+}
+
+// tn93's sums over a unit's rows in row order (swifttn93.cpp:2838-2848): s0 += rs[3 r], w0 += rw[3 r] for r < n, by one
+// block. The block stages 2,048 rows in shared memory and loads the next ones while warp 0 adds the sums and warp 1 the
+// weights. 30,000 rows: 291 us with one thread adding them one by one, 105 us so.
+constexpr int kReduceChunk = 2048;
+template <int THREADS>
+__device__ __forceinline__ void chain_rows(const double *rs, const double *rw, long n, double *s0, double *w0)
+{
+  __shared__ double ss[kReduceChunk], sw[kReduceChunk];
+  constexpr int kPer = kReduceChunk / THREADS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double a[kPer], b[kPer], s = 0.;
+  auto load = [&](long r0) {
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+      const long r = r0 + k * THREADS + threadIdx.x;
+      a[k] = r < n ? rs[r * 3] : 0.;
+      b[k] = r < n ? rw[r * 3] : 0.;
+    }
+  };
+  load(0);
+  for (long r0 = 0; r0 < n; r0 += kReduceChunk) {
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+      ss[k * THREADS + threadIdx.x] = a[k];
+      sw[k * THREADS + threadIdx.x] = b[k];
+    }
+    __syncthreads();
+    load(r0 + kReduceChunk);
+    if (warp < 2) s = chain_shared(warp ? sw : ss, (int)min((long)kReduceChunk, n - r0), s);
+  }
+  if (warp < 2 && lane == 0) *(warp ? w0 : s0) = s;
+}
+
+// one warp per row: tn93's row sums in column order (swifttn93.cpp:2594-2602). The self-pair weights come first, as tn93
+// adds them when the row starts (swifttn93.cpp:2405-2415). Without -m the terms are added 128 at a time with the bits of
+// one after the other (chain_sum.cuh): 22.4 M pairs 231 us
+// with one shuffle and add a term, 81 us so.
 __device__ __forceinline__ void sum_rows(const RowArgs &a, long bx)
 {
   __shared__ double sterm[kWarps][32], sw[kWarps][32];
@@ -1377,37 +1521,35 @@ __device__ __forceinline__ void sum_rows(const RowArgs &a, long bx)
   }
   const double *drow = a.dist + (size_t)(i - a.r0) * a.ncols - a.colbase;
   if (!rc.fst) {
-    // Single bin: every lane adds the chunk's 32 terms in column order (the same chain in every lane, so no lane
-    // waits for another); skipped pairs and columns past the end add +0.0, which leaves a non-negative sum
+    // Single bin: 128 columns at a time; skipped pairs and columns past the end add +0.0, which leaves a non-negative sum
     // unchanged. The weights are integers: their double sum is exact, in any order, while the total stays below
     // 2^53, so they are added as integers (and re-added one by one in the rare case the total is larger).
-    // The next chunk's distance and count are loaded before this chunk's chain runs, so the loads overlap it.
+    // The next columns' distances and counts are loaded before these are added, so the loads overlap the chain.
     unsigned long long wsum = 0;
-    double raw = 0.;
-    long cj = 0;
-    if (lb + lane < cend) {
-      raw = drow[lb + lane];
-      cj = a.counts[lb + lane];
-    }
-    for (long j0 = lb; j0 < cend; j0 += 32) {
-      const long j = j0 + lane, jn = j + 32;
-      double raw_n = 0.;
-      long cj_n = 0;
-      if (jn < cend) {
-        raw_n = drow[jn];
-        cj_n = a.counts[jn];
-      }
-      double term = 0.;
-      if (j < cend && (uint64_t)__double_as_longlong(raw) != kSkipBits) {
-        const double t = raw <= 0. ? 0. : raw;
-        const long w = cnt_i * cj;
-        term = __dmul_rn(t, (double)w);
-        wsum += (unsigned long long)w;
-      }
+    double raw[4];
+    long cj[4];
+    auto load = [&](long j0) {
 #pragma unroll
-      for (int l = 0; l < 32; l++) s0 = __dadd_rn(s0, __shfl_sync(0xffffffffu, term, l));
-      raw = raw_n;
-      cj = cj_n;
+      for (int q = 0; q < 4; q++) {
+        const long j = j0 + 32 * q + lane;
+        raw[q] = j < cend ? drow[j] : __longlong_as_double((long long)kSkipBits);
+        cj[q] = j < cend ? a.counts[j] : 0;
+      }
+    };
+    load(lb);
+    for (long j0 = lb; j0 < cend; j0 += 128) {
+      double t[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        t[q] = 0.;
+        if ((uint64_t)__double_as_longlong(raw[q]) != kSkipBits) {
+          const long w = cnt_i * cj[q];
+          t[q] = __dmul_rn(raw[q] <= 0. ? 0. : raw[q], (double)w);
+          wsum += (unsigned long long)w;
+        }
+      }
+      load(j0 + 128);
+      s0 = chain_add128(s0, t);
     }
     for (int o = 16; o; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
     const unsigned long long svs = (!rc.cross && cnt_i > 1) ? (unsigned long long)(cnt_i * (cnt_i - 1l)) >> 1 : 0;
@@ -1681,36 +1823,22 @@ __global__ void __launch_bounds__(256) write_batch_kernel(const RowArgs *descs, 
 
 // Per alignment of a batch (single-file runs, bin 0 only): links, skips and maximum over its (row, segment)
 // slots, and tn93's mean numerator and weight: the rows' sums added in row order from 0 (swifttn93.cpp:2838-2848).
-// One block per alignment; thread 0 adds a shared-memory stage of the row sums in order.
+// One block per alignment.
 __global__ void __launch_bounds__(256) aln_reduce_kernel(const RowArgs *descs, double *out /* [K][3] */,
                                                          long long *cnt /* [K][2] */)
 {
-  __shared__ double ss[2048], sw[2048];
   __shared__ long long rl[8], rs[8];
   __shared__ double rm[8];
   const RowArgs &a = descs[blockIdx.x];
   const long nr = a.r1 - a.r0, ms = a.maxseg;
   long long links = 0, skipped = 0;
-  double m = 0., s0 = 0., w0 = 0.;
+  double m = 0.;
   for (long g = threadIdx.x; g < nr * ms; g += 256) {
     links += a.seg_links[g];
     skipped += a.seg_skip[g];
     m = fmax(m, a.seg_max[g * 3]);
   }
-  for (long r0 = 0; r0 < nr; r0 += 2048) {
-    const int n = (int)min(2048l, nr - r0);
-    for (int k = threadIdx.x; k < n; k += 256) {
-      ss[k] = a.row_sum[(r0 + k) * 3];
-      sw[k] = a.row_w[(r0 + k) * 3];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int k = 0; k < n; k++) {
-        s0 = __dadd_rn(s0, ss[k]);
-        w0 = __dadd_rn(w0, sw[k]);
-      }
-    __syncthreads();
-  }
+  chain_rows<256>(a.row_sum, a.row_w, nr, out + blockIdx.x * 3 + 1, out + blockIdx.x * 3 + 2);
   for (int o = 16; o; o >>= 1) {
     links += __shfl_xor_sync(0xffffffffu, links, o);
     skipped += __shfl_xor_sync(0xffffffffu, skipped, o);
@@ -1729,8 +1857,6 @@ __global__ void __launch_bounds__(256) aln_reduce_kernel(const RowArgs *descs, d
       m = fmax(m, rm[w]);
     }
     out[blockIdx.x * 3] = m;
-    out[blockIdx.x * 3 + 1] = s0;
-    out[blockIdx.x * 3 + 2] = w0;
     cnt[blockIdx.x * 2] = links;
     cnt[blockIdx.x * 2 + 1] = skipped;
   }
@@ -2974,7 +3100,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   std::vector<uint32_t> wcnt;
   if (sparse_w) {
     TRY(ensure(ctx, ctx->wcount, N * sizeof(uint32_t)));
-    wcount_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>((const uint64_t *)ctx->planes.p, N, W, rc.NP, Npad,
+    wcount_kernel<<<(unsigned)((N + 31) / 32), 32 * kWlWarps, 0, st>>>((const uint64_t *)ctx->planes.p, N, W, rc.NP, Npad,
                                                                 (uint32_t *)ctx->wcount.p);
     CU(cudaGetLastError());
     ctx->launches++;
@@ -2997,7 +3123,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
       TRY(ensure(ctx, ctx->wloff, (N + 1) * sizeof(uint32_t)));
       TRY(ensure(ctx, ctx->wl, std::max<size_t>(t, 1) * sizeof(uint32_t)));
       CU(cudaMemcpyAsync(ctx->wloff.p, woff.data(), (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-      wlist_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>((const uint64_t *)ctx->planes.p, N, W, rc.NP, Npad,
+      wlist_kernel<<<(unsigned)((N + 31) / 32), 32 * kWlWarps, 0, st>>>((const uint64_t *)ctx->planes.p, N, W, rc.NP, Npad,
                                                                  (const uint32_t *)ctx->wloff.p, (uint32_t *)ctx->wl.p);
       CU(cudaGetLastError());
       ctx->launches++;
@@ -4079,42 +4205,26 @@ __global__ void __launch_bounds__(256) qwrite_kernel(RowArgs a)
 }
 
 // Per query: links, skips and maxima over the reference rows, and tn93's mean numerator and weight: the rows' sums
-// added in row order, as tn93's writer adds them (swifttn93.cpp:2838-2848). One block per query: the block stages
-// chunks of row sums in shared memory with coalesced loads (and reduces the order-free counts and maxima), then
-// thread 0 adds the chunk in row order. Only bin 0 is used in a server batch (no -m).
-constexpr int kReduceChunk = 2048;
-
-__global__ void __launch_bounds__(256) query_reduce_kernel(RowArgs a, int nq, double *qout /* [nq][9] */,
+// added in row order, as tn93's writer adds them (swifttn93.cpp:2838-2848). One block per query. Only bin 0 is used in a
+// server batch (no -m).
+__global__ void __launch_bounds__(512) query_reduce_kernel(RowArgs a, int nq, double *qout /* [nq][9] */,
                                                            long long *qlinks /* [nq][2] */)
 {
-  __shared__ double ss[kReduceChunk], sw[kReduceChunk];
-  __shared__ long long rl[8], rs[8];
-  __shared__ double rm[8];
+  __shared__ long long rl[16], rs[16];
+  __shared__ double rm[16];
   const int q = blockIdx.x;
   const long nr = a.nrows;
   const size_t base = (size_t)q * nr;
+  double *o = qout + (size_t)q * 9;
   long long links = 0, skipped = 0;
-  double m = 0., s0 = 0., w0 = 0.;
-  for (long r0 = 0; r0 < nr; r0 += kReduceChunk) {
-    const int n = (int)min((long)kReduceChunk, nr - r0);
-    for (int k = threadIdx.x; k < n; k += 256) {
-      const size_t slot = base + r0 + k;
-      links += a.seg_links[slot];
-      skipped += a.seg_skip[slot];
-      m = fmax(m, a.seg_max[slot * 3]);
-      ss[k] = a.row_sum[slot * 3];
-      sw[k] = a.row_w[slot * 3];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll 8
-      for (int k = 0; k < n; k++) {
-        s0 = __dadd_rn(s0, ss[k]);
-        w0 = __dadd_rn(w0, sw[k]);
-      }
-    }
-    __syncthreads();
+  double m = 0.;
+#pragma unroll 4
+  for (long r = threadIdx.x; r < nr; r += 512) {
+    links += a.seg_links[base + r];
+    skipped += a.seg_skip[base + r];
+    m = fmax(m, a.seg_max[(base + r) * 3]);
   }
+  chain_rows<512>(a.row_sum + base * 3, a.row_w + base * 3, nr, o + 3, o + 6);
   for (int o = 16; o; o >>= 1) {
     links += __shfl_xor_sync(0xffffffffu, links, o);
     skipped += __shfl_xor_sync(0xffffffffu, skipped, o);
@@ -4127,17 +4237,14 @@ __global__ void __launch_bounds__(256) query_reduce_kernel(RowArgs a, int nq, do
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; w++) {
+    for (int w = 1; w < 16; w++) {
       links += rl[w];
       skipped += rs[w];
       m = fmax(m, rm[w]);
     }
-    double *o = qout + (size_t)q * 9;
     o[0] = m;
     o[1] = o[2] = 0.;
-    o[3] = s0;
     o[4] = o[5] = 0.;
-    o[6] = w0;
     o[7] = o[8] = 0.;
     qlinks[q * 2] = links;
     qlinks[q * 2 + 1] = skipped;
@@ -4700,7 +4807,7 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
     CU(launch_scan(RA.seg_bytes, (unsigned long long *)RA.seg_off, (long)nslot, (unsigned long long *)srv->total.p,
                    (unsigned long long *)srv->scantmp.p, st));
     ctx->launches++;
-    query_reduce_kernel<<<(unsigned)nq, 256, 0, st>>>(RA, nq, (double *)srv->qout.p, (long long *)srv->qlinks.p);
+    query_reduce_kernel<<<(unsigned)nq, 512, 0, st>>>(RA, nq, (double *)srv->qout.p, (long long *)srv->qlinks.p);
     CU(cudaGetLastError());
     ctx->launches++;
     CU(cudaEventRecord(E[4], st));
