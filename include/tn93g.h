@@ -180,7 +180,8 @@ typedef int (*tn93g_query_sink)(void *user, int query, const char *bytes, size_t
  * batched replay, statistics, sums, scan, per-alignment reduction and text. sink(user, k, bytes, n) receives
  * alignment k's whole distance file body and sums[k] its summary, exactly as tn93g_run on that alignment alone
  * would give them. rows_per_warp (NULL: 4) picks each alignment's pair-tile height (8 x 1, 2 or 4 rows by 32
- * columns) and pair_blocks (0: 2) the resident blocks per SM of the pair kernel (2 or 3); neither changes a result.
+ * columns) and pair_blocks (0: 2) the resident blocks per SM of the pair kernel (2 or 3), for the alignments that take
+ * the fused pair kernel (popcount path, N plane under resolve, more than 1,023 events); neither changes a result.
  * Replaces: one tn93 process per alignment (swifttn93.cpp:2222-2966 runs one file). */
 int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *alignments, const tn93g_opts *opts,
                     const int *rows_per_warp, int pair_blocks, tn93g_query_sink sink, void *user,

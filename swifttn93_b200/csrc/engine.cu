@@ -2005,6 +2005,20 @@ bool pair_split(const PairArgs &A)
   return A.tcagg && A.ev2 && A.rc.packed && A.rc.Lc * A.rc.Npad < (1l << 32) && (!A.rc.wplane || A.wl_off);
 }
 
+// Columns of a segment and rows of a warp in the formula kernel, for nrows x ncols pairs: a warp takes one segment of a few
+// rows, or, where each column has a summary unit of its own (a server batch), a strip of 32 columns down many rows, so that
+// a warp's pairs belong to one or two units. Long segments and several rows keep the atomics of a warp's totals rare (22.4 M
+// pairs: 0.85 ms with 1,024 columns, 0.90 with 512); small launches take shorter segments, down to 128 columns, so that the
+// SMs have two waves of warps (1,801 x 1,203 in bands of 0.2-0.4 M pairs: 0.10 -> 0.05 ms a band), and rows are added up
+// only past four waves.
+void formula_shape(long nrows, long ncols, bool units, int &segw, int &rpw)
+{
+  segw = units ? 32 : kSeg;
+  while (segw > 128 && nrows * ((ncols + segw - 1) / segw) < 148 * 48) segw /= 2;
+  const long nseg = (ncols + segw - 1) / segw;
+  rpw = (int)std::max<long>(1, std::min<long>(1024 / std::min<long>(segw, ncols), nrows * nseg / (148 * 128)));
+}
+
 // The pair stage of rows [A.r0, A.r1) and the columns from A.cstart (32 ncolblocks of them). Fused kernel: 4 resident
 // blocks per SM (64 registers a thread) with the tensor-core counts and no N plane, 3 (80) with it, 2 with the popcount
 // loop, which needs the registers. TN93G_PAIR_BLOCKS=2|3|4 overrides.
@@ -2025,16 +2039,10 @@ cudaError_t launch_pair(const PairArgs &A, long ncolblocks, long nrows, cudaStre
                           : A.tc16      ? launch_event_t<false, false, true>(A, ge, st)
                                         : launch_event_t<false, false, false>(A, ge, st);
     if (e != cudaSuccess) return e;
-    // formula: a warp takes one segment of a few rows, or, where each column has a summary unit of its own (a server
-    // batch), a strip of 32 columns down many rows, so that a warp's pairs belong to one or two units. Long segments and
-    // several rows keep the atomics of a warp's totals rare (22.4 M pairs: 0.85 ms with 1,024 columns, 0.90 with 512);
-    // small launches take shorter segments, down to 128 columns, so that the SMs have two waves of warps (1,801 x 1,203 in
-    // bands of 0.2-0.4 M pairs: 0.10 -> 0.05 ms a band), and rows are added up only past four waves.
     const long jlo = std::max(A.cstart, A.tcncols ? A.tccolbase : A.colbase);
-    int segw = A.ex.colunit ? 32 : kSeg;
-    while (segw > 128 && nrows * ((jend - jlo + segw - 1) / segw) < 148 * 48) segw /= 2;
+    int segw, rpw;
+    formula_shape(nrows, jend - jlo, A.ex.colunit != nullptr, segw, rpw);
     const long nseg = (jend - jlo + segw - 1) / segw;
-    const int rpw = (int)std::max<long>(1, std::min<long>(1024 / std::min<long>(segw, jend - jlo), nrows * nseg / (148 * 128)));
     const dim3 gf((unsigned)((nrows + kWarps * rpw - 1) / (kWarps * rpw)), (unsigned)nseg);
     if (A.lin) {
       if (A.tc16)
@@ -2113,7 +2121,7 @@ struct DevBuf {
   size_t n = 0;
 };
 
-constexpr int kBatchBufs = 56;
+constexpr int kBatchBufs = 64;
 constexpr int kMaxTcChunks = 48;         // row chunks of a band on the tensor-core count path
 // Pairs per chunk of the tensor-core path (count kernel, then pair kernel): 16 M pairs, 256 MB of 16-byte records.
 // Larger chunks amortise the persistent count kernel's pipeline fill and drain and the pair kernel's last wave
@@ -2207,6 +2215,16 @@ int ensure(tn93g_ctx *ctx, DevBuf &b, size_t bytes)
   b.n = bytes;
   ctx->used += bytes;
   return TN93G_OK;
+}
+
+// gives b back; the stream's work on it ends first (cudaFree waits for the device)
+void release(tn93g_ctx *ctx, DevBuf &b)
+{
+  if (!b.p) return;
+  cudaFree(b.p);
+  ctx->used -= b.n;
+  b.p = nullptr;
+  b.n = 0;
 }
 
 int ensure_pinned(tn93g_ctx *ctx, size_t bytes)
@@ -4976,7 +4994,7 @@ enum BatchBuf {
   BB_NAMES, BB_NAMEOFF, BB_NAMELEN, BB_COUNTS, BB_DIST, BB_RQ, BB_RQN, BB_COUNTERS, BB_PDESC, BB_RDESC, BB_ROWDESC,
   BB_TILES, BB_NEXT, BB_BLOCKS, BB_SBYTES, BB_SOFF, BB_SLINKS, BB_SSKIP, BB_SMAX, BB_RSUM, BB_RW, BB_HIST, BB_TOTAL,
   BB_SCANTMP, BB_RED, BB_REDC, BB_FIRST, BB_FIRSTIDX, BB_OUT, BB_OH, BB_TCAGG, BB_TCDESC, BB_TCTILES, BB_TCERR,
-  BB_UND, BB_UNDN, BB_AMB, BB_SCANDESC, BB_PACKDESC, BB_TRDESC, BB_OHDESC, BB_BOFF, BB_COUNT
+  BB_UND, BB_UNDN, BB_AMB, BB_SCANDESC, BB_PACKDESC, BB_TRDESC, BB_OHDESC, BB_BOFF, BB_EV2, BB_THREE, BB_SPLIT, BB_COUNT
 };
 static_assert(BB_COUNT <= kBatchBufs, "batch buffer table");
 
@@ -5076,6 +5094,19 @@ __global__ void gather_u64_kernel(const unsigned long long *src, const long *idx
 {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) dst[k] = src[idx[k]];
+}
+
+template <bool WPLANE, bool GAPMM, bool PACK>
+cudaError_t launch_event_batch(const PairArgs *descs, const int4 *blocks, size_t n, cudaStream_t st)
+{
+  static PerDevice attr;
+  const cudaError_t e = attr.once([] {
+    return cudaFuncSetAttribute(event_batch_kernel<WPLANE, GAPMM, PACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)EvTile<WPLANE>::smem);
+  });
+  if (e != cudaSuccess) return e;
+  event_batch_kernel<WPLANE, GAPMM, PACK><<<(unsigned)n, kEvThreads, EvTile<WPLANE>::smem, st>>>(descs, blocks);
+  return cudaGetLastError();
 }
 
 template <int MINB>
@@ -5202,6 +5233,7 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   CU(cudaStreamSynchronize(st));
   std::vector<RunConsts> RC(K);
   std::vector<int32_t> varcol;
+  std::vector<char> three(K, 0);  // three-fold codes anywhere (not under skip): the events kernel marks their sequences
   std::vector<size_t> vc_off(K + 1), pl_off(K + 1), cc_off(K + 1), cct_off(K + 1), evo_off(K + 1);
   vc_off[0] = pl_off[0] = cc_off[0] = cct_off[0] = evo_off[0] = 0;
   for (int k = 0; k < K; k++) {
@@ -5227,6 +5259,7 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
     rc.resolve_all = ctx->exact_sums;
     for (long p = 0; p < L; p++) {
       const uint32_t m = seen[seen_off[k] + p];
+      three[k] |= (m & 0x7800u) != 0 && o->mode != TN93G_SKIP;
       if (m && !(m & (m - 1)) && m < 16) {
         const int b = __builtin_ctz(m);
         rc.constT++;
@@ -5306,25 +5339,72 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   std::vector<uint32_t> evc(NR), evo(evo_off[K]);
   CU(cudaMemcpyAsync(evc.data(), bb[BB_EVCOUNT].p, NR * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   CU(cudaStreamSynchronize(st));
+  // Which alignments take the records path (event and formula kernels, as pair_split; average, gapmm and skip with the
+  // weighted operand image): all with variable columns on the tensor-core path but those with more than kPackedMaxEvents
+  // events in a sequence, with an N plane under resolve (the batch makes no N word lists) or with a code matrix past 32-bit
+  // offsets. 24 alignments of 50-2,000 x 900-3,000 in three modes: pair stage and replay 2.12 -> 0.93 ms. When its
+  // larger records do not fit, every alignment takes the fused kernel.
+  const bool use_tc = ctx->count_path == 1;
+  std::vector<char> split(K, 0), lin(K, 0);
+  std::vector<size_t> rec(K), ag_off(K + 1, 0);  // bytes of a pair's record; the alignments' records
   size_t nev = 0;
-  for (int k = 0; k < K; k++) {
-    uint32_t max_ev = 0;
-    for (long i = 0; i < alns[k].n; i++) {
-      evo[evo_off[k] + i] = (uint32_t)nev;
-      nev += pad_events(evc[row_base[k] + i]);
-      max_ev = std::max(max_ev, pad_events(evc[row_base[k] + i]));
+  auto plan_events = [&](bool may_split) -> int {
+    nev = 0;
+    for (int k = 0; k < K; k++) {
+      const bool on = use_tc && RC[k].W > 0 && alns[k].n > 1;
+      lin[k] = on && may_split && weighted_mode(opts[k].mode);
+      const bool none = lin[k] && !three[k];  // no list: nothing reads one
+      uint32_t max_ev = 0;
+      for (long i = 0; i < alns[k].n; i++) {
+        const uint32_t n = none ? 0 : pad_events(evc[row_base[k] + i]);
+        evo[evo_off[k] + i] = (uint32_t)nev;
+        nev += n;
+        max_ev = std::max(max_ev, n);
+      }
+      evo[evo_off[k] + alns[k].n] = (uint32_t)nev;
+      RC[k].packed = max_ev <= (uint32_t)kPackedMaxEvents;
+      split[k] = lin[k] || (on && may_split && RC[k].packed && !RC[k].wplane && RC[k].Lc * RC[k].Npad < (1l << 32));
+      // the fused kernel reads whole counts; the others write a pair's final sixteenths back into its record
+      rec[k] = (split[k] ? 32 * alns[k].L : 2 * RC[k].Lc) < 65536 ? 16 : 32;
+      ag_off[k + 1] = ag_off[k] + (on ? (size_t)alns[k].n * alns[k].n * rec[k] : 0);
     }
-    evo[evo_off[k] + alns[k].n] = (uint32_t)nev;
-    RC[k].packed = max_ev <= (uint32_t)kPackedMaxEvents;
+    if (nev >= (1ull << 32)) return TN93G_ETOOBIG;
+    TRY(ensure(ctx, bb[BB_EV], std::max<size_t>(nev, 1) * sizeof(uint32_t)));
+    if (may_split) {
+      TRY(ensure(ctx, bb[BB_EV2], std::max<size_t>(nev, 1) * sizeof(uint2)));
+      TRY(ensure(ctx, bb[BB_THREE], NR));
+    }
+    if (use_tc) TRY(ensure(ctx, bb[BB_TCAGG], std::max<size_t>(ag_off[K], 16)));
+    return TN93G_OK;
+  };
+  // the pair stage's other large buffers come first, so that only the records path itself can be what does not fit
+  std::vector<size_t> d_off(K + 1), q_off(K + 1);
+  d_off[0] = q_off[0] = 0;
+  for (int k = 0; k < K; k++) {
+    const size_t N = alns[k].n;
+    d_off[k + 1] = d_off[k] + N * N;
+    q_off[k + 1] = q_off[k] + std::max<size_t>(N * (N - 1) / 2, 1);
   }
-  if (nev >= (1ull << 32)) return TN93G_ETOOBIG;
-  TRY(ensure(ctx, bb[BB_EV], std::max<size_t>(nev, 1) * sizeof(uint32_t)));
+  TRY(ensure(ctx, bb[BB_DIST], d_off[K] * sizeof(double)));
+  TRY(ensure(ctx, bb[BB_RQ], q_off[K] * sizeof(unsigned long long)));
+  int planned = plan_events(use_tc);
+  if (use_tc && planned != TN93G_OK && planned != TN93G_ETOOBIG) {
+    cudaGetLastError();
+    release(ctx, bb[BB_EV2]);
+    planned = plan_events(false);
+  }
+  TRY(planned);
   CU(cudaMemcpyAsync(bb[BB_EVOFF].p, evo.data(), evo_off[K] * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
   {
     // every alignment's sparse events (one block per 8 sequences)
     std::vector<long> nbe(K);
     for (int k = 0; k < K; k++) {
       PA[k].ev = (uint32_t *)bb[BB_EV].p;
+      if (split[k]) {
+        PA[k].ev2 = (uint2 *)bb[BB_EV2].p;
+        PA[k].ev2_Npad = (uint32_t)RC[k].Npad;
+        PA[k].three = three[k] ? (uint8_t *)bb[BB_THREE].p + row_base[k] : nullptr;
+      }
       nbe[k] = (RC[k].W && evo[evo_off[k] + alns[k].n] > evo[evo_off[k]]) ? (RC[k].N + kWarps - 1) / kWarps : 0;
     }
     CU(cudaMemcpyAsync(bb[BB_PACKDESC].p, PA.data(), K * sizeof(PackArgs), cudaMemcpyHostToDevice, st));
@@ -5373,18 +5453,13 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   CU(cudaMemcpyAsync(bb[BB_SITE].p, h_site.data(), h_site.size() * sizeof(SiteEntry), cudaMemcpyHostToDevice, st));
   CU(cudaEventRecord(E[1], st));
   //------------------------------------------------------------------ pair stage
-  std::vector<size_t> d_off(K + 1), q_off(K + 1), seg_base(K + 1);
-  d_off[0] = q_off[0] = seg_base[0] = 0;
+  std::vector<size_t> seg_base(K + 1, 0);
   std::vector<long> maxseg(K);
   for (int k = 0; k < K; k++) {
     const size_t N = alns[k].n;
-    d_off[k + 1] = d_off[k] + N * N;
-    q_off[k + 1] = q_off[k] + std::max<size_t>(N * (N - 1) / 2, 1);
     maxseg[k] = std::max<long>(1, ((long)N + kSeg - 1) / kSeg);
     seg_base[k + 1] = seg_base[k] + N * maxseg[k];
   }
-  TRY(ensure(ctx, bb[BB_DIST], d_off[K] * sizeof(double)));
-  TRY(ensure(ctx, bb[BB_RQ], q_off[K] * sizeof(unsigned long long)));
   TRY(ensure(ctx, bb[BB_RQN], K * sizeof(unsigned)));
   TRY(ensure(ctx, bb[BB_COUNTERS], (size_t)K * 4 * sizeof(unsigned long long)));
   CU(cudaMemsetAsync(bb[BB_RQN].p, 0, K * sizeof(unsigned), st));
@@ -5446,11 +5521,10 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   std::vector<int> order(K);
   for (int k = 0; k < K; k++) order[k] = k;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return RC[a].Lc > RC[b].Lc; });
-  // tensor-core count path: per alignment a one-hot operand image and its clean-site aggregates ([7][n][n]),
-  // computed by one launch over every alignment's 32 x 64 tiles
-  const bool use_tc = ctx->count_path == 1;
+  // tensor-core count path: per alignment an operand image and its pairs' records ([n][n]), computed by one launch over
+  // every alignment's 32 x 64 tiles
   if (use_tc) {
-    std::vector<size_t> oh_off(K + 1, 0), ag_off(K + 1, 0);
+    std::vector<size_t> oh_off(K + 1, 0);
     std::vector<TcArgs> TD(K);
     std::vector<int4> tct;
     for (int k = 0; k < K; k++) {
@@ -5458,9 +5532,6 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
       const bool on = RC[k].W > 0 && N > 1;
       const long NB = (N + 31) / 32 + 1, KS = (RC[k].Lc + kTcStageK - 1) / kTcStageK;
       oh_off[k + 1] = oh_off[k] + (on ? (size_t)KS * NB * kTcBlockBytes : 0);
-      // byte offsets, each alignment's block 16-byte aligned
-      const size_t rec = 2 * RC[k].Lc < 65536 ? 16 : 32;  // bytes of a pair's record
-      ag_off[k + 1] = ag_off[k] + (on ? (size_t)N * N * rec : 0);
       TcArgs &T = TD[k];
       memset(&T, 0, sizeof T);
       T.NB = NB;
@@ -5476,7 +5547,6 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
       T.cend = N;
     }
     TRY(ensure(ctx, bb[BB_OH], std::max<size_t>(oh_off[K], 16)));
-    TRY(ensure(ctx, bb[BB_TCAGG], std::max<size_t>(ag_off[K], 16)));
     TRY(ensure(ctx, bb[BB_TCERR], sizeof(unsigned long long)));
     CU(cudaMemsetAsync(bb[BB_TCERR].p, 0, sizeof(unsigned long long), st));
     std::vector<OneHotDesc> ohd(K);
@@ -5486,16 +5556,20 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
       TcArgs &T = TD[k];
       T.onehot = (const uint8_t *)bb[BB_OH].p + oh_off[k];
       T.agg = (char *)bb[BB_TCAGG].p + ag_off[k];
-      T.agg16 = 2 * RC[k].Lc < 65536;
+      T.agg16 = rec[k] == 16;
       T.err = (unsigned long long *)bb[BB_TCERR].p;
       T.wait_ns = ctx->wait_ns;
       T.skip_fill_block = -1;
-      ohd[k] = OneHotDesc{PA[k].cc, T.N, RC[k].Lc, T.NB, T.KS, (uint8_t *)bb[BB_OH].p + oh_off[k], tc_classes(opts[k].mode, false)};
+      ohd[k] = OneHotDesc{PA[k].cc, T.N, RC[k].Lc, T.NB, T.KS, (uint8_t *)bb[BB_OH].p + oh_off[k],
+                          tc_classes(opts[k].mode, lin[k])};
       nbo[k] = (T.NB * 32 * T.KS * (kTcStageK / 16) + 255) / 256;
       for (long i0 = 0; i0 < T.N - 1; i0 += kTcRows)
         for (long j0 = (i0 + 1) / kTcCols * kTcCols; j0 < T.N; j0 += kTcCols) tct.push_back(make_int4(k, (int)i0, (int)j0, 0));
       PD[k].tcagg = T.agg;
       PD[k].tc16 = T.agg16;
+      PD[k].lin = lin[k];
+      PD[k].ev2 = PA[k].ev2;
+      PD[k].three = PA[k].three;
     }
     {
       // every alignment's one-hot operand image in one launch
@@ -5529,7 +5603,7 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   for (int cls = 0; cls < 3; cls++)
     for (int k : order) {
       const int kc = RC[k].gapmm ? 2 : RC[k].wplane ? 1 : 0;
-      if (kc != cls || !RC[k].W) continue;
+      if (kc != cls || !RC[k].W || split[k]) continue;
       const int rpw = rows_per_warp ? rows_per_warp[k] : kRowsPerWarp, trows = kWarps * rpw;
       const long N = alns[k].n;
       for (long i0 = 0; i0 < N - 1; i0 += trows)
@@ -5559,6 +5633,48 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
                         : launch_pair_batch_t<2>(ctx->sms, cls >= 1, cls == 2, dp, tp, cls_n[cls], nx, st));
     ctx->launches++;
     tbase += cls_n[cls];
+  }
+  // the records path: event tiles (by record width), then formula blocks (by record width and weighted image)
+  std::vector<int4> sb;
+  size_t sb_at[7] = {0};
+  for (int c = 0; c < 6; c++) {
+    for (int k : order) {
+      const long N = alns[k].n;
+      const bool w16 = rec[k] == 16;
+      if (!split[k]) continue;
+      if (c < 2) {
+        const int rows = EvTile<false>::rows;
+        if (lin[k] || w16 != (c == 0)) continue;
+        for (long i0 = 0; i0 < N - 1; i0 += rows)
+          for (long j0 = i0 / kEvCols * kEvCols; j0 < N; j0 += kEvCols)
+            sb.push_back(make_int4(k, (int)(j0 / kEvCols), (int)(i0 / rows), 0));
+      } else if (w16 == (c % 2 == 0) && (bool)lin[k] == (c >= 4)) {
+        int segw, rpw;
+        formula_shape(N, N, false, segw, rpw);
+        for (long by = 0; by * segw < N - 1; by++)  // the segments of a row start at its first column
+          for (long bx = 0; bx * kWarps * rpw < N - 1 - by * segw; bx++)
+            sb.push_back(make_int4(k, (int)bx, (int)by, rpw << 11 | segw));
+      }
+    }
+    sb_at[c + 1] = sb.size();
+  }
+  if (!sb.empty()) {
+    TRY(ensure(ctx, bb[BB_SPLIT], sb.size() * sizeof(int4)));
+    CU(cudaMemcpyAsync(bb[BB_SPLIT].p, sb.data(), sb.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
+    const PairArgs *dp = (const PairArgs *)bb[BB_PDESC].p;
+    for (int c = 0; c < 6; c++) {
+      const int4 *bl = (const int4 *)bb[BB_SPLIT].p + sb_at[c];
+      const size_t n = sb_at[c + 1] - sb_at[c];
+      if (!n) continue;
+      if (c == 0) CU((launch_event_batch<false, false, true>(dp, bl, n, st)));
+      if (c == 1) CU((launch_event_batch<false, false, false>(dp, bl, n, st)));
+      if (c == 2) formula_batch_kernel<true, false><<<(unsigned)n, 256, 0, st>>>(dp, bl);
+      if (c == 3) formula_batch_kernel<false, false><<<(unsigned)n, 256, 0, st>>>(dp, bl);
+      if (c == 4) formula_batch_kernel<true, true><<<(unsigned)n, 256, 0, st>>>(dp, bl);
+      if (c == 5) formula_batch_kernel<false, true><<<(unsigned)n, 256, 0, st>>>(dp, bl);
+      CU(cudaGetLastError());
+      ctx->launches++;
+    }
   }
   for (int k = 0; k < K; k++)
     if (!RC[k].W && alns[k].n > 1) {
@@ -5675,7 +5791,11 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   bool any_emit = false;
   for (int k = 0; k < K; k++) any_emit |= RC[k].emit;
   if (any_emit && total) {
-    if (bb[BB_OUT].n < total) TRY(ensure(ctx, bb[BB_OUT], total + total / 4));
+    if (bb[BB_OUT].n < total && ensure(ctx, bb[BB_OUT], total + total / 4) != TN93G_OK) {
+      cudaGetLastError();
+      release(ctx, bb[BB_TCAGG]);  // the records are not read any more
+      TRY(ensure(ctx, bb[BB_OUT], total + total / 4));
+    }
     TRY(ensure_pinned(ctx, total));
     for (int k = 0; k < K; k++) RA[k].out = (char *)bb[BB_OUT].p;
     CU(cudaMemcpyAsync(bb[BB_ROWDESC].p, RA.data(), K * sizeof(RowArgs), cudaMemcpyHostToDevice, st));

@@ -201,8 +201,9 @@ __device__ __forceinline__ int next_item(int *counter)
 
 __device__ __forceinline__ int ev_slot(int x) { return (x & 1) * 32 + (x >> 1); }
 
+// tile (bx, by) of the columns from a.cstart and the rows from a.r0, by all threads of the block
 template <bool WPLANE, bool GAPMM, bool PACK>
-__global__ void __launch_bounds__(kEvThreads, 2) event_kernel(PairArgs a)
+__device__ __forceinline__ void event_tile(const PairArgs &a, int bx, int by)
 {
   using T = EvTile<WPLANE>;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -211,7 +212,7 @@ __global__ void __launch_bounds__(kEvThreads, 2) event_kernel(PairArgs a)
   const int lane = threadIdx.x & 31;
   if (threadIdx.x < 2) items[threadIdx.x] = 0;
   // tiles start on even rows and columns (two codes per load); rows before r0 and columns before colbase are skipped
-  const int i0 = (int)(a.r0 & ~1l) + (int)blockIdx.y * T::rows, j0 = (int)(a.cstart & ~1l) + (int)blockIdx.x * kEvCols;
+  const int i0 = (int)(a.r0 & ~1l) + by * T::rows, j0 = (int)(a.cstart & ~1l) + bx * kEvCols;
   const int N = (int)rc.N, r1 = (int)a.r1;
   if (i0 >= r1 || j0 >= N || (!rc.cross && j0 + kEvCols - 1 <= i0)) return;
   const EventTables &ET = *reinterpret_cast<const EventTables *>(smem);
@@ -465,6 +466,29 @@ __global__ void __launch_bounds__(kEvThreads, 2) event_kernel(PairArgs a)
   }
 }
 
+template <bool WPLANE, bool GAPMM, bool PACK>
+__global__ void __launch_bounds__(kEvThreads, 2) event_kernel(PairArgs a)
+{
+  event_tile<WPLANE, GAPMM, PACK>(a, blockIdx.x, blockIdx.y);
+}
+
+// A batch of alignments: each block's (descriptor, bx, by, z). A descriptor's copy in shared memory, for all threads.
+__device__ __forceinline__ const PairArgs &batch_args(const PairArgs *descs, int k)
+{
+  __shared__ __align__(16) unsigned char raw[sizeof(PairArgs)];
+  for (int q = threadIdx.x; q < (int)(sizeof(PairArgs) / 4); q += blockDim.x)
+    reinterpret_cast<int32_t *>(raw)[q] = reinterpret_cast<const int32_t *>(&descs[k])[q];
+  __syncthreads();
+  return *reinterpret_cast<const PairArgs *>(raw);
+}
+
+template <bool WPLANE, bool GAPMM, bool PACK>
+__global__ void __launch_bounds__(kEvThreads, 2) event_batch_kernel(const PairArgs *descs, const int4 *blocks)
+{
+  const int4 b = blocks[blockIdx.x];
+  event_tile<WPLANE, GAPMM, PACK>(batch_args(descs, b.x), b.y, b.z);
+}
+
 // Whether pair (i, j) has a contribution that is not a multiple of 1/16 in a run whose records hold everything else: the
 // three-fold events of either sequence against the other's codes. Out of line: few sequences have one.
 __device__ __noinline__ bool three_pair(const uint8_t *flag, const uint8_t *three, const uint32_t *ev_off,
@@ -488,7 +512,7 @@ __device__ __noinline__ bool three_pair(const uint8_t *flag, const uint8_t *thre
 // under gapmm.
 constexpr int kFmQueue = 64;
 template <bool REC16, bool LIN>
-__global__ void __launch_bounds__(256, 3) formula_kernel(PairArgs a, long jlo, long jhi, int segw, int rpw)
+__device__ __forceinline__ void formula_rows(const PairArgs &a, long jlo, long jhi, int segw, int rpw, int bx, int by)
 {
   __shared__ double qlo[kWarps][kFmQueue], qhi[kWarps][kFmQueue];
   __shared__ int qi[kWarps][kFmQueue], qj[kWarps][kFmQueue];
@@ -535,19 +559,31 @@ __global__ void __launch_bounds__(256, 3) formula_kernel(PairArgs a, long jlo, l
       amb_add(a.ex.amb, other, unit, lo, hi, w);
     amb_warp_flush(a.ex.amb, other);
   };
-  const long ra = a.r0 + (blockIdx.x * (long)kWarps + warp) * rpw, rb = min(a.r1, ra + rpw);
+  const long ra = a.r0 + (bx * (long)kWarps + warp) * rpw, rb = min(a.r1, ra + rpw);
   for (long i = ra; i < rb; i++) {
     const long lb = rc.cross ? rc.n1 : i + 1;
-    const long s0 = (rc.cross ? jlo : max(lb, jlo)) + (long)blockIdx.y * segw;
+    const long s0 = (rc.cross ? jlo : max(lb, jlo)) + (long)by * segw;
     const long c0 = max(lb, s0), c1 = min(min(rc.N, jhi), s0 + segw);
     const size_t rec0 = (size_t)(i - a.r0) * tn - tb;
     double *const drow = a.dist + (size_t)(i - a.r0) * a.ncols - a.colbase;
     uint32_t q0 = 0, q1 = 0;
+    uint64_t gw = 0;
     bool ti = false;
     if (LIN) {
       if (rc.gapmm) {
-        q0 = a.wl_off ? a.wl_off[i] : 0u;
-        q1 = a.wl_off ? a.wl_off[i + 1] : (uint32_t)rc.W;
+        if (a.wl_off) {
+          q0 = a.wl_off[i];
+          q1 = a.wl_off[i + 1];
+        } else {
+          // no word lists (a batch): the row's nonzero gap words among the first 64 as a mask, the words past them all (24
+          // alignments of 900-3,000 columns: 0.33 ms of formula with every word read, 0.24 so)
+          const uint64_t *G = a.planes + 4 * rc.Npad + i;
+          const bool g0 = lane < rc.W && __ldg(G + (size_t)lane * rc.NP * rc.Npad);
+          const bool g1 = lane + 32 < rc.W && __ldg(G + (size_t)(lane + 32) * rc.NP * rc.Npad);
+          gw = (uint64_t)__ballot_sync(0xffffffffu, g0) | (uint64_t)__ballot_sync(0xffffffffu, g1) << 32;
+          q0 = 64;
+          q1 = (uint32_t)max(64l, rc.W);
+        }
       }
       ti = a.three && a.three[i];
     }
@@ -587,11 +623,12 @@ __global__ void __launch_bounds__(256, 3) formula_kernel(PairArgs a, long jlo, l
           ag[6] += 16 * (int)rc.constNf[2];
           if (rc.gapmm) {
             int n = 0;
-            for (uint32_t q = q0; q < q1; q++) {
-              const uint64_t *G = a.planes + ((size_t)(a.wl_off ? __ldg(a.wl + q) : q) * rc.NP + 4) * rc.Npad;
-              const uint64_t gi = __ldg(G + i);
-              if (gi) n += popc(gi & __ldg(G + j));
-            }
+            auto gaps = [&](uint32_t w) {
+              const uint64_t *G = a.planes + ((size_t)w * rc.NP + 4) * rc.Npad;
+              n += popc(__ldg(G + i) & __ldg(G + j));
+            };
+            for (uint64_t m = gw; m; m &= m - 1) gaps((uint32_t)__ffsll((long long)m) - 1);
+            for (uint32_t q = q0; q < q1; q++) gaps(a.wl_off ? __ldg(a.wl + q) : q);
             ag[0] -= 16 * n;
             ag[1] -= 4 * n;
             ag[2] -= 2 * n;
@@ -653,4 +690,19 @@ __global__ void __launch_bounds__(256, 3) formula_kernel(PairArgs a, long jlo, l
   if (qn) drain(qn);
   count_flags(a.counters, namb, nund);
   if (a.ex.amb) amb_warp_flush(a.ex.amb, al);
+}
+
+template <bool REC16, bool LIN>
+__global__ void __launch_bounds__(256, 3) formula_kernel(PairArgs a, long jlo, long jhi, int segw, int rpw)
+{
+  formula_rows<REC16, LIN>(a, jlo, jhi, segw, rpw, blockIdx.x, blockIdx.y);
+}
+
+// a batch of alignments: each block's (descriptor, bx, by, rows per warp * 2048 + columns of a segment)
+template <bool REC16, bool LIN>
+__global__ void __launch_bounds__(256, 3) formula_batch_kernel(const PairArgs *descs, const int4 *blocks)
+{
+  const int4 b = blocks[blockIdx.x];
+  const PairArgs &a = batch_args(descs, b.x);
+  formula_rows<REC16, LIN>(a, 0, a.rc.N, b.w & 2047, b.w >> 11, b.y, b.z);
 }
