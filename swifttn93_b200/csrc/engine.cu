@@ -26,6 +26,7 @@
 #include <atomic>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -2165,6 +2166,8 @@ struct tn93g_ctx {
   size_t pin2_n[2] = {0, 0};
   void *pstats = nullptr;
   size_t pstats_n = 0;
+  void *upload_pin = nullptr;  // upload_host's pieces (two a thread) and the events of their copies
+  cudaEvent_t upload_ev[8] = {nullptr};
   // device buffers of freed sets, kept for the next upload (repeated upload/free skips the allocator)
   std::vector<std::pair<void *, size_t>> set_pool;
   double timings[8] = {0};
@@ -2279,6 +2282,95 @@ int ensure_keep(tn93g_ctx *ctx, DevBuf &b, size_t bytes, size_t keep)
     int r_ = (x);                \
     if (r_ != TN93G_OK) return r_; \
   } while (0)
+
+// Host memory on its way to the device: n bytes from src to dst, behind the work of the context's stream.
+struct HostSpan {
+  void *dst;
+  const void *src;
+  size_t n;
+};
+
+// Queues the copies of the spans on the context's stream; pageable memory has been read when it returns. A copy from
+// pageable memory goes through the driver's staging buffer, filled by the calling thread alone (16-18 GB/s here, a third of
+// the link). From kUploadMin bytes on, up to kUploadThreads threads fill pinned buffers of the context instead, piece by
+// piece, and queue each piece's copy: 60 MB 3.4 -> 1.4 ms. The threads end with the call; where one cannot be started, or
+// the buffers cannot be allocated, the rest do its work.
+constexpr int kUploadThreads = 4;
+constexpr size_t kUploadPiece = 1 << 20;
+constexpr size_t kUploadMin = 4 << 20;
+
+int upload_host(tn93g_ctx *ctx, const std::vector<HostSpan> &spans)
+{
+  struct Piece {
+    char *dst;
+    const char *src;
+    size_t n;
+  };
+  std::vector<Piece> pieces;
+  for (const HostSpan &h : spans) {
+    cudaPointerAttributes pa;
+    bool direct = h.n < kUploadMin / 16;  // many small copies cost more than the staging saves
+    if (!direct) {
+      const cudaError_t e = cudaPointerGetAttributes(&pa, h.src);
+      if (e != cudaSuccess) cudaGetLastError();
+      direct = e == cudaSuccess && pa.type != cudaMemoryTypeUnregistered;  // pinned already
+    }
+    if (direct) {
+      if (h.n) CU(cudaMemcpyAsync(h.dst, h.src, h.n, cudaMemcpyHostToDevice, ctx->stream));
+      continue;
+    }
+    for (size_t at = 0; at < h.n; at += kUploadPiece)
+      pieces.push_back({(char *)h.dst + at, (const char *)h.src + at, std::min(kUploadPiece, h.n - at)});
+  }
+  size_t bytes = 0;
+  for (const Piece &p : pieces) bytes += p.n;
+  bool staged = bytes >= kUploadMin;
+  if (staged && !ctx->upload_pin) {
+    if (cudaHostAlloc(&ctx->upload_pin, 2 * kUploadThreads * kUploadPiece, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      ctx->upload_pin = nullptr;
+      staged = false;
+    }
+    for (int q = 0; staged && q < 2 * kUploadThreads; q++)
+      if (!ctx->upload_ev[q]) CU(cudaEventCreateWithFlags(&ctx->upload_ev[q], cudaEventDisableTiming));
+  }
+  if (!staged) {
+    for (const Piece &p : pieces) CU(cudaMemcpyAsync(p.dst, p.src, p.n, cudaMemcpyHostToDevice, ctx->stream));
+    return TN93G_OK;
+  }
+  std::atomic<size_t> next{0};
+  std::atomic<int> failed{0};
+  auto work = [&](int t) {
+    cudaSetDevice(ctx->device);
+    for (int turn = 0;; turn++) {
+      const size_t k = next++;
+      if (k >= pieces.size() || failed) break;
+      const int b = 2 * t + (turn & 1);
+      char *pin = (char *)ctx->upload_pin + b * kUploadPiece;
+      cudaError_t e = cudaEventSynchronize(ctx->upload_ev[b]);  // the buffer's previous copy (an earlier call's too)
+      if (e == cudaSuccess) {
+        memcpy(pin, pieces[k].src, pieces[k].n);
+        e = cudaMemcpyAsync(pieces[k].dst, pin, pieces[k].n, cudaMemcpyHostToDevice, ctx->stream);
+      }
+      if (e == cudaSuccess) e = cudaEventRecord(ctx->upload_ev[b], ctx->stream);
+      if (e != cudaSuccess) failed = (int)e;
+    }
+  };
+  std::thread helpers[kUploadThreads - 1];
+  const int most = std::min<int>(kUploadThreads, std::max(1u, std::thread::hardware_concurrency()));
+  for (int t = 1; t < most; t++) {
+    try {
+      helpers[t - 1] = std::thread(work, t);
+    } catch (const std::system_error &) {
+      break;
+    }
+  }
+  work(0);
+  for (std::thread &h : helpers)
+    if (h.joinable()) h.join();
+  CU((cudaError_t)(int)failed);
+  return TN93G_OK;
+}
 
 // The host's C library log of every listed argument: the decision oracle for pairs whose printed bytes or
 // decisions depend on how that log rounds (the reference calls the same function, swifttn93.cpp:1954-2001).
@@ -2626,6 +2718,9 @@ void tn93g_destroy(tn93g_ctx *ctx)
       if (e) cudaEventDestroy(e);
   }
   if (ctx->total.p) cudaFree(ctx->total.p);
+  if (ctx->upload_pin) cudaFreeHost(ctx->upload_pin);
+  for (cudaEvent_t e : ctx->upload_ev)
+    if (e) cudaEventDestroy(e);
   for (auto &b : ctx->set_pool) cudaFree(b.first);
   if (ctx->pstats) cudaFreeHost(ctx->pstats);
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
@@ -2692,7 +2787,15 @@ static int upload_set(tn93g_ctx *ctx, tn93g_set **out, const uint8_t *codes, cud
   if ((e = take((void **)&s->d_names, nbytes + 1, 2)) != cudaSuccess) return fail(e);
   if ((e = take((void **)&s->d_name_off, N * sizeof(uint64_t), 3)) != cudaSuccess) return fail(e);
   if ((e = take((void **)&s->d_name_len, N * sizeof(int32_t), 4)) != cudaSuccess) return fail(e);
-  if ((e = cudaMemcpyAsync(s->d_codes, codes, (size_t)N * L, codes_kind, ctx->stream)) != cudaSuccess) return fail(e);
+  if (codes_kind == cudaMemcpyHostToDevice) {
+    const int rc = upload_host(ctx, {{s->d_codes, codes, (size_t)N * L}});
+    if (rc != TN93G_OK) {
+      tn93g_free_set(ctx, s);
+      return rc;
+    }
+  } else if ((e = cudaMemcpyAsync(s->d_codes, codes, (size_t)N * L, codes_kind, ctx->stream)) != cudaSuccess) {
+    return fail(e);
+  }
   if ((e = cudaMemcpyAsync(s->d_counts, copy_counts, N * sizeof(long), cudaMemcpyHostToDevice, ctx->stream)) !=
       cudaSuccess)
     return fail(e);
@@ -5182,9 +5285,11 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   std::vector<uint64_t> noff(NR);
   std::vector<int32_t> nlen(NR);
   std::vector<long> cnts(NR);
+  std::vector<HostSpan> spans;
+  for (int k = 0; k < K; k++)
+    spans.push_back({(uint8_t *)bb[BB_CODES].p + code_off[k], alns[k].codes, code_off[k + 1] - code_off[k]});
+  TRY(upload_host(ctx, spans));
   for (int k = 0; k < K; k++) {
-    CU(cudaMemcpyAsync((uint8_t *)bb[BB_CODES].p + code_off[k], alns[k].codes, code_off[k + 1] - code_off[k],
-                       cudaMemcpyHostToDevice, st));
     if (name_base[k + 1] > name_base[k])
       CU(cudaMemcpyAsync((char *)bb[BB_NAMES].p + name_base[k], alns[k].names, name_base[k + 1] - name_base[k],
                          cudaMemcpyHostToDevice, st));
