@@ -1215,14 +1215,11 @@ cudaError_t launch_scan(const unsigned long long *in, unsigned long long *out, l
 }
 
 //------------------------------------------------------------------------------------------------ rows
-__device__ __forceinline__ int digits_of(long v)
+__device__ __forceinline__ int digits_of(long v)  // of 0 <= v < 2^31 (a sequence's number)
 {
-  int n = 1;
-  while (v >= 10) {
-    v /= 10;
-    n++;
-  }
-  return n;
+  const uint32_t u = (uint32_t)v;
+  return 1 + (u >= 10u) + (u >= 100u) + (u >= 1000u) + (u >= 10000u) + (u >= 100000u) + (u >= 1000000u) + (u >= 10000000u) +
+         (u >= 100000000u) + (u >= 1000000000u);
 }
 
 struct PairView {
@@ -1695,10 +1692,124 @@ struct Stager {
   }
 };
 
+// Lines in 8-byte words. A byte at a time (load a byte, store a byte) a line of 36 bytes took about 500 instructions of a
+// warp for 32 of them and 22.4 M of them 611-649 us; by words of 8 shifted into place 602 us, column numbers (-f csvn) 449 ->
+// 325 us per 1.6 M. What bounds it is latency: loading the next columns' codes and names early (more registers, 3 blocks
+// instead of 4 on an SM) took 687 us.
+constexpr int kLineName = 64;  // longest name (and start of a line) written by words
+
+// the end of a line as little-endian words: delimiter, distance, newline (16 bytes at most); bytes past n are zero
+struct LineEnd {
+  uint64_t lo, hi;
+  int n;
+};
+
+// any distance, by fmt_code (out of line: its scratch and the big-number conversion stay out of the writer's registers)
+__device__ __noinline__ LineEnd line_end_any(uint32_t code, double d, char delim)
+{
+  LineEnd e;
+  char g[24];
+  const int n = fmt_code(code, d, g);
+  e.lo = (unsigned char)delim;
+  e.hi = 0;
+  for (int k = 0; k <= n; k++) {
+    const uint64_t c = k < n ? (unsigned char)g[k] : 10u;
+    if (k < 7)
+      e.lo |= c << 8 * (k + 1);
+    else
+      e.hi |= c << 8 * (k - 7);
+  }
+  e.n = n + 2;
+  return e;
+}
+
+__device__ __forceinline__ LineEnd line_end(uint32_t code, double d, char delim)
+{
+  const int X = (int)((code >> 20) & 63u) - 16;
+  LineEnd e;
+  if (code >> 30 == 1 && X < 0 && X >= -4) {
+    // "0." , -X - 1 zeros, the digits without their trailing zeros. The six digits as bytes: q = 1000 a + b, both in
+    // 16-bit lanes, hundreds by 41 / 4096 and tens by 103 / 1024 (exact below 1,000 and below 100).
+    const uint32_t q = code & 0xFFFFFu, hi3 = q / 1000u, v = hi3 | (q - 1000u * hi3) << 16;
+    const uint32_t h = (v * 41u >> 12) & 0x000F000Fu, r = v - 100u * h, t = (r * 103u >> 10) & 0x000F000Fu, u = r - 10u * t;
+    const uint64_t D = (uint64_t)((h & 0xFFFFu) | (t & 0xFFFFu) << 8 | (u & 0xFFFFu) << 16) |
+                       (uint64_t)((h >> 16) | (t >> 16) << 8 | (u >> 16) << 16) << 24;
+    const int nd = (71 - __clzll((long long)D)) >> 3, z = -X - 1;
+    const uint64_t body = ((D | 0x303030303030ull) & ((1ull << 8 * nd) - 1)) | 10ull << 8 * nd;
+    const uint64_t pre = (uint64_t)(unsigned char)delim | 0x2E3000ull | (0x303030000000ull & ((1ull << 8 * (3 + z)) - 1));
+    const int s = 8 * (3 + z);
+    e.lo = pre | body << s;
+    e.hi = body >> (64 - s);
+    e.n = 3 + z + nd + 1;
+    return e;
+  }
+  return line_end_any(code, d, delim);
+}
+
+// a line byte by byte (out of line, as few lines come here)
+__device__ __noinline__ void put_line_bytes(char *o, const RowArgs &a, long i, long j, const LineEnd &e)
+{
+  char g[16];
+  for (int k = 0; k < e.n - 2; k++) g[k] = (char)((k < 7 ? e.lo >> 8 * (k + 1) : e.hi >> 8 * (k - 7)));
+  put_line(o, a, i, j, 0, a.names + a.name_off[i], a.name_len[i], g, e.n - 2);
+}
+
+// the decimal digits of v < 10^8, first digit in the low byte: four 2-digit lanes (100 by 5243 / 2^19, exact below 43,699;
+// 10 by 103 / 1024), leading zeros shifted out
+__device__ __forceinline__ uint64_t number_word(uint32_t v)
+{
+  const uint32_t a = v / 10000u, b = v - 10000u * a;
+  const uint32_t a1 = a * 5243u >> 19, b1 = b * 5243u >> 19;
+  const uint64_t t = (uint64_t)(a1 | (a - 100u * a1) << 16) | (uint64_t)(b1 | (b - 100u * b1) << 16) << 32;
+  const uint64_t u = (t * 103u >> 10) & 0x000F000F000F000Full;
+  const uint64_t d = u | (t - 10u * u) << 8;
+  const int z = v ? (__ffsll((long long)d) - 1) & ~7 : 56;
+  return (d | 0x3030303030303030ull) >> z;
+}
+
+// a stream of bytes on its way to aligned words: acc holds the s / 8 bytes of the word at p that came so far
+struct LineWords {
+  uint64_t *p, acc;
+  int s;
+  __device__ __forceinline__ void put8(uint64_t x)
+  {
+    *p++ = acc | x << s;
+    acc = x >> 1 >> (63 - s);
+  }
+  __device__ __forceinline__ void put(uint64_t x, int n)  // the n low bytes of x (1 to 8); the others are zero
+  {
+    acc |= x << s;
+    const int t = s + 8 * n;
+    if (t >= 64) {
+      *p++ = acc;
+      acc = x >> 1 >> (63 - s);
+    }
+    s = t & 63;
+  }
+  // n bytes (0 or more) from the unaligned address src, by the aligned words that hold them
+  __device__ __forceinline__ void put_name(const char *src, int n)
+  {
+    const uint64_t *q = reinterpret_cast<const uint64_t *>(reinterpret_cast<uintptr_t>(src) & ~(uintptr_t)7);
+    const int o = (int)(reinterpret_cast<uintptr_t>(src) & 7), words = (o + n + 7) >> 3, f = 8 * o;
+    uint64_t cur = words ? __ldg(q) : 0;
+    for (int left = n, k = 1; left > 0; left -= 8, k++) {
+      const uint64_t nxt = k < words ? __ldg(q + k) : 0;
+      const uint64_t x = cur >> f | nxt << 1 << (63 - f);
+      cur = nxt;
+      if (left >= 8)
+        put8(x);
+      else
+        put(x & ((1ull << 8 * left) - 1), left);
+    }
+  }
+};
+
 // one warp per (row, segment): the segment's text at its scanned offset (the row's self line in segment 0)
+template <bool DCODE>
 __device__ __forceinline__ void write_rows(const RowArgs &a, long bx, int sg)
 {
   __shared__ __align__(16) char stage[kWarps][kStage];
+  __shared__ uint64_t prefix[kWarps][kLineName / 8 + 1];
   const RunConsts &rc = a.rc;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long i = a.r0 + bx * kWarps + warp;
@@ -1748,25 +1859,42 @@ __device__ __forceinline__ void write_rows(const RowArgs &a, long bx, int sg)
     } else
       S.fill = sl;
   }
-  const int dli = rc.format == 1 ? digits_of(i) : 0;
+  // the lines' common start in words: name i (or its number) and a delimiter
+  const int n1 = (rc.format == 0 ? nli : digits_of(i)) + 1;
+  uint64_t *const pw = prefix[warp];
+  if (n1 <= kLineName) {
+    if (lane <= kLineName / 8) pw[lane] = 0;
+    __syncwarp();
+    char *const pc = reinterpret_cast<char *>(pw);
+    if (rc.format == 0) {
+      for (int k = lane; k < nli; k += 32) pc[k] = ni[k];
+    } else if (lane == 0) {
+      fmt_long(i, pc);
+    }
+    if (lane == 0) pc[n1 - 1] = rc.delim;
+    __syncwarp();
+  }
   for (long j0 = c0; j0 < c1; j0 += 32) {
     const long j = j0 + lane;
     double thisD = 0.;
     bool put;
     uint32_t code = 0;
-    if (a.dcode) {
+    if (DCODE) {
       // the stats kernel's code of this pair: printed or not, and its digits
       code = j < c1 ? a.dcode[(size_t)(i - a.r0) * a.ncols + (j - a.colbase)] : 0u;
       put = code != 0;
       if (put && (code >> 30) == 3u) linked_pair(a, i, j, thisD);
     } else {
       put = j < c1 && linked_pair(a, i, j, thisD);
+      int gl;
+      if (put) code = print_code(thisD, gl);
     }
-    char g[24];
-    int gl = 0, len = 0;
+    LineEnd e = {0, 0, 0};
+    int n2 = 0, len = 0;
     if (put) {
-      gl = a.dcode ? fmt_code(code, thisD, g) : fmt_g(thisD, g);
-      len = rc.format == 0 ? nli + a.name_len[j] + gl + 3 : dli + digits_of(j) + gl + 3;
+      e = line_end(code, thisD, rc.delim);
+      n2 = rc.format == 0 ? a.name_len[j] : digits_of(j);
+      len = n1 + n2 + e.n;
     }
     int pre = len;
     for (int o = 1; o < 32; o <<= 1) {
@@ -1776,19 +1904,44 @@ __device__ __forceinline__ void write_rows(const RowArgs &a, long bx, int sg)
     const int total = __shfl_sync(0xffffffffu, pre, 31);
     if (total == 0) continue;
     if (S.head + S.fill + total > kStage) S.flush(lane);
-    if (S.head + total > kStage) {
-      // a chunk larger than the staging buffer (very long names): write it in place
-      if (S.gpos + total > S.gend) {
-        S.over = true;
-        break;
+    const bool whole = S.head + total > kStage;  // larger than the staging buffer (very long names): written in place
+    if (whole && S.gpos + total > S.gend) {
+      S.over = true;
+      break;
+    }
+    const unsigned puts = __ballot_sync(0xffffffffu, put);
+    if (whole || n1 > kLineName || __any_sync(0xffffffffu, put && (n2 > (rc.format == 0 ? kLineName : 8) || len < 8))) {
+      if (put) {
+        put_line_bytes(whole ? (char *)(S.gpos + pre - len) : S.buf + S.head + S.fill + (pre - len), a, i, j, e);
       }
-      if (put) put_line((char *)(S.gpos + pre - len), a, i, j, 0, ni, nli, g, gl);
+    } else {
+      // Lines meet inside 8-byte words: a lane leaves the bytes before its line zero in its first word (the first lane
+      // keeps what stands there), and adds its own last bytes to the next lane's first word once that is stored. Lines of
+      // 8 bytes or more: a word holds bytes of two lines at most.
+      LineWords w;
+      if (put) {
+        const int at = S.head + S.fill + (pre - len);
+        w.p = reinterpret_cast<uint64_t *>(S.buf + (at & ~7));
+        w.s = 8 * (at & 7);
+        w.acc = (puts & lanemask_lt()) ? 0 : *w.p & ((1ull << w.s) - 1);
+        for (int k = 0; k < n1 >> 3; k++) w.put8(pw[k]);
+        if (n1 & 7) w.put(pw[n1 >> 3], n1 & 7);
+        if (rc.format == 0)
+          w.put_name(a.names + a.name_off[j], n2);
+        else
+          w.put(number_word((uint32_t)j), n2);
+        w.put(e.lo, min(e.n, 8));
+        if (e.n > 8) w.put(e.hi, e.n - 8);
+      }
       __syncwarp();
+      const bool last = lane == 31 - __clz(puts);
+      if (put && w.s) *w.p = last ? w.acc : *w.p | w.acc;
+    }
+    __syncwarp();
+    if (whole) {
       S.gpos += total;
       S.head = (int)(S.gpos & 15);
     } else {
-      if (put) put_line(S.buf + S.head + S.fill + (pre - len), a, i, j, 0, ni, nli, g, gl);
-      __syncwarp();
       S.fill += total;
     }
   }
@@ -1796,7 +1949,7 @@ __device__ __forceinline__ void write_rows(const RowArgs &a, long bx, int sg)
   if (S.over && lane == 0) atomicAdd(a.err, 1ull);
 }
 
-__global__ void __launch_bounds__(256, 4) write_kernel(RowArgs a) { write_rows(a, blockIdx.x, blockIdx.y); }
+__global__ void __launch_bounds__(256, 4) write_kernel(const __grid_constant__ RowArgs a) { write_rows<true>(a, blockIdx.x, blockIdx.y); }
 
 // Batched row stage: block b of the batch is row block blocks[b].y of alignment blocks[b].x; blockIdx.y is the
 // segment (blocks past an alignment's segment count exit).
@@ -1814,12 +1967,12 @@ __global__ void __launch_bounds__(256) sum_batch_kernel(const RowArgs *descs, co
   sum_rows(descs[B.x], B.y);
 }
 
-__global__ void __launch_bounds__(256) write_batch_kernel(const RowArgs *descs, const int2 *blocks)
+__global__ void __launch_bounds__(256, 3) write_batch_kernel(const RowArgs *descs, const int2 *blocks)
 {
   const int2 B = blocks[blockIdx.x];
   const RowArgs &a = descs[B.x];
   if ((long)blockIdx.y >= a.maxseg) return;
-  write_rows(a, B.y, blockIdx.y);
+  write_rows<false>(a, B.y, blockIdx.y);
 }
 
 // Per alignment of a batch (single-file runs, bin 0 only): links, skips and maximum over its (row, segment)
@@ -2784,7 +2937,7 @@ static int upload_set(tn93g_ctx *ctx, tn93g_set **out, const uint8_t *codes, cud
   };
   if ((e = take((void **)&s->d_codes, (size_t)N * L, 0)) != cudaSuccess) return fail(e);
   if ((e = take((void **)&s->d_counts, N * sizeof(long), 1)) != cudaSuccess) return fail(e);
-  if ((e = take((void **)&s->d_names, nbytes + 1, 2)) != cudaSuccess) return fail(e);
+  if ((e = take((void **)&s->d_names, nbytes + 8, 2)) != cudaSuccess) return fail(e);
   if ((e = take((void **)&s->d_name_off, N * sizeof(uint64_t), 3)) != cudaSuccess) return fail(e);
   if ((e = take((void **)&s->d_name_len, N * sizeof(int32_t), 4)) != cudaSuccess) return fail(e);
   if (codes_kind == cudaMemcpyHostToDevice) {
@@ -5278,7 +5431,7 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   }
   const size_t NR = row_base[K];
   TRY(ensure(ctx, bb[BB_CODES], code_off[K]));
-  TRY(ensure(ctx, bb[BB_NAMES], name_base[K] + 1));
+  TRY(ensure(ctx, bb[BB_NAMES], name_base[K] + 8));  // names are read by the aligned words that hold them
   TRY(ensure(ctx, bb[BB_NAMEOFF], NR * sizeof(uint64_t)));
   TRY(ensure(ctx, bb[BB_NAMELEN], NR * sizeof(int32_t)));
   TRY(ensure(ctx, bb[BB_COUNTS], NR * sizeof(long)));
