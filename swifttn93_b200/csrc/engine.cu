@@ -2164,13 +2164,14 @@ bool pair_split(const PairArgs &A)
 // a warp's pairs belong to one or two units. Long segments and several rows keep the atomics of a warp's totals rare (22.4 M
 // pairs: 0.85 ms with 1,024 columns, 0.90 with 512); small launches take shorter segments, down to 128 columns, so that the
 // SMs have two waves of warps (1,801 x 1,203 in bands of 0.2-0.4 M pairs: 0.10 -> 0.05 ms a band), and rows are added up
-// only past four waves.
+// only past four waves, strips past one (a strip's row has few pairs, and its warp four atomics on its query's words: 32
+// columns x 30,000 rows 109 us with a row to a warp, 59 us with 8).
 void formula_shape(long nrows, long ncols, bool units, int &segw, int &rpw)
 {
   segw = units ? 32 : kSeg;
   while (segw > 128 && nrows * ((ncols + segw - 1) / segw) < 148 * 48) segw /= 2;
   const long nseg = (ncols + segw - 1) / segw;
-  rpw = (int)std::max<long>(1, std::min<long>(1024 / std::min<long>(segw, ncols), nrows * nseg / (148 * 128)));
+  rpw = (int)std::max<long>(1, std::min<long>(1024 / std::min<long>(segw, ncols), nrows * nseg / (148 * (units ? 24 : 128))));
 }
 
 // The pair stage of rows [A.r0, A.r1) and the columns from A.cstart (32 ncolblocks of them). Fused kernel: 4 resident
@@ -4482,7 +4483,7 @@ __global__ void __launch_bounds__(256) qwrite_kernel(RowArgs a)
 // added in row order, as tn93's writer adds them (swifttn93.cpp:2838-2848). One block per query. Only bin 0 is used in a
 // server batch (no -m).
 __global__ void __launch_bounds__(512) query_reduce_kernel(RowArgs a, int nq, double *qout /* [nq][9] */,
-                                                           long long *qlinks /* [nq][2] */)
+                                                           long long *qlinks /* [nq][3]: links, skips, text offset */)
 {
   __shared__ long long rl[16], rs[16];
   __shared__ double rm[16];
@@ -4520,8 +4521,9 @@ __global__ void __launch_bounds__(512) query_reduce_kernel(RowArgs a, int nq, do
     o[1] = o[2] = 0.;
     o[4] = o[5] = 0.;
     o[7] = o[8] = 0.;
-    qlinks[q * 2] = links;
-    qlinks[q * 2 + 1] = skipped;
+    qlinks[q * 3] = links;
+    qlinks[q * 3 + 1] = skipped;
+    qlinks[q * 3 + 2] = (long long)a.seg_off[base];
   }
 }
 
@@ -4542,8 +4544,10 @@ struct tn93g_server {
   bool tc = false;
   bool lin = false;  // the records hold the ambiguity codes (average, gapmm, skip)
   int tc16 = 0;
-  long tc_NB = 0, tc_KS = 0;
+  long tc_NB = 0, tc_KS = 0, tc_chunk = 0;
   DevBuf ohimg, tcagg, tcerr;
+  void *hstat = nullptr;  // a batch's statistics in host memory that the device maps
+  size_t hstat_n = 0;
   // exactness: the undecided list (capacity und_cap entries; grown for an exact-sums pass), its count, the
   // per-query bounds, the query of each column, the replay descriptor the resolver reads
   DevBuf und, undn, amb, colunit, rdesc;
@@ -4552,8 +4556,14 @@ struct tn93g_server {
 };
 
 namespace {
-constexpr long kServerTcChunk = 128;  // query columns per tensor-core count launch (a multiple of 64): the
-                                      // records of a 30,000-sequence reference x 128 columns (61 MB) stay in L2
+// Query columns per chunk of the tensor-core records (counts, events, formula), a multiple of 64; chunks end on the count
+// kernel's 64-column tiles. 40 queries (1,280 columns) against 30,000 sequences, pair stage:
+// 5.03 ms with chunks of 128 from the reference's last row (three 64-column tiles each), 3.91 so.
+constexpr long kServerTcChunk = 512, kServerTcChunkMin = 128;
+
+// words of the statistics of a batch of nq queries: total, undecided, counters, error word, and per query 9 sums, 3 counts,
+// 4 bounds and the histogram
+size_t server_stats(size_t nq) { return 7 + nq * (9 + 3 + 4 + 3 * kHistBins); }
 
 // opt-in to the count kernel's dynamic shared memory on the current device
 int tc_attr(tn93g_ctx *ctx)
@@ -4582,6 +4592,7 @@ void tn93g_server_destroy(tn93g_server *srv)
       if (ctx) ctx->used -= b->n;
     }
   if (srv->pin) cudaFreeHost(srv->pin);
+  if (srv->hstat) cudaFreeHost(srv->hstat);
   delete srv;
 }
 
@@ -4759,7 +4770,8 @@ int tn93g_server_create(tn93g_ctx *ctx, tn93g_server **out, const uint8_t *codes
     SV(ensure(ctx, srv->total, sizeof(unsigned long long)));
     SV(ensure(ctx, srv->segcols, (nq + 1) * sizeof(long)));
     SV(ensure(ctx, srv->qout, (size_t)nq * 9 * sizeof(double)));
-    SV(ensure(ctx, srv->qlinks, (size_t)nq * 2 * sizeof(long long)));
+    SV(ensure(ctx, srv->qlinks, (size_t)nq * 3 * sizeof(long long)));
+    SV(ensure_pinned_at(ctx, srv->hstat, srv->hstat_n, server_stats(nq) * sizeof(unsigned long long), cudaHostAllocMapped));
     SV(ensure(ctx, srv->scantmp, (2 * (nslot / kScanTile + 1) + 1) * sizeof(unsigned long long)));
     srv->und_cap = (unsigned)std::min<size_t>(std::max<size_t>(4096, dslots / 64), 0xFFFFFFF0u);
     SV(ensure(ctx, srv->und, (size_t)srv->und_cap * 2 * sizeof(unsigned long long)));
@@ -4781,8 +4793,15 @@ int tn93g_server_create(tn93g_ctx *ctx, tn93g_server **out, const uint8_t *codes
     srv->tc_KS = (L + kTcStageK - 1) / kTcStageK;
     srv->tc16 = 32 * L < 65536;
     const size_t img = (size_t)srv->tc_KS * srv->tc_NB * kTcBlockBytes;
-    const size_t agg = (size_t)N * kServerTcChunk * (srv->tc16 ? 16 : 32);
-    if (ensure(ctx, srv->ohimg, img) == TN93G_OK && ensure(ctx, srv->tcagg, agg) == TN93G_OK &&
+    // a chunk that holds the largest batch from any first column, or the smallest one where that does not fit
+    srv->tc_chunk = std::min<long>(kServerTcChunk, std::max(kServerTcChunkMin, (max_batch_sequences + 127) / 64 * 64));
+    const size_t agg = (size_t)N * (srv->tc16 ? 16 : 32);
+    const bool room = ensure(ctx, srv->ohimg, img) == TN93G_OK;
+    if (room && ensure(ctx, srv->tcagg, agg * srv->tc_chunk) != TN93G_OK) {
+      cudaGetLastError();
+      srv->tc_chunk = kServerTcChunkMin;
+    }
+    if (room && ensure(ctx, srv->tcagg, agg * srv->tc_chunk) == TN93G_OK &&
         ensure(ctx, srv->tcerr, sizeof(unsigned long long)) == TN93G_OK) {
       srv->tc = true;
       srv->lin = weighted_mode(opts->mode);
@@ -4846,11 +4865,11 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
   std::vector<int32_t> nl(Q);
   std::vector<long> cnt(Q);
   size_t nb = srv->names_ref;
-  std::vector<size_t> qname_base(nq);
+  std::string qnames;  // the queries' names, one after the other
   for (int q = 0; q < nq; q++) {
     size_t qn = 0;
     for (long k = 0; k < queries[q].n; k++) qn = std::max(qn, queries[q].name_off[k] + (size_t)queries[q].name_len[k]);
-    qname_base[q] = nb;
+    qnames.append(queries[q].names, qn);
     for (long k = 0; k < queries[q].n; k++) {
       off[qstart[q] + k] = nb + queries[q].name_off[k];
       nl[qstart[q] + k] = (int32_t)queries[q].name_len[k];
@@ -4863,10 +4882,9 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
   for (int q = 0; q < nq; q++) {
     CU(cudaMemcpyAsync((uint8_t *)srv->qcodes.p + (size_t)qstart[q] * L, queries[q].codes, (size_t)queries[q].n * L,
                        cudaMemcpyHostToDevice, st));
-    size_t qn = 0;
-    for (long k = 0; k < queries[q].n; k++) qn = std::max(qn, queries[q].name_off[k] + (size_t)queries[q].name_len[k]);
-    if (qn) CU(cudaMemcpyAsync((char *)srv->names.p + qname_base[q], queries[q].names, qn, cudaMemcpyHostToDevice, st));
   }
+  if (!qnames.empty())
+    CU(cudaMemcpyAsync((char *)srv->names.p + srv->names_ref, qnames.data(), qnames.size(), cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync((uint64_t *)srv->name_off.p + Nref, off.data(), Q * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync((int32_t *)srv->name_len.p + Nref, nl.data(), Q * sizeof(int32_t), cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync((long *)srv->counts.p + Nref, cnt.data(), Q * sizeof(long), cudaMemcpyHostToDevice, st));
@@ -4985,8 +5003,8 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
     A.ex = ex;
     if (srv->tc) {
       // per chunk of query columns: counts on the tensor cores, then the pair kernel
-      for (long c0 = Nref; c0 < Nref + Q; c0 += kServerTcChunk) {
-        const long c1 = std::min(Nref + Q, c0 + kServerTcChunk);
+      for (long c0 = Nref, c1; c0 < Nref + Q; c0 = c1) {
+        c1 = std::min(Nref + Q, c0 / kTcCols * kTcCols + srv->tc_chunk);
         TcArgs T;
         T.onehot = (const uint8_t *)srv->ohimg.p;
         T.NB = srv->tc_NB;
@@ -4996,7 +5014,7 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
         T.cross = true;
         T.r0 = 0;
         T.r1 = Nref;
-        T.ncols = kServerTcChunk;
+        T.ncols = srv->tc_chunk;
         T.colbase = c0;
         T.cstart = c0 / kTcCols * kTcCols;
         T.cend = c1;
@@ -5010,7 +5028,7 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
         PairArgs AC = A;
         AC.tcagg = srv->tcagg.p;
         AC.tc16 = srv->tc16;
-        AC.tcncols = kServerTcChunk;
+        AC.tcncols = srv->tc_chunk;
         AC.tccolbase = c0;
         AC.cstart = c0;
         CU(launch_pair(AC, (c1 - c0 + 31) / 32, Nref, st));
@@ -5069,9 +5087,9 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
   const dim3 g2((unsigned)((Nref + 255) / 256), (unsigned)nq);
   unsigned long long total = 0, und = 0;
   std::vector<double> qo((size_t)nq * 9);
-  std::vector<long long> ql((size_t)nq * 2);
+  std::vector<long long> ql((size_t)nq * 3);
   std::vector<unsigned long long> qoff(nq + 1), hist((size_t)nq * 3 * kHistBins), ambw((size_t)nq * 4);
-  unsigned long long counters[4];
+  unsigned long long counters[4], tcerr = 0;
   // row stage (per-query statistics and row sums, scan, per-query reduction) and its results on the host
   auto rows_and_read = [&]() -> int {
     CU(cudaMemsetAsync(srv->hist.p, 0, (size_t)nq * 3 * kHistBins * sizeof(unsigned long long), st));
@@ -5085,17 +5103,44 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
     CU(cudaGetLastError());
     ctx->launches++;
     CU(cudaEventRecord(E[4], st));
-    CU(cudaMemcpyAsync(&total, srv->total.p, sizeof total, cudaMemcpyDeviceToHost, st));
-    CU(cudaMemcpyAsync(qo.data(), srv->qout.p, qo.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CU(cudaMemcpyAsync(ql.data(), srv->qlinks.p, ql.size() * sizeof(long long), cudaMemcpyDeviceToHost, st));
-    for (int q = 0; q < nq; q++)
-      CU(cudaMemcpyAsync(&qoff[q], (unsigned long long *)srv->soff.p + (size_t)q * Nref, sizeof(unsigned long long),
-                         cudaMemcpyDeviceToHost, st));
-    CU(cudaMemcpyAsync(hist.data(), srv->hist.p, hist.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                       st));
-    CU(cudaMemcpyAsync(counters, srv->counters.p, sizeof counters, cudaMemcpyDeviceToHost, st));
-    CU(cudaMemcpyAsync(&und, srv->undn.p, sizeof und, cudaMemcpyDeviceToHost, st));
+    // the statistics to the host in one kernel (a copy of a few words to pageable memory takes about 10 us; there were
+    // six of them and one a query: 0.5 ms for 40 queries)
+    unsigned long long *dst = nullptr;
+    CU(cudaHostGetDevicePointer((void **)&dst, srv->hstat, 0));
+    Gather g;
+    g.k = 0;
+    auto add = [&](const void *src, size_t nwords) {
+      g.src[g.k] = (const unsigned long long *)src;
+      g.dst[g.k] = dst;
+      g.n[g.k++] = (long)nwords;
+      dst += nwords;
+    };
+    add(srv->total.p, 1);
+    add(srv->undn.p, 1);
+    add(srv->counters.p, 4);
+    if (srv->tc) add(srv->tcerr.p, 1);
+    add(srv->qout.p, qo.size());
+    add(srv->qlinks.p, ql.size());
+    add(srv->amb.p, ambw.size());
+    add(srv->hist.p, hist.size());
+    gather_kernel<<<16, 256, 0, st>>>(g);
+    CU(cudaGetLastError());
+    ctx->launches++;
     CU(cudaStreamSynchronize(st));
+    const unsigned long long *h = (const unsigned long long *)srv->hstat;
+    auto take = [&](void *to, size_t nwords) {
+      memcpy(to, h, nwords * sizeof *h);
+      h += nwords;
+    };
+    take(&total, 1);
+    take(&und, 1);
+    take(counters, 4);
+    if (srv->tc) take(&tcerr, 1);
+    take(qo.data(), qo.size());
+    take(ql.data(), ql.size());
+    take(ambw.data(), ambw.size());
+    take(hist.data(), hist.size());
+    for (int q = 0; q < nq; q++) qoff[q] = (unsigned long long)ql[q * 3 + 2];
     return TN93G_OK;
   };
   // finishes the listed undecided pairs with the C library's logarithms and runs the row stage again
@@ -5113,13 +5158,9 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
   };
   TRY(enqueue_pairs(false));
   TRY(rows_and_read());
-  if (srv->tc) {
-    unsigned long long tcerr = 0;
-    CU(cudaMemcpy(&tcerr, srv->tcerr.p, sizeof tcerr, cudaMemcpyDeviceToHost));
-    if (tcerr) {
-      ctx->err = "the tensor-core count kernel timed out waiting for its pipeline";
-      return TN93G_ETIMEOUT;
-    }
+  if (tcerr) {
+    ctx->err = "the tensor-core count kernel timed out waiting for its pipeline";
+    return TN93G_ETIMEOUT;
   }
   const long ambiguous0 = (long)counters[0];
   // more undecided pairs than the list holds: grow it and run the batch's pair stage again (the same pairs are
@@ -5135,15 +5176,14 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
   if (und > srv->und_cap) TRY(grow_and_rerun(false));
   if (und) TRY(resolve_and_reread());
   // per query: the JSON numbers certain for every rounding of the C library's log, or an exact-sums pass
-  CU(cudaMemcpy(ambw.data(), srv->amb.p, ambw.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
   std::vector<tn93g_summary> S(nq);
   auto fill_summaries = [&]() {
     for (int q = 0; q < nq; q++) {
       tn93g_summary &X = S[q];
       memset(&X, 0, sizeof X);
       X.pairwise = (unsigned long)Nref * (unsigned long)queries[q].n;
-      X.links = (long)ql[q * 2];
-      X.skipped = (long)ql[q * 2 + 1];
+      X.links = (long)ql[q * 3];
+      X.skipped = (long)ql[q * 3 + 1];
       for (int k = 0; k < 3; k++) {
         X.max[k] = qo[q * 9 + k];
         X.mean[k] = qo[q * 9 + 3 + k];
@@ -5187,10 +5227,11 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
     ctx->launches++;
     CU(cudaEventRecord(E[5], st));
     CU(cudaMemcpyAsync(srv->pin, srv->out.p, total, cudaMemcpyDeviceToHost, st));
-    CU(cudaMemcpyAsync(&counters[3], (unsigned long long *)srv->counters.p + 3, sizeof(unsigned long long),
+    CU(cudaMemcpyAsync(srv->hstat, (unsigned long long *)srv->counters.p + 3, sizeof(unsigned long long),
                        cudaMemcpyDeviceToHost, st));
     CU(cudaEventRecord(E[6], st));
     CU(cudaStreamSynchronize(st));
+    memcpy(&counters[3], srv->hstat, sizeof counters[3]);
     float ms = 0.f;
     CU(cudaEventElapsedTime(&ms, E[4], E[5]));
     ctx->timings[4] = ms;
@@ -5438,20 +5479,21 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   std::vector<uint64_t> noff(NR);
   std::vector<int32_t> nlen(NR);
   std::vector<long> cnts(NR);
+  std::string names;  // the alignments' names, one after the other: one copy
+  names.reserve(name_base[K]);
   std::vector<HostSpan> spans;
   for (int k = 0; k < K; k++)
     spans.push_back({(uint8_t *)bb[BB_CODES].p + code_off[k], alns[k].codes, code_off[k + 1] - code_off[k]});
   TRY(upload_host(ctx, spans));
   for (int k = 0; k < K; k++) {
-    if (name_base[k + 1] > name_base[k])
-      CU(cudaMemcpyAsync((char *)bb[BB_NAMES].p + name_base[k], alns[k].names, name_base[k + 1] - name_base[k],
-                         cudaMemcpyHostToDevice, st));
+    names.append(alns[k].names, name_base[k + 1] - name_base[k]);
     for (long i = 0; i < alns[k].n; i++) {
       noff[row_base[k] + i] = name_base[k] + alns[k].name_off[i];
       nlen[row_base[k] + i] = (int32_t)alns[k].name_len[i];
       cnts[row_base[k] + i] = alns[k].copy_counts[i];
     }
   }
+  if (!names.empty()) CU(cudaMemcpyAsync(bb[BB_NAMES].p, names.data(), names.size(), cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(bb[BB_NAMEOFF].p, noff.data(), NR * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(bb[BB_NAMELEN].p, nlen.data(), NR * sizeof(int32_t), cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(bb[BB_COUNTS].p, cnts.data(), NR * sizeof(long), cudaMemcpyHostToDevice, st));
