@@ -2320,6 +2320,9 @@ struct tn93g_ctx {
   size_t pin2_n[2] = {0, 0};
   void *pstats = nullptr;
   size_t pstats_n = 0;
+  std::string tab_key;   // what agg and site hold (run_impl; empty: nothing)
+  void *hrun = nullptr;  // pinned block of a run's small transfers
+  size_t hrun_n = 0;
   void *upload_pin = nullptr;  // upload_host's pieces (two a thread) and the events of their copies
   cudaEvent_t upload_ev[8] = {nullptr};
   // device buffers of freed sets, kept for the next upload (repeated upload/free skips the allocator)
@@ -2330,13 +2333,13 @@ struct tn93g_ctx {
   DevBuf bb[kBatchBufs];  // buffers of tn93g_batch_run (indexed by BatchBuf)
   int count_path = 1;  // clean-site counts: 0 popcounts on the CUDA cores, 1 tensor cores (tcgen05)
   int sms = 148;       // streaming multiprocessors of the device (persistent and grid-stride launches)
-  DevBuf ohimg, tcagg, tcerr;
+  DevBuf ohimg, tcagg;
   uint64_t wait_ns = kTcWaitNs;  // limit of each bounded device wait
   bool exact_sums = false;       // tn93g_set_exact_sums
   int fault = TN93G_FAULT_NONE;  // test hook for the next run (tn93g_inject_fault)
   // exactness: undecided lists and counts per band parity, the summary units' bounds, the resolver's entries and
   // run descriptors, and the logarithm's band and candidate spread (tn93g_set_log_band)
-  DevBuf und[2], undn, amb, undwork, rdesc;
+  DevBuf und[2], undn, undwork, rdesc;
   double log_band = kLogBand, log_spread = kLogSpread;
 };
 
@@ -2856,7 +2859,7 @@ void tn93g_destroy(tn93g_ctx *ctx)
     if (b->p) cudaFree(b->p);
   for (DevBuf &b : ctx->bb)
     if (b.p) cudaFree(b.p);
-  for (DevBuf *b : {&ctx->ohimg, &ctx->tcagg, &ctx->tcerr, &ctx->und[0], &ctx->und[1], &ctx->undn, &ctx->amb,
+  for (DevBuf *b : {&ctx->ohimg, &ctx->tcagg, &ctx->und[0], &ctx->und[1], &ctx->undn,
                     &ctx->undwork, &ctx->rdesc})
     if (b->p) cudaFree(b->p);
   if (ctx->d_logt) cudaFree(ctx->d_logt);
@@ -2872,6 +2875,7 @@ void tn93g_destroy(tn93g_ctx *ctx)
       if (e) cudaEventDestroy(e);
   }
   if (ctx->total.p) cudaFree(ctx->total.p);
+  if (ctx->hrun) cudaFreeHost(ctx->hrun);
   if (ctx->upload_pin) cudaFreeHost(ctx->upload_pin);
   for (cudaEvent_t e : ctx->upload_ev)
     if (e) cudaEventDestroy(e);
@@ -3252,6 +3256,9 @@ int tn93g_run_to_device(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn9
   return rc;
 }
 
+constexpr size_t kRunScalars = 17;       // words of a run's scalars (run_impl)
+constexpr size_t kRunPinned = 4 << 20;  // pinned bytes kept for a run's small transfers
+
 static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_opts *opts, tn93g_sink sink, void *user,
                     tn93g_summary *sum, bool to_device, long row_begin, long row_end, double *row_sums, int flags)
 {
@@ -3292,24 +3299,42 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   CU(cudaEventRecord(E[0], st));
 
   //------------------------------------------------------------------ pack
-  TRY(ensure(ctx, ctx->seen, L * sizeof(uint32_t)));
-  TRY(ensure(ctx, ctx->nN, sizeof(unsigned long long)));
-  CU(cudaMemsetAsync(ctx->seen.p, 0, L * sizeof(uint32_t), st));
-  CU(cudaMemsetAsync(ctx->nN.p, 0, sizeof(unsigned long long), st));
+  // The host's side of the small transfers: one pinned block (a copy to or from pageable memory costs about 10 us more), or
+  // pageable memory for very long or many sequences. The device's scalars and column masks are each one buffer, cleared
+  // and copied in one piece.
+  const size_t seen_n = ((size_t)L * sizeof(uint32_t) + 7) / 8 * 8 + sizeof(unsigned long long);  // masks, then the N count
+  const size_t host_part[6] = {seen_n, (size_t)L * sizeof(int32_t), N * sizeof(uint32_t), (N + 1) * sizeof(uint32_t),
+                               N * sizeof(uint32_t), (N + 1) * sizeof(uint32_t)};
+  size_t host_at[7] = {kRunScalars * sizeof(unsigned long long)};
+  for (int q = 0; q < 6; q++) host_at[q + 1] = (host_at[q] + host_part[q] + 7) / 8 * 8;
+  std::vector<char> host_big;
+  char *host = nullptr;
+  if (host_at[6] <= kRunPinned) {
+    TRY(ensure_pinned_at(ctx, ctx->hrun, ctx->hrun_n, kRunPinned));
+    host = (char *)ctx->hrun;
+  } else {
+    host_big.resize(host_at[6]);
+    host = host_big.data();
+  }
+  unsigned long long *const h_scalars = (unsigned long long *)host;
+  const uint32_t *const seen = (const uint32_t *)(host + host_at[0]);
+  int32_t *const h_varcol = (int32_t *)(host + host_at[1]);
+  uint32_t *const evc = (uint32_t *)(host + host_at[2]), *const evoff = (uint32_t *)(host + host_at[3]);
+  uint32_t *const wcnt = (uint32_t *)(host + host_at[4]), *const woff = (uint32_t *)(host + host_at[5]);
+  TRY(ensure(ctx, ctx->seen, seen_n));
+  CU(cudaMemsetAsync(ctx->seen.p, 0, seen_n, st));
   {
     dim3 g((unsigned)((L + 255) / 256), (unsigned)((N + 63) / 64));
-    colscan_kernel<<<g, 256, 0, st>>>(set->d_codes, N, L, (uint32_t *)ctx->seen.p, (unsigned long long *)ctx->nN.p);
+    colscan_kernel<<<g, 256, 0, st>>>(set->d_codes, N, L, (uint32_t *)ctx->seen.p,
+                                      (unsigned long long *)((char *)ctx->seen.p + seen_n) - 1);
     CU(cudaGetLastError());
     ctx->launches++;
   }
-  std::vector<uint32_t> seen(L);
-  unsigned long long nN = 0;
-  CU(cudaMemcpyAsync(seen.data(), ctx->seen.p, L * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  CU(cudaMemcpyAsync(&nN, ctx->nN.p, sizeof nN, cudaMemcpyDeviceToHost, st));
+  CU(cudaMemcpyAsync(host + host_at[0], ctx->seen.p, seen_n, cudaMemcpyDeviceToHost, st));
   CU(cudaStreamSynchronize(st));
+  const unsigned long long nN = *((const unsigned long long *)(host + host_at[0] + seen_n) - 1);
   // a column is constant when every sequence has the same clean base there: each pair gets (b, b)
-  std::vector<int32_t> varcol;
-  varcol.reserve(L);
+  long Lc = 0;
   bool three = false;
   for (long p = 0; p < L; p++) {
     const uint32_t m = seen[p];
@@ -3320,9 +3345,8 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
       rc.constNf[b] += 2;
       rc.constCnt[b]++;
     } else
-      varcol.push_back((int32_t)p);
+      h_varcol[Lc++] = (int32_t)p;
   }
-  const long Lc = (long)varcol.size();
   const long W = (Lc + 63) / 64;
   const long Npad = (N + 31) / 32 * 32;
   rc.Lc = Lc;
@@ -3338,7 +3362,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   TRY(ensure(ctx, ctx->evcount, N * sizeof(uint32_t)));
   TRY(ensure(ctx, ctx->evoff, (N + 1) * sizeof(uint32_t)));
   TRY(ensure(ctx, ctx->three, N));
-  if (Lc) CU(cudaMemcpyAsync(ctx->varcol.p, varcol.data(), Lc * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+  if (Lc) CU(cudaMemcpyAsync(ctx->varcol.p, h_varcol, Lc * sizeof(int32_t), cudaMemcpyHostToDevice, st));
   CU(cudaMemsetAsync(ctx->planes.p, 0, (size_t)std::max<long>(W, 1) * rc.NP * Npad * sizeof(uint64_t), st));
   CU(cudaMemsetAsync(ctx->evcount.p, 0, N * sizeof(uint32_t), st));
   PackArgs pa;
@@ -3372,21 +3396,17 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   const bool use_ev = !lin || (three && opts->mode != TN93G_SKIP);  // events are needed: all, or for three-fold codes
   // per sequence, its nonzero N-plane words (the pair kernel's sparse N-plane pass); counted here, listed below
   bool sparse_w = rc.wplane && W > 0 && (!lin || rc.gapmm);
-  std::vector<uint32_t> wcnt;
   if (sparse_w) {
     TRY(ensure(ctx, ctx->wcount, N * sizeof(uint32_t)));
     wcount_kernel<<<(unsigned)((N + 31) / 32), 32 * kWlWarps, 0, st>>>((const uint64_t *)ctx->planes.p, N, W, rc.NP, Npad,
                                                                 (uint32_t *)ctx->wcount.p);
     CU(cudaGetLastError());
     ctx->launches++;
-    wcnt.resize(N);
-    CU(cudaMemcpyAsync(wcnt.data(), ctx->wcount.p, N * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    CU(cudaMemcpyAsync(wcnt, ctx->wcount.p, N * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   }
-  std::vector<uint32_t> evc(N), evoff(N + 1);
-  if (use_ev) CU(cudaMemcpyAsync(evc.data(), ctx->evcount.p, N * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  if (use_ev) CU(cudaMemcpyAsync(evc, ctx->evcount.p, N * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   if (use_ev || sparse_w) CU(cudaStreamSynchronize(st));
   if (sparse_w) {
-    std::vector<uint32_t> woff(N + 1);
     unsigned long long t = 0;
     for (long i = 0; i < N; i++) {
       woff[i] = (uint32_t)t;
@@ -3397,26 +3417,24 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
       woff[N] = (uint32_t)t;
       TRY(ensure(ctx, ctx->wloff, (N + 1) * sizeof(uint32_t)));
       TRY(ensure(ctx, ctx->wl, std::max<size_t>(t, 1) * sizeof(uint32_t)));
-      CU(cudaMemcpyAsync(ctx->wloff.p, woff.data(), (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+      CU(cudaMemcpyAsync(ctx->wloff.p, woff, (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
       wlist_kernel<<<(unsigned)((N + 31) / 32), 32 * kWlWarps, 0, st>>>((const uint64_t *)ctx->planes.p, N, W, rc.NP, Npad,
                                                                  (const uint32_t *)ctx->wloff.p, (uint32_t *)ctx->wl.p);
       CU(cudaGetLastError());
       ctx->launches++;
-      // the host copy must outlive the asynchronous upload
-      CU(cudaStreamSynchronize(st));
     }
   }
   evoff[0] = 0;
   uint32_t max_ev = 0;
   for (long i = 0; i < N; i++) {
-    const uint32_t n = pad_events(evc[i]);
+    const uint32_t n = use_ev ? pad_events(evc[i]) : 0;
     evoff[i + 1] = evoff[i] + n;
     max_ev = std::max(max_ev, n);
   }
   rc.packed = max_ev <= (uint32_t)kPackedMaxEvents;
   TRY(ensure(ctx, ctx->ev, std::max<size_t>(evoff[N], 1) * sizeof(uint32_t)));
   TRY(ensure(ctx, ctx->ev2, std::max<size_t>(evoff[N], 1) * sizeof(uint2)));
-  CU(cudaMemcpyAsync(ctx->evoff.p, evoff.data(), (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+  CU(cudaMemcpyAsync(ctx->evoff.p, evoff, (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
   pa.ev = (uint32_t *)ctx->ev.p;
   pa.ev2 = (uint2 *)ctx->ev2.p;
   pa.ev2_Npad = (uint32_t)Npad;
@@ -3425,20 +3443,25 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     CU(cudaGetLastError());
     ctx->launches++;
   }
-  // tables of this mode
-  build_tables(ctx->h_tab, opts->mode, opts->subset);
-  fill_pair_tables(*ctx->h_tab, rc.wplane, ctx->h_ptab);
-  TRY(ensure(ctx, ctx->agg, sizeof(PairTables)));
-  TRY(ensure(ctx, ctx->site, sizeof(ctx->h_tab->site)));
-  CU(cudaMemcpyAsync(ctx->agg.p, ctx->h_ptab, sizeof(PairTables), cudaMemcpyHostToDevice, st));
-  CU(cudaMemcpyAsync(ctx->site.p, ctx->h_tab->site, sizeof(ctx->h_tab->site), cudaMemcpyHostToDevice, st));
+  // tables of this mode: they depend on the mode, the subset of codes and the N plane alone, so the last run's stay on the
+  // device until a run needs others (with the small transfers above, building and copying them took 0.15 of the 0.49 ms of a 50 x 900 run)
+  std::string tab_key(1, (char)(2 * opts->mode + (rc.wplane ? 1 : 0)));
+  if (opts->mode == TN93G_SUBSET) tab_key.append((const char *)opts->subset, sizeof opts->subset);
+  if (tab_key != ctx->tab_key) {
+    ctx->tab_key.clear();
+    build_tables(ctx->h_tab, opts->mode, opts->subset);
+    fill_pair_tables(*ctx->h_tab, rc.wplane, ctx->h_ptab);
+    TRY(ensure(ctx, ctx->agg, sizeof(PairTables)));
+    TRY(ensure(ctx, ctx->site, sizeof(ctx->h_tab->site)));
+    CU(cudaMemcpyAsync(ctx->agg.p, ctx->h_ptab, sizeof(PairTables), cudaMemcpyHostToDevice, st));
+    CU(cudaMemcpyAsync(ctx->site.p, ctx->h_tab->site, sizeof(ctx->h_tab->site), cudaMemcpyHostToDevice, st));
+    ctx->tab_key = tab_key;
+  }
   // tensor-core count path: the one-hot operand image of every sequence (an extra 32-sequence block at the end,
   // which the last 64-column tile reads)
   const long tc_NB = (N + 31) / 32 + 1, tc_KS = (Lc + kTcStageK - 1) / kTcStageK;
   if (use_tc) {
     TRY(ensure(ctx, ctx->ohimg, (size_t)tc_KS * tc_NB * kTcBlockBytes));
-    TRY(ensure(ctx, ctx->tcerr, sizeof(unsigned long long)));
-    CU(cudaMemsetAsync(ctx->tcerr.p, 0, sizeof(unsigned long long), st));
     const long nthr = tc_NB * 32 * tc_KS * (kTcStageK / 16);
     onehot_kernel<<<(unsigned)((nthr + 255) / 256), 256, 0, st>>>((const uint8_t *)ctx->cc.p, N, Lc, tc_NB, tc_KS,
                                                                   (uint8_t *)ctx->ohimg.p, 0, tc_NB * 32,
@@ -3573,15 +3596,15 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   };
   TRY(size_buffers(0));
   TRY(ensure(ctx, ctx->rqn, sizeof(unsigned)));
-  TRY(ensure(ctx, ctx->counters, 4 * sizeof(unsigned long long)));
+  // the run's scalars: 4 counters, the 3 summary units' bounds (4 words each), the count kernel's error word
+  TRY(ensure(ctx, ctx->counters, kRunScalars * sizeof(unsigned long long)));
+  CU(cudaMemsetAsync(ctx->counters.p, 0, kRunScalars * sizeof(unsigned long long), st));
+  unsigned long long *const d_amb = (unsigned long long *)ctx->counters.p + 4, *const d_tcerr = d_amb + 12;
   // per band parity: its histogram (added on the host, so a band's row stage can run again), its undecided list
   TRY(ensure(ctx, ctx->hist, 2 * 3 * kHistBins * sizeof(unsigned long long)));
   TRY(ensure(ctx, ctx->total, 2 * sizeof(unsigned long long)));
   TRY(ensure(ctx, ctx->undn, 2 * sizeof(unsigned long long)));
-  TRY(ensure(ctx, ctx->amb, 3 * 4 * sizeof(unsigned long long)));
   TRY(ensure(ctx, ctx->rdesc, 2 * sizeof(ReplayArgs)));
-  CU(cudaMemsetAsync(ctx->amb.p, 0, 3 * 4 * sizeof(unsigned long long), st));
-  CU(cudaMemsetAsync(ctx->counters.p, 0, 4 * sizeof(unsigned long long), st));
   double max_[3] = {0, 0, 0}, mean[3] = {0, 0, 0}, wc[3] = {0, 0, 0};
   unsigned long long hist_total[3 * kHistBins];
   memset(hist_total, 0, sizeof hist_total);
@@ -3676,7 +3699,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     add(RA.hist, h.hist, 3 * kHistBins);
     add((unsigned long long *)ctx->undn.p + par, h.und, 1);
     if (use_tc)
-      add(ctx->tcerr.p, h.tcerr, 1);
+      add(d_tcerr, h.tcerr, 1);
     else
       *h.tcerr = 0;
     gather_kernel<<<32, 256, 0, st>>>(g);
@@ -3700,7 +3723,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     ex.und_n = (unsigned *)((unsigned long long *)ctx->undn.p + par);
     ex.und_cap = und_cap_par[par];
     ex.und_k = 0;
-    ex.amb = (unsigned long long *)ctx->amb.p;
+    ex.amb = d_amb;
     ex.counts = set->d_counts;
     ex.colunit = nullptr;
     PairArgs A;
@@ -3753,7 +3776,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
         T.cend = N;
         T.agg = ctx->tcagg.p;
         T.agg16 = tc16;
-        T.err = (unsigned long long *)ctx->tcerr.p;
+        T.err = d_tcerr;
         T.wait_ns = ctx->wait_ns;
         T.skip_fill_block = fault_pending ? 0 : -1;
         fault_pending = false;
@@ -4037,11 +4060,13 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     dev_off = tot;
     if (!to_device && sink && sink(user, (const char *)ctx->pinned, tot)) return TN93G_ESINK;
   }
-  unsigned long long counters[4], ambw[12];
-  CU(cudaMemcpyAsync(counters, ctx->counters.p, sizeof counters, cudaMemcpyDeviceToHost, st));
-  CU(cudaMemcpyAsync(ambw, ctx->amb.p, sizeof ambw, cudaMemcpyDeviceToHost, st));
+  CU(cudaMemcpyAsync(h_scalars, ctx->counters.p, kRunScalars * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
   CU(cudaEventRecord(E[9], st));
   CU(cudaStreamSynchronize(st));
+  unsigned long long counters[4], ambw[12];
+  memcpy(counters, h_scalars, sizeof counters);
+  memcpy(ambw, h_scalars + 4, sizeof ambw);
+  const unsigned long long tcerr = h_scalars[16];
   if (trace) {
     float d9;
     CU(cudaEventElapsedTime(&d9, E[0], E[9]));
@@ -4065,13 +4090,9 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   sum->undecided = 0;  // every listed pair was finished with the C library's logarithms
   sum->pairs_replayed = (long)counters[2];
   ctx->dev_out_n = dev_off;
-  if (use_tc) {
-    unsigned long long tcerr = 0;
-    CU(cudaMemcpy(&tcerr, ctx->tcerr.p, sizeof tcerr, cudaMemcpyDeviceToHost));
-    if (tcerr) {
-      ctx->err = "the tensor-core count kernel timed out waiting for its pipeline";
-      return TN93G_ETIMEOUT;
-    }
+  if (tcerr) {
+    ctx->err = "the tensor-core count kernel timed out waiting for its pipeline";
+    return TN93G_ETIMEOUT;
   }
   if (counters[3]) {
     ctx->err = "internal error: a row's text did not match its counted length";
