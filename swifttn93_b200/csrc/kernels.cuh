@@ -124,6 +124,7 @@ struct ReplayArgs {
   unsigned long long *counters;
   const LogTable *logt;
   ExactSink ex;
+  const uint32_t *ev_off = nullptr, *ev = nullptr;  // every sequence's events (ev nullptr: sites are found in the planes)
 };
 
 // One undecided pair on its way through the host: the walk writes the formula's exact inputs and the arguments of
