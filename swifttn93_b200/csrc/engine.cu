@@ -1509,38 +1509,101 @@ __device__ __forceinline__ double chain_shared(const double *x, int n, double s)
   return s;
 }
 
-// tn93's sums over a unit's rows in row order (swifttn93.cpp:2838-2848): s0 += rs[3 r], w0 += rw[3 r] for r < n, by one
-// block. The block stages 2,048 rows in shared memory and loads the next ones while warp 0 adds the sums and warp 1 the
-// weights. 30,000 rows: 291 us with one thread adding them one by one, 105 us so.
+// tn93's sum over a unit's rows in row order (swifttn93.cpp:2838-2848), *s0 = rs[0] + rs[STRIDE] + ... of n rows, by one block.
+// The block stages 2,048 rows in shared memory, loading the next ones meanwhile; each warp adds its share of them for the
+// binade that the sum stands in, and warp 0 puts the shares together: a share with a half-way term or past the binade is
+// added in smaller groups, and past the binade the shares that follow are formed anew. 30,000 rows: 291 us with one thread
+// adding them one by one, 105 us with one warp in groups, 88 us so.
 constexpr int kReduceChunk = 2048;
-template <int THREADS>
-__device__ __forceinline__ void chain_rows(const double *rs, const double *rw, long n, double *s0, double *w0)
+template <int THREADS, int STRIDE>
+__device__ __forceinline__ void chain_rows(const double *rs, long n, double *s0)
 {
-  __shared__ double ss[kReduceChunk], sw[kReduceChunk];
-  constexpr int kPer = kReduceChunk / THREADS;
+  constexpr int kPer = kReduceChunk / THREADS, kW = THREADS / 32, kShare = kReduceChunk / kW;
+  __shared__ double ss[kReduceChunk], part[kW], s_sh;
+  __shared__ int state[kW], from_sh;  // state of a share: 0 not addable, 1 addable, 2 all zero
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double a[kPer], b[kPer], s = 0.;
+  double a[kPer], s = 0.;
   auto load = [&](long r0) {
 #pragma unroll
     for (int k = 0; k < kPer; k++) {
       const long r = r0 + k * THREADS + threadIdx.x;
-      a[k] = r < n ? rs[r * 3] : 0.;
-      b[k] = r < n ? rw[r * 3] : 0.;
+      a[k] = r < n ? rs[r * STRIDE] : 0.;
     }
   };
   load(0);
   for (long r0 = 0; r0 < n; r0 += kReduceChunk) {
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kPer; k++) {
-      ss[k * THREADS + threadIdx.x] = a[k];
-      sw[k * THREADS + threadIdx.x] = b[k];
-    }
+    for (int k = 0; k < kPer; k++) ss[k * THREADS + threadIdx.x] = a[k];
     __syncthreads();
     load(r0 + kReduceChunk);
-    if (warp < 2) s = chain_shared(warp ? sw : ss, (int)min((long)kReduceChunk, n - r0), s);
+    const int m = (int)min((long)kReduceChunk, n - r0);  // past m: zeros
+    for (int from = 0; from < kW && from * kShare < m;) {
+      ChainBinade c;
+      const bool valid = chain_binade(s, c);
+      if (warp >= from) {
+        bool ok = valid, zero = true;
+        double y = 0.;
+#pragma unroll
+        for (int k = 0; k < kPer; k++) {
+          const double t = ss[warp * kShare + 32 * k + lane];
+          y = __dadd_rn(y, chain_round(c, t, ok));
+          zero &= t == 0.;
+        }
+        y = warp_total(y);
+        ok = __all_sync(0xffffffffu, ok);
+        zero = __all_sync(0xffffffffu, zero);
+        if (lane == 0) {
+          part[warp] = y;
+          state[warp] = zero ? 2 : ok ? 1 : 0;
+        }
+      }
+      __syncthreads();
+      if (warp == 0) {
+        int w = from;
+        while (w < kW && w * kShare < m) {
+          const int st = state[w];
+          const double s1 = __dadd_rn(s, part[w]);
+          if (st == 2 || (st == 1 && s1 < c.end)) {
+            if (st == 1) s = s1;
+            w++;
+            continue;
+          }
+          s = chain_shared(ss + w * kShare, min(kShare, m - w * kShare), s);
+          w++;
+          if (!valid || !(s < c.end)) break;
+        }
+        if (lane == 0) {
+          s_sh = s;
+          from_sh = w;
+        }
+      }
+      __syncthreads();
+      s = s_sh;
+      from = from_sh;
+    }
   }
-  if (warp < 2 && lane == 0) *(warp ? w0 : s0) = s;
+  if (threadIdx.x == 0) *s0 = s;
+}
+
+// the sum of weights, whole numbers: exact in any order while below 2^53 (chain_weights adds them one by one past that).
+// Every thread brings its part and whether all its terms were whole; the result is valid in thread 0.
+template <int THREADS, int STRIDE>
+__device__ __forceinline__ void chain_weights(const double *rw, long n, double part, bool whole, double *w0)
+{
+  __shared__ double ws[THREADS / 32];
+  part = warp_total(part);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = part;
+  whole = __syncthreads_and(whole);
+  if (threadIdx.x == 0) {
+    double w = 0.;
+    for (int k = 0; k < THREADS / 32; k++) w = __dadd_rn(w, ws[k]);
+    if (!whole || !(w < 0x1p53)) {
+      w = 0.;
+      for (long r = 0; r < n; r++) w = __dadd_rn(w, rw[r * STRIDE]);
+    }
+    *w0 = w;
+  }
 }
 
 // one warp per row: tn93's row sums in column order (swifttn93.cpp:2594-2602). The self-pair weights come first, as tn93
@@ -2040,7 +2103,15 @@ __global__ void __launch_bounds__(256) aln_reduce_kernel(const RowArgs *descs, d
     skipped += a.seg_skip[g];
     m = fmax(m, a.seg_max[g * 3]);
   }
-  chain_rows<256>(a.row_sum, a.row_w, nr, out + blockIdx.x * 3 + 1, out + blockIdx.x * 3 + 2);
+  double w = 0.;
+  bool whole = true;
+  for (long r = threadIdx.x; r < nr; r += 256) {
+    const double x = a.row_w[r * 3];
+    whole &= x >= 0. && x == floor(x);
+    w = __dadd_rn(w, x);
+  }
+  chain_weights<256, 3>(a.row_w, nr, w, whole, out + blockIdx.x * 3 + 2);
+  chain_rows<256, 3>(a.row_sum, nr, out + blockIdx.x * 3 + 1);
   for (int o = 16; o; o >>= 1) {
     links += __shfl_xor_sync(0xffffffffu, links, o);
     skipped += __shfl_xor_sync(0xffffffffu, skipped, o);
@@ -2368,6 +2439,7 @@ struct tn93g_ctx {
   size_t pin2_n[2] = {0, 0};
   void *pstats = nullptr;
   size_t pstats_n = 0;
+  std::vector<std::pair<int, std::string>> batch_keys, batch_site_keys;  // what BB_AGG and BB_SITE hold
   std::string tab_key;   // what agg and site hold (run_impl; empty: nothing)
   void *hrun = nullptr;  // pinned block of a run's small transfers
   size_t hrun_n = 0;
@@ -2719,12 +2791,39 @@ int tn93g_inject_fault(tn93g_ctx *ctx, int fault)
   return TN93G_OK;
 }
 
+// A band's links, skips and maxima over its n (row, segment) slots into tot[5] (zeroed before): links, skips, and the three
+// maxima as bit patterns (not negative). The host took them from a copy of every slot: 2.2 MB over the link for 6,700 rows
+// of 7 segments (51 us of gather_kernel, and the host's loop over them), 0.1 MB so: 0.14 ms less a run of 22.4 M pairs.
+__global__ void __launch_bounds__(256) band_totals_kernel(const long long *links, const long long *skip, const double *mx,
+                                                          long n, unsigned long long *tot)
+{
+  long long l = 0, k = 0;
+  double m[3] = {0., 0., 0.};
+  for (long t = blockIdx.x * 256l + threadIdx.x; t < n; t += gridDim.x * 256l) {
+    l += links[t];
+    k += skip[t];
+    for (int q = 0; q < 3; q++) m[q] = fmax(m[q], mx[t * 3 + q]);
+  }
+  for (int o = 16; o; o >>= 1) {
+    l += __shfl_xor_sync(0xffffffffu, l, o);
+    k += __shfl_xor_sync(0xffffffffu, k, o);
+    for (int q = 0; q < 3; q++) m[q] = fmax(m[q], __shfl_xor_sync(0xffffffffu, m[q], o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (l) atomicAdd(&tot[0], (unsigned long long)l);
+    if (k) atomicAdd(&tot[1], (unsigned long long)k);
+    for (int q = 0; q < 3; q++)
+      if (m[q] > 0.) atomicMax(&tot[2 + q], (unsigned long long)__double_as_longlong(m[q]));
+  }
+}
+
 // Copies up to nine ranges of 8-byte words into pinned host memory that the device maps (a band's statistics), so
 // that they reach the host without a copy-engine transfer, which would queue behind the band texts in flight.
 struct Gather {
   const unsigned long long *src[9];
   unsigned long long *dst[9];
   long n[9];
+  int stride[9];  // words from one source word to the next
   int k;
 };
 
@@ -2732,7 +2831,7 @@ __global__ void __launch_bounds__(256) gather_kernel(Gather g)
 {
   const long stride = (long)gridDim.x * blockDim.x;
   for (int r = 0; r < g.k; r++)
-    for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < g.n[r]; t += stride) g.dst[r][t] = g.src[r][t];
+    for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < g.n[r]; t += stride) g.dst[r][t] = g.src[r][t * g.stride[r]];
 }
 
 //------------------------------------------------------------------------------------------------ self-test
@@ -3304,6 +3403,7 @@ int tn93g_run_to_device(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn9
   return rc;
 }
 
+constexpr long kBandWords = 3 * kHistBins + 5;  // a band's histograms and totals (band_totals_kernel)
 constexpr size_t kRunScalars = 17;       // words of a run's scalars (run_impl)
 constexpr size_t kRunPinned = 4 << 20;  // pinned bytes kept for a run's small transfers
 
@@ -3634,10 +3734,9 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
       TRY(ensure(ctx, ctx->und[q], (size_t)und_cap * 2 * sizeof(unsigned long long)));
       und_cap_par[q] = und_cap;
     }
-    // pinned staging of a band's statistics: row sums and weights (3 each), segment maxima (3 each), segment links
-    // and skips, total bytes, the band's histogram, its undecided count and the count kernel's error word
-    stat_stride = (size_t)band * 6 * sizeof(double) + (size_t)nseg * (3 * sizeof(double) + 2 * sizeof(long long)) +
-                  (3 + 3 * kHistBins) * sizeof(unsigned long long);
+    // pinned staging of a band's statistics: row sums and weights (3 each at most), total bytes, the band's histogram and
+    // totals, its undecided count and the count kernel's error word
+    stat_stride = (size_t)band * 6 * sizeof(double) + (3 + kBandWords) * sizeof(unsigned long long);
     TRY(ensure_pinned_at(ctx, ctx->pstats, ctx->pstats_n, 2 * stat_stride, cudaHostAllocMapped));
     CU(cudaHostGetDevicePointer((void **)&d_pstats, ctx->pstats, 0));
     return TN93G_OK;
@@ -3649,7 +3748,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   CU(cudaMemsetAsync(ctx->counters.p, 0, kRunScalars * sizeof(unsigned long long), st));
   unsigned long long *const d_amb = (unsigned long long *)ctx->counters.p + 4, *const d_tcerr = d_amb + 12;
   // per band parity: its histogram (added on the host, so a band's row stage can run again), its undecided list
-  TRY(ensure(ctx, ctx->hist, 2 * 3 * kHistBins * sizeof(unsigned long long)));
+  TRY(ensure(ctx, ctx->hist, 2 * kBandWords * sizeof(unsigned long long)));
   TRY(ensure(ctx, ctx->total, 2 * sizeof(unsigned long long)));
   TRY(ensure(ctx, ctx->undn, 2 * sizeof(unsigned long long)));
   TRY(ensure(ctx, ctx->rdesc, 2 * sizeof(ReplayArgs)));
@@ -3658,9 +3757,9 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   memset(hist_total, 0, sizeof hist_total);
   long links = 0, skipped = 0, resolved = 0;
   float ms = 0;
+  const int bins = rc.fst ? 3 : 1;  // sums of a row that can be other than zero
   struct HostStats {
-    double *sum, *w, *max;
-    long long *links, *skip;
+    double *sum, *w;  // [row][bins]
     unsigned long long *total, *hist, *und, *tcerr;
   };
   auto host_stats = [&](int par) {
@@ -3668,12 +3767,9 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     HostStats h;
     h.sum = (double *)base;
     h.w = h.sum + band * 3;
-    h.max = h.w + band * 3;
-    h.links = (long long *)(h.max + nseg * 3);
-    h.skip = h.links + nseg;
-    h.total = (unsigned long long *)(h.skip + nseg);
+    h.total = (unsigned long long *)(h.w + band * 3);
     h.hist = h.total + 1;
-    h.und = h.hist + 3 * kHistBins;
+    h.und = h.hist + kBandWords;
     h.tcerr = h.und + 1;
     return h;
   };
@@ -3698,7 +3794,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     RA.seg_max = (double *)ctx->rmax.p + par * nseg * 3;
     RA.row_sum = (double *)ctx->rsum.p + par * band * 3;
     RA.row_w = (double *)ctx->rw.p + par * band * 3;
-    RA.hist = (unsigned long long *)ctx->hist.p + par * 3 * kHistBins;
+    RA.hist = (unsigned long long *)ctx->hist.p + par * kBandWords;
     RA.seg_off = (const unsigned long long *)ctx->roff.p + par * nseg;
     RA.seg_cols = nullptr;
     RA.nrows = RA.r1 - RA.r0;
@@ -3714,7 +3810,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     const long nr = bands[bi].second - bands[bi].first;
     cudaEvent_t *K = ctx->evk[par];
     RowArgs RA = row_args(bi);
-    CU(cudaMemsetAsync(RA.hist, 0, 3 * kHistBins * sizeof(unsigned long long), st));
+    CU(cudaMemsetAsync(RA.hist, 0, kBandWords * sizeof(unsigned long long), st));
     stats_kernel<<<dim3((unsigned)((nr + kWarps - 1) / kWarps), (unsigned)maxseg), 256, 0, st>>>(RA);
     CU(cudaGetLastError());
     ctx->launches++;
@@ -3725,6 +3821,10 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     scan_kernel<<<1, 1024, 0, st>>>(RA.seg_bytes, (unsigned long long *)RA.seg_off, nr * maxseg, dtot);
     CU(cudaGetLastError());
     ctx->launches++;
+    band_totals_kernel<<<(unsigned)std::min<long>(64, (nr * maxseg + 255) / 256), 256, 0, st>>>(
+        RA.seg_links, RA.seg_skip, RA.seg_max, nr * maxseg, RA.hist + 3 * kHistBins);
+    CU(cudaGetLastError());
+    ctx->launches++;
     CU(cudaEventRecord(K[3], st));
     // the band's statistics into the mapped staging (device addresses at the same offsets as host_stats')
     const HostStats h = host_stats(par);
@@ -3733,18 +3833,16 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     };
     Gather g;
     g.k = 0;
-    auto add = [&](const void *src, const void *hdst, long nwords) {
+    auto add = [&](const void *src, const void *hdst, long nwords, int stride = 1) {
       g.src[g.k] = (const unsigned long long *)src;
       g.dst[g.k] = dev(hdst);
+      g.stride[g.k] = stride;
       g.n[g.k++] = nwords;
     };
-    add(RA.row_sum, h.sum, nr * 3);
-    add(RA.row_w, h.w, nr * 3);
-    add(RA.seg_max, h.max, nr * maxseg * 3);
-    add(RA.seg_links, h.links, nr * maxseg);
-    add(RA.seg_skip, h.skip, nr * maxseg);
+    add(RA.row_sum, h.sum, nr * bins, 3 / bins);
+    add(RA.row_w, h.w, nr * bins, 3 / bins);
     add(dtot, h.total, 1);
-    add(RA.hist, h.hist, 3 * kHistBins);
+    add(RA.hist, h.hist, kBandWords);
     add((unsigned long long *)ctx->undn.p + par, h.und, 1);
     if (use_tc)
       add(d_tcerr, h.tcerr, 1);
@@ -3968,26 +4066,28 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
       CU(cudaEventSynchronize(K[4]));
     }
     for (int q = 0; q < 3 * kHistBins; q++) hist_total[q] += h.hist[q];
+    const unsigned long long *const bt = h.hist + 3 * kHistBins;
+    links += (long)bt[0];
+    skipped += (long)bt[1];
+    for (int q = 0; q < 3; q++) {
+      double m;
+      memcpy(&m, &bt[2 + q], sizeof m);
+      max_[q] = std::max(max_[q], m);
+    }
     // rows in order (swifttn93.cpp:2838-2848)
-    for (long r = 0; r < nr; r++) {
-      for (long g = r * maxseg; g < (r + 1) * maxseg; g++) {
-        links += h.links[g];
-        skipped += h.skip[g];
-        for (int q = 0; q < 3; q++)
-          if (h.max[g * 3 + q] > max_[q]) max_[q] = h.max[g * 3 + q];
+    for (long r = 0; r < nr; r++)
+      for (int q = 0; q < bins; q++) {
+        mean[q] += h.sum[r * bins + q];
+        wc[q] += h.w[r * bins + q];
       }
-      for (int q = 0; q < 3; q++) {
-        mean[q] += h.sum[r * 3 + q];
-        wc[q] += h.w[r * 3 + q];
-      }
-      if (row_sums) {
+    if (row_sums)
+      for (long r = 0; r < nr; r++) {
         double *o = row_sums + (size_t)(bands[bi].first - row_begin + r) * 6;
         for (int q = 0; q < 3; q++) {
-          o[q] = h.sum[r * 3 + q];
-          o[3 + q] = h.w[r * 3 + q];
+          o[q] = q < bins ? h.sum[r * bins + q] : 0.;
+          o[3 + q] = q < bins ? h.w[r * bins + q] : 0.;
         }
       }
-    }
     const unsigned long long tot = *h.total;
     if (!(rc.emit && !hyphy && tot)) return TN93G_OK;
     sum->output_bytes += tot;
@@ -4502,15 +4602,9 @@ __global__ void __launch_bounds__(256) qstats_kernel(RowArgs a)
     a.seg_bytes[slot] = bytes;
     a.seg_links[slot] = links;
     a.seg_skip[slot] = skipped;
-    a.seg_max[slot * 3] = mx;
-    a.seg_max[slot * 3 + 1] = 0.;
-    a.seg_max[slot * 3 + 2] = 0.;
-    a.row_sum[slot * 3] = s0;
-    a.row_sum[slot * 3 + 1] = 0.;
-    a.row_sum[slot * 3 + 2] = 0.;
-    a.row_w[slot * 3] = w0;
-    a.row_w[slot * 3 + 1] = 0.;
-    a.row_w[slot * 3 + 2] = 0.;
+    a.seg_max[slot] = mx;  // one word a slot here: a batch has one histogram bin
+    a.row_sum[slot] = s0;
+    a.row_w[slot] = w0;
   }
   __syncthreads();
   unsigned long long *hist = a.hist + (size_t)q * 3 * kHistBins;
@@ -4563,14 +4657,19 @@ __global__ void __launch_bounds__(512) query_reduce_kernel(RowArgs a, int nq, do
   const size_t base = (size_t)q * nr;
   double *o = qout + (size_t)q * 9;
   long long links = 0, skipped = 0;
-  double m = 0.;
+  double m = 0., w = 0.;
+  bool whole = true;
 #pragma unroll 4
   for (long r = threadIdx.x; r < nr; r += 512) {
     links += a.seg_links[base + r];
     skipped += a.seg_skip[base + r];
-    m = fmax(m, a.seg_max[(base + r) * 3]);
+    m = fmax(m, a.seg_max[base + r]);
+    const double x = a.row_w[base + r];
+    whole &= x >= 0. && x == floor(x);
+    w = __dadd_rn(w, x);
   }
-  chain_rows<512>(a.row_sum + base * 3, a.row_w + base * 3, nr, o + 3, o + 6);
+  chain_weights<512, 1>(a.row_w + base, nr, w, whole, o + 6);
+  chain_rows<512, 1>(a.row_sum + base, nr, o + 3);
   for (int o = 16; o; o >>= 1) {
     links += __shfl_xor_sync(0xffffffffu, links, o);
     skipped += __shfl_xor_sync(0xffffffffu, skipped, o);
@@ -4834,9 +4933,9 @@ int tn93g_server_create(tn93g_ctx *ctx, tn93g_server **out, const uint8_t *codes
     SV(ensure(ctx, srv->soff, nslot * sizeof(unsigned long long)));
     SV(ensure(ctx, srv->slinks, nslot * sizeof(long long)));
     SV(ensure(ctx, srv->sskip, nslot * sizeof(long long)));
-    SV(ensure(ctx, srv->smax, nslot * 3 * sizeof(double)));
-    SV(ensure(ctx, srv->rsum, nslot * 3 * sizeof(double)));
-    SV(ensure(ctx, srv->rw, nslot * 3 * sizeof(double)));
+    SV(ensure(ctx, srv->smax, nslot * sizeof(double)));
+    SV(ensure(ctx, srv->rsum, nslot * sizeof(double)));
+    SV(ensure(ctx, srv->rw, nslot * sizeof(double)));
     SV(ensure(ctx, srv->hist, (size_t)nq * 3 * kHistBins * sizeof(unsigned long long)));
     SV(ensure(ctx, srv->total, sizeof(unsigned long long)));
     SV(ensure(ctx, srv->segcols, (nq + 1) * sizeof(long)));
@@ -5185,6 +5284,7 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
     auto add = [&](const void *src, size_t nwords) {
       g.src[g.k] = (const unsigned long long *)src;
       g.dst[g.k] = dst;
+      g.stride[g.k] = 1;
       g.n[g.k++] = (long)nwords;
       dst += nwords;
     };
@@ -5792,8 +5892,7 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   // tables: one copy per distinct (mode, ambiguity subset, N plane); the site tables per (mode, subset)
   std::vector<int> tab_of(K), site_of(K);
   std::vector<std::pair<int, std::string>> keys, site_keys;
-  std::vector<PairTables> h_agg;
-  std::vector<SiteEntry> h_site;
+  std::vector<int> key_of, site_key_of;  // an alignment with that key
   for (int k = 0; k < K; k++) {
     const std::string sub((const char *)opts[k].subset, sizeof opts[k].subset);
     const std::string sk = opts[k].mode == TN93G_SUBSET ? sub : std::string();
@@ -5803,27 +5902,42 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
       if (keys[q] == key) t = (int)q;
     for (size_t q = 0; q < site_keys.size(); q++)
       if (site_keys[q] == skey) u = (int)q;
-    if (t < 0 || u < 0) build_tables(ctx->h_tab, opts[k].mode, opts[k].subset);
     if (t < 0) {
-      h_agg.emplace_back();
-      fill_pair_tables(*ctx->h_tab, RC[k].wplane, &h_agg.back());
       t = (int)keys.size();
       keys.push_back(key);
+      key_of.push_back(k);
     }
     if (u < 0) {
-      const SiteEntry *se = &ctx->h_tab->site[0][0];
-      h_site.insert(h_site.end(), se, se + sizeof(ctx->h_tab->site) / sizeof(SiteEntry));
       u = (int)site_keys.size();
       site_keys.push_back(skey);
+      site_key_of.push_back(k);
     }
     tab_of[k] = t;
     site_of[k] = u;
   }
+  // the last batch's tables stay on the device until a batch needs others (they depend on these keys alone)
   const size_t site_n = sizeof(ctx->h_tab->site) / sizeof(SiteEntry);
-  TRY(ensure(ctx, bb[BB_AGG], h_agg.size() * sizeof(PairTables)));
-  TRY(ensure(ctx, bb[BB_SITE], h_site.size() * sizeof(SiteEntry)));
-  CU(cudaMemcpyAsync(bb[BB_AGG].p, h_agg.data(), h_agg.size() * sizeof(PairTables), cudaMemcpyHostToDevice, st));
-  CU(cudaMemcpyAsync(bb[BB_SITE].p, h_site.data(), h_site.size() * sizeof(SiteEntry), cudaMemcpyHostToDevice, st));
+  if (keys != ctx->batch_keys || site_keys != ctx->batch_site_keys) {
+    ctx->batch_keys.clear();
+    std::vector<PairTables> h_agg(keys.size());
+    std::vector<SiteEntry> h_site;
+    for (size_t q = 0; q < keys.size(); q++) {
+      build_tables(ctx->h_tab, opts[key_of[q]].mode, opts[key_of[q]].subset);
+      fill_pair_tables(*ctx->h_tab, RC[key_of[q]].wplane, &h_agg[q]);
+    }
+    for (int k : site_key_of) {
+      build_tables(ctx->h_tab, opts[k].mode, opts[k].subset);
+      const SiteEntry *se = &ctx->h_tab->site[0][0];
+      h_site.insert(h_site.end(), se, se + site_n);
+    }
+    TRY(ensure(ctx, bb[BB_AGG], h_agg.size() * sizeof(PairTables)));
+    TRY(ensure(ctx, bb[BB_SITE], h_site.size() * sizeof(SiteEntry)));
+    CU(cudaMemcpyAsync(bb[BB_AGG].p, h_agg.data(), h_agg.size() * sizeof(PairTables), cudaMemcpyHostToDevice, st));
+    CU(cudaMemcpyAsync(bb[BB_SITE].p, h_site.data(), h_site.size() * sizeof(SiteEntry), cudaMemcpyHostToDevice, st));
+    CU(cudaStreamSynchronize(st));  // the host copies end here
+    ctx->batch_keys = keys;
+    ctx->batch_site_keys = site_keys;
+  }
   CU(cudaEventRecord(E[1], st));
   //------------------------------------------------------------------ pair stage
   std::vector<size_t> seg_base(K + 1, 0);
