@@ -1442,10 +1442,9 @@ __device__ __forceinline__ void stats_rows(const RowArgs &a, long bx, int sg)
     if (sh[t]) atomicAdd(&a.hist[t], sh[t]);
 }
 
-// Resident blocks per SM for the stats kernel 6 (40 registers) and the write kernel 4 (64): more warps hide their load
-// latency better than fewer spills would (same box, per 22.4 M pairs: stats + sums 0.80 ms with 3 blocks, 0.76 with
-// 4, 0.72 with 6; write 0.78 ms with 3, 0.68 with 4, 0.91 with 6; 2 blocks without spills were slower still)
-__global__ void __launch_bounds__(256, 6) stats_kernel(RowArgs a) { stats_rows(a, blockIdx.x, blockIdx.y); }
+// Resident blocks per SM for the stats and write kernels 4 (64 registers): same box, per 22.4 M pairs, row stage (stats,
+// sums, scan, totals) 0.50 ms with 4, 0.56 with 5, 0.54 with 6; write 0.60 ms with 4, 0.69 with 3, 0.91 with 6.
+__global__ void __launch_bounds__(256, 4) stats_kernel(RowArgs a) { stats_rows(a, blockIdx.x, blockIdx.y); }
 
 
 // Sums in order by a warp (chain_sum.cuh): s and the result are the same in every lane.
@@ -4967,6 +4966,8 @@ int tn93g_server_create(tn93g_ctx *ctx, tn93g_server **out, const uint8_t *codes
     srv->tc_chunk = std::min<long>(kServerTcChunk, std::max(kServerTcChunkMin, (max_batch_sequences + 127) / 64 * 64));
     const size_t agg = (size_t)N * (srv->tc16 ? 16 : 32);
     const bool room = ensure(ctx, srv->ohimg, img) == TN93G_OK;
+    // under a budget the larger chunk has to leave as much again for what batches grow (text, undecided lists)
+    if (ctx->budget && ctx->used + 2 * agg * srv->tc_chunk > ctx->budget) srv->tc_chunk = kServerTcChunkMin;
     if (room && ensure(ctx, srv->tcagg, agg * srv->tc_chunk) != TN93G_OK) {
       cudaGetLastError();
       srv->tc_chunk = kServerTcChunkMin;
@@ -5861,9 +5862,16 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   TRY(ensure(ctx, bb[BB_DIST], d_off[K] * sizeof(double)));
   TRY(ensure(ctx, bb[BB_RQ], q_off[K] * sizeof(unsigned long long)));
   int planned = plan_events(use_tc);
+  if (use_tc && planned == TN93G_OK && ctx->budget) {  // under a budget, what comes after needs its share
+    size_t rest = (1 << 20) + NR * 512;                // lists and row arrays, then the operand images
+    for (int k = 0; k < K; k++)
+      rest += (size_t)(alns[k].n / 32 + 2) * ((RC[k].Lc + kTcStageK - 1) / kTcStageK) * kTcBlockBytes;
+    if (ctx->used + rest > ctx->budget) planned = TN93G_ENOMEM;
+  }
   if (use_tc && planned != TN93G_OK && planned != TN93G_ETOOBIG) {
     cudaGetLastError();
     release(ctx, bb[BB_EV2]);
+    release(ctx, bb[BB_TCAGG]);
     planned = plan_events(false);
   }
   TRY(planned);

@@ -18,9 +18,11 @@
 #if defined(__CUDACC__)
 #define TN_HD __host__ __device__ __forceinline__
 #define TN_HDI __host__ __device__
+#define TN_HDN __host__ __device__ __noinline__ static
 #else
 #define TN_HD static inline
 #define TN_HDI static
+#define TN_HDN static
 #endif
 
 #if defined(__CUDA_ARCH__)
@@ -520,8 +522,21 @@ TN_HD uint64_t dec_scale_fast(uint64_t m, int e2, int s, int &cmp)
   return q;
 }
 
-// six significant digits of d > 0 (finite), rounded half-to-even on the exact binary value
-TN_HD Dec decimal6(double d)
+// 10^s for 0 <= s <= 11
+#if defined(__CUDACC__)
+__constant__ double kPow10d[12] = {1e0, 1e1, 1e2, 1e3, 1e4, 1e5, 1e6, 1e7, 1e8, 1e9, 1e10, 1e11};
+#endif
+TN_HD double pow10d(int s)
+{
+#if defined(__CUDA_ARCH__)
+  return kPow10d[s];
+#else
+  return (double)pow10u(s);
+#endif
+}
+
+// the same for any d > 0, by whole numbers: out of line, as decimal6 decides almost every value itself
+TN_HDN Dec decimal6_exact(double d)
 {
   const uint64_t b = TBITS(d);
   const int be = (int)((b >> 52) & 0x7ff);
@@ -566,6 +581,33 @@ TN_HD Dec decimal6(double d)
   Dec r;
   r.q = (uint32_t)q;
   r.X = X;
+  return r;
+}
+
+// Six significant digits of d > 0 (finite), rounded half-to-even on the exact binary value. In [1e-5, 1e5) the scaled
+// double t = d 10^(5 - X) is within 2e-10 of the exact product (10^s is exact up to 10^22, so one rounding), which decides
+// the digits unless its fraction is within 1e-6 of a half; a floor one too low has a fraction next to 1 and rounds up to the
+// same digits. X: floor(log10 2^e) from the binary exponent (78,913 / 2^18 for log10 2, exact floors for -18 <= e <= 17), one
+// more where t reaches 10^6. (The row stage of 22.4 M distances: 0.57 -> 0.50 ms.)
+TN_HD Dec decimal6(double d)
+{
+  if (!(d >= 1e-5 && d < 1e5)) return decimal6_exact(d);
+  const int e = (int)(TBITS(d) >> 52) - 1023;
+  Dec r;
+  r.X = (e * 78913) >> 18;
+  double t = TMUL(d, pow10d(5 - r.X));
+  if (t >= 1e6) {
+    r.X++;
+    t = TMUL(d, pow10d(5 - r.X));
+  }
+  r.q = (uint32_t)t;
+  const double f = TSUB(t, (double)r.q);
+  if (f > 0.499999 && f < 0.500001) return decimal6_exact(d);
+  r.q += f > 0.5 ? 1u : 0u;
+  if (r.q == 1000000u) {
+    r.q = 100000u;
+    r.X++;
+  }
   return r;
 }
 
