@@ -172,9 +172,23 @@ __device__ __forceinline__ void onehot_body(const uint8_t *__restrict__ cc, long
   const long seq = seq0 + t / nchunk, ch = t % nchunk;
   const long s = ch / (kTcStageK / 16), c = ch % (kTcStageK / 16);
   const long k0 = ch * 16;
+  // the 16 codes by the aligned words that hold them (a load for each code: 2,000 x 29,900 121 us, 103 us so)
   uint32_t code[16];
+  if (seq < N && k0 + 16 <= Lc) {
+    const uintptr_t ad = reinterpret_cast<uintptr_t>(cc + seq * Lc + k0);
+    const uint64_t *p = reinterpret_cast<const uint64_t *>(ad & ~(uintptr_t)7);
+    const int f = 8 * (int)(ad & 7);
+    const uint64_t x0 = __ldg(p), x1 = __ldg(p + 1), x2 = f ? __ldg(p + 2) : 0;
+    const uint64_t lo = x0 >> f | x1 << 1 << (63 - f), hi = x1 >> f | x2 << 1 << (63 - f);
 #pragma unroll
-  for (int q = 0; q < 16; q++) code[q] = (seq < N && k0 + q < Lc) ? sw[cc[seq * Lc + k0 + q] & 31] : 0u;
+    for (int q = 0; q < 8; q++) {
+      code[q] = sw[(int)(lo >> 8 * q) & 31];
+      code[q + 8] = sw[(int)(hi >> 8 * q) & 31];
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 16; q++) code[q] = (seq < N && k0 + q < Lc) ? sw[cc[seq * Lc + k0 + q] & 31] : 0u;
+  }
   const long b = seq / 32, sl = seq % 32;
   uint8_t *blk = img + ((size_t)s * NB + b) * kTcBlockBytes;
   // 4 x 4 byte transposes: class cls of four columns to a word
