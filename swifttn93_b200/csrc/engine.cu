@@ -1299,7 +1299,13 @@ struct PairView {
   double thisD;
 };
 
-__device__ __forceinline__ PairView view_pair(const RowArgs &a, long i, long j, long cnt_i)
+__device__ __forceinline__ double raw_pair(const RowArgs &a, long i, long j)
+{
+  return a.dist[(size_t)(i - a.r0) * a.ncols + (j - a.colbase)];
+}
+
+// pair (i, j), whose raw distance the caller has read (for j < N)
+__device__ __forceinline__ PairView view_pair(const RowArgs &a, long i, long j, long cnt_i, double raw)
 {
   const RunConsts &rc = a.rc;
   PairView v;
@@ -1310,7 +1316,6 @@ __device__ __forceinline__ PairView view_pair(const RowArgs &a, long i, long j, 
   v.w = 0;
   v.thisD = -1.0;
   if (!v.valid) return v;
-  const double raw = a.dist[(size_t)(i - a.r0) * a.ncols + (j - a.colbase)];
   v.w = cnt_i * a.counts[j];
   if (rc.fst) v.bin = i < rc.n1 ? (j >= rc.n1 ? 2 : 0) : 1;
   if ((uint64_t)__double_as_longlong(raw) != kSkipBits) {
@@ -1407,7 +1412,7 @@ __device__ __forceinline__ void stats_rows(const RowArgs &a, long bx, int sg)
     }
     for (long j0 = c0; j0 < c1; j0 += 32) {
       const long j = j0 + lane;
-      PairView v = view_pair(a, i, j, cnt_i);
+      PairView v = view_pair(a, i, j, cnt_i, j < rc.N ? raw_pair(a, i, j) : 0.);
       if (j >= c1) v.valid = v.computed = v.linked = false;
       // histogram: lanes with the same bin add once (their weights summed when all are 1)
       const int key = v.computed ? v.bin * kHistBins + v.hb : -1;
@@ -1534,7 +1539,7 @@ __device__ __forceinline__ double chain_shared(const double *x, int n, double s)
 // The block stages 2,048 rows in shared memory, loading the next ones meanwhile; each warp adds its share of them for the
 // binade that the sum stands in, and warp 0 puts the shares together: a share with a half-way term or past the binade is
 // added in smaller groups, and past the binade the shares that follow are formed anew. 30,000 rows: 291 us with one thread
-// adding them one by one, 105 us with one warp in groups, 88 us so.
+// adding them one by one, 105 us with one warp in groups, 80 us so.
 constexpr int kReduceChunk = 2048;
 template <int THREADS, int STRIDE>
 __device__ __forceinline__ void chain_rows(const double *rs, long n, double *s0)
@@ -1825,8 +1830,8 @@ struct Stager {
 };
 
 // Lines in 8-byte words. A byte at a time (load a byte, store a byte) a line of 36 bytes took about 500 instructions of a
-// warp for 32 of them and 22.4 M of them 611-649 us; by words of 8 shifted into place 602 us, column numbers (-f csvn) 449 ->
-// 325 us per 1.6 M. What bounds it is latency: loading the next columns' codes and names early (more registers, 3 blocks
+// warp for 32 of them and 22.4 M of them 611-649 us; by words of 8 shifted into place 602 us (630 since the exact
+// digits of rare values are a call), column numbers (-f csvn) 449 -> 325 us per 1.6 M. What bounds it is latency: loading the next columns' codes and names early (more registers, 3 blocks
 // instead of 4 on an SM) took 687 us.
 constexpr int kLineName = 64;  // longest name (and start of a line) written by words
 
@@ -4592,8 +4597,15 @@ __global__ void __launch_bounds__(256) qstats_kernel(RowArgs a)
   double mx = 0., s0 = 0., w0 = 0.;
   long long links = 0, skipped = 0;
   unsigned long long bytes = 0;
+  // A thread's distances lie next to each other, its neighbours' a row apart: four are loaded together (a 32-byte sector),
+  // before any is used (40 queries x 30,000 rows: 510 us one at a time, 446 us so).
+  double raw[4];
   for (long j = c0; j < c1; j++) {
-    PairView v = view_pair(a, ii, j, cnt_i);
+    const int at = (int)(j - c0) & 3;
+    if (at == 0)
+#pragma unroll
+      for (int k = 0; k < 4; k++) raw[k] = j + k < c1 ? raw_pair(a, ii, j + k) : 0.;
+    PairView v = view_pair(a, ii, j, cnt_i, at == 0 ? raw[0] : at == 1 ? raw[1] : at == 2 ? raw[2] : raw[3]);
     if (!row) v.valid = v.computed = v.linked = false;
     const int key = v.computed ? v.hb : -1;
     const unsigned peers = __match_any_sync(0xffffffffu, key);
