@@ -2610,6 +2610,7 @@ int upload_host(tn93g_ctx *ctx, const std::vector<HostSpan> &spans)
     size_t n;
   };
   std::vector<Piece> pieces;
+  std::vector<const HostSpan *> pageable;
   for (const HostSpan &h : spans) {
     cudaPointerAttributes pa;
     bool direct = h.n < kUploadMin / 16;  // many small copies cost more than the staging saves
@@ -2622,6 +2623,7 @@ int upload_host(tn93g_ctx *ctx, const std::vector<HostSpan> &spans)
       if (h.n) CU(cudaMemcpyAsync(h.dst, h.src, h.n, cudaMemcpyHostToDevice, ctx->stream));
       continue;
     }
+    pageable.push_back(&h);
     for (size_t at = 0; at < h.n; at += kUploadPiece)
       pieces.push_back({(char *)h.dst + at, (const char *)h.src + at, std::min(kUploadPiece, h.n - at)});
   }
@@ -2638,7 +2640,7 @@ int upload_host(tn93g_ctx *ctx, const std::vector<HostSpan> &spans)
       if (!ctx->upload_ev[q]) CU(cudaEventCreateWithFlags(&ctx->upload_ev[q], cudaEventDisableTiming));
   }
   if (!staged) {
-    for (const Piece &p : pieces) CU(cudaMemcpyAsync(p.dst, p.src, p.n, cudaMemcpyHostToDevice, ctx->stream));
+    for (const HostSpan *h : pageable) CU(cudaMemcpyAsync(h->dst, h->src, h->n, cudaMemcpyHostToDevice, ctx->stream));
     return TN93G_OK;
   }
   std::atomic<size_t> next{0};
