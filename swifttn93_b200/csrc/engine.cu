@@ -663,7 +663,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs &a, const unsigned char
   const PackedTables &PT = *reinterpret_cast<const PackedTables *>(smem);
   const AggEntry *EW = ew_entries(smem, packed);
   // block-uniform exits: no valid pair in the tile
-  if (i0 >= a.r1 || j0 >= rc.N) return;
+  if (i0 >= a.r1 || j0 >= a.cend) return;
   if (!rc.cross && j0 + kTile - 1 <= i0) return;
   const long Np = rc.Npad;
   // N-plane cross terms from the sequences' nonzero N words (row side and column side), when the clean-site counts
@@ -731,7 +731,7 @@ __device__ __forceinline__ void pair_tile(const PairArgs &a, const unsigned char
     const long i = i0 + warp + kWarps * r;
     if (i >= a.r1) break;
     const long lb = rc.cross ? rc.n1 : i + 1;
-    const bool valid = j >= lb && j < rc.N;
+    const bool valid = j >= lb && j < a.cend;
     if (!__any_sync(0xffffffffu, valid)) continue;
     Counts c = Counts{0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     const bool tc = a.tcagg != nullptr;  // clean-site counts from the tensor-core kernel
@@ -862,7 +862,7 @@ __global__ void __launch_bounds__(256, MINB) pair_kernel(PairArgs a)
   int *colacc = reinterpret_cast<int *>(smem_raw + kTabSmem);
   const long i0 = a.r0 + blockIdx.y * (long)kTile;
   const long j0 = a.cstart + blockIdx.x * (long)kTile;
-  if (i0 >= a.r1 || j0 >= a.rc.N || (!a.rc.cross && j0 + kTile - 1 <= i0)) return;
+  if (i0 >= a.r1 || j0 >= a.cend || (!a.rc.cross && j0 + kTile - 1 <= i0)) return;
   load_pair_tables(a.tab, smem_raw, a.rc.packed, WPLANE && a.rc.fallback_avg);
   __syncthreads();
   pair_tile<WPLANE, GAPMM>(a, smem_raw, colacc, i0, j0, kRowsPerWarp);
@@ -2330,7 +2330,7 @@ cudaError_t launch_pair(const PairArgs &A, long ncolblocks, long nrows, cudaStre
   }();
   dim3 g((unsigned)ncolblocks, (unsigned)((nrows + kTile - 1) / kTile));
   if (pair_split(A)) {
-    const long jend = std::min<long>(A.rc.N, A.cstart + ncolblocks * kTile), jbeg = A.cstart & ~1l, ibeg = A.r0 & ~1l;
+    const long jend = std::min<long>(A.cend, A.cstart + ncolblocks * kTile), jbeg = A.cstart & ~1l, ibeg = A.r0 & ~1l;
     const long rows = A.rc.wplane ? EvTile<true>::rows : EvTile<false>::rows;
     const dim3 ge((unsigned)((jend - jbeg + kEvCols - 1) / kEvCols), (unsigned)((A.r1 - ibeg + rows - 1) / rows));
     const cudaError_t e = A.lin         ? cudaSuccess
@@ -3915,6 +3915,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     A.r1 = r1;
     A.ncols = ncols;
     A.colbase = colbase;
+    A.cend = N;
     A.dist = (double *)ctx->dist.p + par * dslots;
     A.replay_q = (unsigned long long *)ctx->rq.p;
     A.replay_n = (unsigned *)ctx->rqn.p;
@@ -4504,6 +4505,7 @@ int noalloc_run(const uint8_t *d_codes, long N, long L, const tn93g_opts *opts, 
   A.ncols = N;
   A.colbase = 0;
   A.cstart = 0;
+  A.cend = N;
   A.dist = d_dist;
   A.replay_q = (unsigned long long *)(S + kNaRq);
   A.replay_n = rqn;
@@ -4762,8 +4764,9 @@ struct tn93g_server {
 
 namespace {
 // Query columns per chunk of the tensor-core records (counts, events, formula), a multiple of 64; chunks end on the count
-// kernel's 64-column tiles. 40 queries (1,280 columns) against 30,000 sequences, pair stage:
-// 5.03 ms with chunks of 128 from the reference's last row (three 64-column tiles each), 3.91 so.
+// kernel's 64-column tiles, so the first one is up to 63 columns narrower, and the pair stage stops where the counts do
+// (PairArgs::cend). 40 queries (1,280 columns) against 30,000 sequences, pair stage: 5.03 ms with chunks of 128 from the
+// reference's last row (three 64-column tiles each), 3.91 so.
 constexpr long kServerTcChunk = 512, kServerTcChunkMin = 128;
 
 // words of the statistics of a batch of nq queries: total, undecided, counters, error word, and per query 9 sums, 3 counts,
@@ -5201,6 +5204,7 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
     A.ncols = Q;
     A.colbase = Nref;
     A.cstart = Nref;
+    A.cend = Nref + Q;
     A.dist = (double *)srv->dist.p;
     A.replay_q = (unsigned long long *)srv->rq.p;
     A.replay_n = (unsigned *)srv->rqn.p;
@@ -5238,6 +5242,7 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
         AC.tcncols = srv->tc_chunk;
         AC.tccolbase = c0;
         AC.cstart = c0;
+        AC.cend = c1;  // the records past it are the next chunk's, not counted yet
         CU(launch_pair(AC, (c1 - c0 + 31) / 32, Nref, st));
         ctx->launches += pair_split(AC) && !AC.lin ? 3 : 2;
       }
@@ -6019,6 +6024,7 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
     A.ncols = alns[k].n;
     A.colbase = 0;
     A.cstart = 0;
+    A.cend = alns[k].n;
     A.dist = (double *)bb[BB_DIST].p + d_off[k];
     A.replay_q = (unsigned long long *)bb[BB_RQ].p + q_off[k];
     A.replay_n = (unsigned *)bb[BB_RQN].p + k;

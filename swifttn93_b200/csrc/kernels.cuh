@@ -89,6 +89,7 @@ struct PairArgs {
   long r0, r1;          // band rows
   long ncols, colbase;  // row stride of dist and the first global column it holds
   long cstart;          // first column of the launch grid (a multiple of 32 past colbase)
+  long cend;            // columns at or past cend are left alone: their records are not counted yet (N: all columns)
   double *dist;
   unsigned long long *replay_q;  // (t << 63) | (i << 31) | j
   unsigned int *replay_n;

@@ -213,8 +213,8 @@ __device__ __forceinline__ void event_tile(const PairArgs &a, int bx, int by)
   if (threadIdx.x < 2) items[threadIdx.x] = 0;
   // tiles start on even rows and columns (two codes per load); rows before r0 and columns before colbase are skipped
   const int i0 = (int)(a.r0 & ~1l) + by * T::rows, j0 = (int)(a.cstart & ~1l) + bx * kEvCols;
-  const int N = (int)rc.N, r1 = (int)a.r1;
-  if (i0 >= r1 || j0 >= N || (!rc.cross && j0 + kEvCols - 1 <= i0)) return;
+  const int N = (int)rc.N, r1 = (int)a.r1, cend = (int)a.cend;
+  if (i0 >= r1 || j0 >= cend || (!rc.cross && j0 + kEvCols - 1 <= i0)) return;
   const EventTables &ET = *reinterpret_cast<const EventTables *>(smem);
   const unsigned char *avg = smem + sizeof(EventTables);
   const AggEntry *EW = reinterpret_cast<const AggEntry *>(smem + sizeof(EventTables) + sizeof(a.tab->packed.avg));
@@ -246,7 +246,7 @@ __device__ __forceinline__ void event_tile(const PairArgs &a, int bx, int by)
     const int iw = min(i0 + lane, N - 1);
     for (int cl = next_item(&items[0]); cl < kEvCols; cl = next_item(&items[0])) {
       const int j = j0 + cl;
-      if (j >= N || (!rc.cross && j <= i0)) continue;  // no pair of the tile reads this column
+      if (j >= cend || (!rc.cross && j <= i0)) continue;  // no pair of the tile reads this column
       uint32_t A[4] = {0u, 0u, 0u, 0u}, B[4] = {0u, 0u, 0u, 0u};
       const uint32_t e0 = soff[T::rows + 1 + cl], e1 = soff[T::rows + 2 + cl];
       add_events2<!WPLANE>(A, B, smem + sizeof ET.row, group, a.ev2, a.ccT + ib, e0, e1);
@@ -269,7 +269,7 @@ __device__ __forceinline__ void event_tile(const PairArgs &a, int bx, int by)
   // the constant columns' share of packed words
   const uint32_t cw[3] = {16u * (uint32_t)rc.constT * 0x10001u,
                           16u * ((uint32_t)rc.constNf[0] + ((uint32_t)rc.constNf[1] << 16)), 16u * (uint32_t)rc.constNf[2]};
-  const int jmin = (int)tb, jmax = (int)min(rc.N, tb + tn);
+  const int jmin = (int)tb, jmax = (int)min(a.cend, tb + tn);
   // below this share of the sites (less a margin over single precision) the -g test cannot fire
   const float gfloor = (float)(rc.resolve_fraction / 16.0) * 0.9999f;
   const int l16 = overlap16(rc);
@@ -501,7 +501,7 @@ __device__ __noinline__ bool three_pair(const uint8_t *flag, const uint8_t *thre
 }
 
 // The formula for the records that event_kernel finished (state 0; 1: queued for the site-order walk, 2: skipped by -l).
-// A warp takes a segment of segw columns of rpw rows. The record's x16 integers go into the formula as they are: every
+// A warp takes a segment of segw columns of rpw rows; the launch's columns are [jlo, jhi), jhi at most cend. The record's x16 integers go into the formula as they are: every
 // quantity scales by a power of two, so each quotient is the same double. A logarithm that the C library may round the
 // other way (17% of the pairs have one, so nearly every warp step would run the certificate for a few lanes) puts the
 // pair's range in a per-warp queue, and the certificate runs for 32 queued pairs at a time.
@@ -563,7 +563,7 @@ __device__ __forceinline__ void formula_rows(const PairArgs &a, long jlo, long j
   for (long i = ra; i < rb; i++) {
     const long lb = rc.cross ? rc.n1 : i + 1;
     const long s0 = (rc.cross ? jlo : max(lb, jlo)) + (long)by * segw;
-    const long c0 = max(lb, s0), c1 = min(min(rc.N, jhi), s0 + segw);
+    const long c0 = max(lb, s0), c1 = min(jhi, s0 + segw);
     const size_t rec0 = (size_t)(i - a.r0) * tn - tb;
     double *const drow = a.dist + (size_t)(i - a.r0) * a.ncols - a.colbase;
     uint32_t q0 = 0, q1 = 0;
@@ -704,5 +704,5 @@ __global__ void __launch_bounds__(256, 3) formula_batch_kernel(const PairArgs *d
 {
   const int4 b = blocks[blockIdx.x];
   const PairArgs &a = batch_args(descs, b.x);
-  formula_rows<REC16, LIN>(a, 0, a.rc.N, b.w & 2047, b.w >> 11, b.y, b.z);
+  formula_rows<REC16, LIN>(a, 0, a.cend, b.w & 2047, b.w >> 11, b.y, b.z);
 }
