@@ -2503,26 +2503,6 @@ namespace {
 // length of an event list with its null events
 uint32_t pad_events(uint32_t n) { return (n + kEvPad - 1) / kEvPad * kEvPad; }
 
-int ensure(tn93g_ctx *ctx, DevBuf &b, size_t bytes)
-{
-  if (bytes <= b.n && b.p) return TN93G_OK;
-  if (b.p) {
-    cudaFree(b.p);
-    ctx->used -= b.n;
-    b.p = nullptr;
-    b.n = 0;
-  }
-  bytes = std::max<size_t>(bytes, 256);
-  if (ctx->budget && ctx->used + bytes > ctx->budget) {
-    ctx->err = "over the context's HBM budget";
-    return TN93G_ENOMEM;
-  }
-  CU(cudaMalloc(&b.p, bytes));
-  b.n = bytes;
-  ctx->used += bytes;
-  return TN93G_OK;
-}
-
 // gives b back; the stream's work on it ends first (cudaFree waits for the device)
 void release(tn93g_ctx *ctx, DevBuf &b)
 {
@@ -2531,6 +2511,49 @@ void release(tn93g_ctx *ctx, DevBuf &b)
   ctx->used -= b.n;
   b.p = nullptr;
   b.n = 0;
+}
+
+// Gives back the memory that only saves time, for a call that has no room without it: a run's event offsets (its pair stage
+// takes the fused kernel from then on, with the same results). Kernels get such a buffer's address from the context at each
+// launch, never from an earlier one. False when there was nothing to give.
+bool reclaim(tn93g_ctx *ctx)
+{
+  const size_t before = ctx->used;
+  release(ctx, ctx->ev2);
+  return ctx->used < before;
+}
+
+// bytes of device memory within the budget; TN93G_ENOMEM where they do not fit
+int take_device(tn93g_ctx *ctx, void **p, size_t bytes)
+{
+  if (ctx->budget && ctx->used + bytes > ctx->budget) {
+    ctx->err = "over the context's HBM budget";
+    return TN93G_ENOMEM;
+  }
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // the caller may do without
+    ctx->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
+    return e == cudaErrorMemoryAllocation ? TN93G_ENOMEM : TN93G_ECUDA;
+  }
+  ctx->used += bytes;
+  return TN93G_OK;
+}
+
+// b of at least `bytes`, its contents lost when it grows. spare: memory that the caller can do without (nothing is given back
+// for it, and no message is left)
+int ensure(tn93g_ctx *ctx, DevBuf &b, size_t bytes, bool spare = false)
+{
+  if (bytes <= b.n && b.p) return TN93G_OK;
+  release(ctx, b);
+  bytes = std::max<size_t>(bytes, 256);
+  int r = take_device(ctx, &b.p, bytes);
+  while (r == TN93G_ENOMEM && !spare && reclaim(ctx)) r = take_device(ctx, &b.p, bytes);
+  if (r == TN93G_OK)
+    b.n = bytes;
+  else if (r == TN93G_ENOMEM && spare)
+    ctx->err.clear();
+  return r;
 }
 
 int ensure_pinned(tn93g_ctx *ctx, size_t bytes)
@@ -2562,12 +2585,10 @@ int ensure_keep(tn93g_ctx *ctx, DevBuf &b, size_t bytes, size_t keep)
 {
   if (bytes <= b.n && b.p) return TN93G_OK;
   bytes = std::max<size_t>(bytes + bytes / 2, 1 << 20);
-  if (ctx->budget && ctx->used + bytes > ctx->budget) {
-    ctx->err = "over the context's HBM budget";
-    return TN93G_ENOMEM;
-  }
   void *p = nullptr;
-  CU(cudaMalloc(&p, bytes));
+  int r = take_device(ctx, &p, bytes);
+  while (r == TN93G_ENOMEM && reclaim(ctx)) r = take_device(ctx, &p, bytes);
+  if (r != TN93G_OK) return r;
   if (keep && b.p) CU(cudaMemcpyAsync(p, b.p, keep, cudaMemcpyDeviceToDevice, ctx->stream));
   if (b.p) {
     CU(cudaStreamSynchronize(ctx->stream));
@@ -2576,7 +2597,6 @@ int ensure_keep(tn93g_ctx *ctx, DevBuf &b, size_t bytes, size_t keep)
   }
   b.p = p;
   b.n = bytes;
-  ctx->used += bytes;
   return TN93G_OK;
 }
 
@@ -3113,7 +3133,12 @@ static int upload_set(tn93g_ctx *ctx, tn93g_set **out, const uint8_t *codes, cud
       return cudaSuccess;
     }
     s->cap[k] = bytes;
-    return cudaMalloc(p, bytes);
+    cudaError_t m = cudaMalloc(p, bytes);
+    while (m == cudaErrorMemoryAllocation && reclaim(ctx)) {
+      cudaGetLastError();
+      m = cudaMalloc(p, bytes);
+    }
+    return m;
   };
   if ((e = take((void **)&s->d_codes, (size_t)N * L, 0)) != cudaSuccess) return fail(e);
   if ((e = take((void **)&s->d_counts, N * sizeof(long), 1)) != cudaSuccess) return fail(e);
@@ -3609,10 +3634,17 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   }
   rc.packed = max_ev <= (uint32_t)kPackedMaxEvents;
   TRY(ensure(ctx, ctx->ev, std::max<size_t>(evoff[N], 1) * sizeof(uint32_t)));
-  TRY(ensure(ctx, ctx->ev2, std::max<size_t>(evoff[N], 1) * sizeof(uint2)));
+  // The events again as event_kernel reads them, where the pair stage takes it (pair_split) and there is room: 8 bytes an
+  // event beside the 4 of the list. Without them the fused kernel runs.
+  bool use_ev2 = use_tc && !lin && rc.packed && Lc * Npad < (1l << 32) && (!rc.wplane || sparse_w);
+  if (use_ev2) {
+    const int r = ensure(ctx, ctx->ev2, std::max<size_t>(evoff[N], 1) * sizeof(uint2), true);
+    if (r != TN93G_ENOMEM) TRY(r);
+    use_ev2 = r == TN93G_OK;
+  }
   CU(cudaMemcpyAsync(ctx->evoff.p, evoff, (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
   pa.ev = (uint32_t *)ctx->ev.p;
-  pa.ev2 = (uint2 *)ctx->ev2.p;
+  pa.ev2 = use_ev2 ? (uint2 *)ctx->ev2.p : nullptr;
   pa.ev2_Npad = (uint32_t)Npad;
   if (W && evoff[N]) {  // no list: nothing reads one
     events_kernel<<<(unsigned)((N + kWarps - 1) / kWarps), 256, 0, st>>>(pa);
@@ -3907,7 +3939,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     A.ccT = (const uint8_t *)ctx->ccT.p;
     A.ev_off = (const uint32_t *)ctx->evoff.p;
     A.ev = (const uint32_t *)ctx->ev.p;
-    A.ev2 = pa.ev2;
+    A.ev2 = use_ev2 ? (const uint2 *)ctx->ev2.p : nullptr;
     A.three = pa.three;
     A.lin = lin;
     A.tab = (const PairTables *)ctx->agg.p;

@@ -1,0 +1,45 @@
+"""Contexts with a memory budget that holds a call's own buffers but not what only makes it faster: the call runs, with the
+bytes of an unlimited context. The budgets are what the calls take without those buffers, found by halving, and half a
+megabyte."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _codes(n, L, ambiguous, seed=1, divergence=0.02):
+    rng = np.random.default_rng(seed)
+    base = rng.integers(0, 4, L)
+    s = np.where(rng.random((n, L)) < divergence, rng.integers(0, 4, (n, L)), base[None]).astype(np.uint8)
+    hit = rng.random((n, L)) < ambiguous
+    s[hit] = rng.choice((5, 6, 7, 8, 9, 10), int(hit.sum()))
+    return s
+
+
+def _names(n):
+    return [f"seq{i:05d}" for i in range(n)]
+
+
+def _engine(megabytes):
+    from swifttn93_b200 import Engine
+
+    return Engine(hbm_budget=int(megabytes * 2**20))
+
+
+@pytest.mark.parametrize("n,L,ambiguous,path,megabytes", [
+    (1200, 9000, 0.095, "tc", 139.5), (1200, 9000, 0.095, "popc", 70.5), (300, 20000, 0.5, "tc", 61.0)],
+    ids=["packed", "popcount", "unpacked"])
+def test_run_without_room_for_event_offsets(n, L, ambiguous, path, megabytes):
+    from swifttn93_b200 import Options
+
+    o, got = Options(threshold=1000.0, mode="resolve", min_overlap=20), []
+    for budget in (0, megabytes):
+        eng = _engine(budget)
+        eng.set_count_path(path)
+        s = eng.upload(_codes(n, L, ambiguous), _names(n))
+        for _ in range(2):
+            body, summ = eng.run(s, o)
+            got.append((body, summ.json(n)))
+        eng.free(s)
+        eng.close()
+    assert all(g == got[0] for g in got)
