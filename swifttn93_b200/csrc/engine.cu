@@ -2487,6 +2487,7 @@ struct tn93g_ctx {
   // run descriptors, and the logarithm's band and candidate spread (tn93g_set_log_band)
   DevBuf und[2], undn, undwork, rdesc;
   double log_band = kLogBand, log_spread = kLogSpread;
+  std::vector<tn93g_server *> servers;  // on this context
 };
 
 namespace {
@@ -2513,13 +2514,17 @@ void release(tn93g_ctx *ctx, DevBuf &b)
   b.n = 0;
 }
 
-// Gives back the memory that only saves time, for a call that has no room without it: a run's event offsets (its pair stage
-// takes the fused kernel from then on, with the same results). Kernels get such a buffer's address from the context at each
-// launch, never from an earlier one. False when there was nothing to give.
+void server_reclaim(tn93g_server *srv);
+
+// Gives back the memory that only saves time, for a call that has no room without it: a run's and the servers' event offsets
+// (the pair stage takes the fused kernel from then on, with the same results) and the servers' larger chunks. Kernels get
+// such a buffer's address from the context or the server at each launch, never from an earlier one. False when there was
+// nothing to give.
 bool reclaim(tn93g_ctx *ctx)
 {
   const size_t before = ctx->used;
   release(ctx, ctx->ev2);
+  for (tn93g_server *s : ctx->servers) server_reclaim(s);
   return ctx->used < before;
 }
 
@@ -4801,6 +4806,21 @@ namespace {
 // reference's last row (three 64-column tiles each), 3.91 so.
 constexpr long kServerTcChunk = 512, kServerTcChunkMin = 128;
 
+// bytes of the records of a chunk of cols query columns
+size_t server_records(const tn93g_server *srv, long cols) { return (size_t)srv->Nref * cols * (srv->tc16 ? 16 : 32); }
+
+// The events' offsets and the larger chunk of records go back to the context. Should the smallest chunk, taken out of what
+// the larger one gave back, fail all the same, the server counts with POPC from then on (same results).
+void server_reclaim(tn93g_server *srv)
+{
+  tn93g_ctx *ctx = srv->ctx;
+  release(ctx, srv->ev2);
+  if (!srv->tc || srv->tc_chunk <= kServerTcChunkMin) return;
+  release(ctx, srv->tcagg);
+  srv->tc_chunk = kServerTcChunkMin;
+  srv->tc = ensure(ctx, srv->tcagg, server_records(srv, kServerTcChunkMin), true) == TN93G_OK;
+}
+
 // words of the statistics of a batch of nq queries: total, undecided, counters, error word, and per query 9 sums, 3 counts,
 // 4 bounds and the histogram
 size_t server_stats(size_t nq) { return 7 + nq * (9 + 3 + 4 + 3 * kHistBins); }
@@ -4833,6 +4853,7 @@ void tn93g_server_destroy(tn93g_server *srv)
     }
   if (srv->pin) cudaFreeHost(srv->pin);
   if (srv->hstat) cudaFreeHost(srv->hstat);
+  if (ctx) ctx->servers.erase(std::remove(ctx->servers.begin(), ctx->servers.end(), srv), ctx->servers.end());
   delete srv;
 }
 
@@ -4957,17 +4978,7 @@ int tn93g_server_create(tn93g_ctx *ctx, tn93g_server **out, const uint8_t *codes
   srv->ev_ref = evo[N];
   srv->ev_cap = srv->ev_ref + (size_t)max_batch_sequences * ((L + kEvPad - 1) / kEvPad * kEvPad);
   SV(ensure(ctx, srv->ev, std::max<size_t>(srv->ev_cap, 1) * sizeof(uint32_t)));
-  SV(ensure(ctx, srv->ev2, std::max<size_t>(srv->ev_cap, 1) * sizeof(uint2)));
   SVC(cudaMemcpyAsync(srv->evoff.p, evo.data(), (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-  pa.ev_off = (const uint32_t *)srv->evoff.p;
-  pa.ev = (uint32_t *)srv->ev.p;
-  pa.ev2 = (uint2 *)srv->ev2.p;
-  pa.ev2_Npad = (uint32_t)Np;
-  pa.three = (uint8_t *)srv->three.p;
-  if (srv->ev_ref) {
-    events_kernel<<<(unsigned)((N + kWarps - 1) / kWarps), 256, 0, st>>>(pa);
-    SVC(cudaGetLastError());
-  }
   // tables of the server's mode
   build_tables(ctx->h_tab, opts->mode, opts->subset);
   fill_pair_tables(*ctx->h_tab, rc.wplane, ctx->h_ptab);
@@ -5035,16 +5046,9 @@ int tn93g_server_create(tn93g_ctx *ctx, tn93g_server **out, const uint8_t *codes
     const size_t img = (size_t)srv->tc_KS * srv->tc_NB * kTcBlockBytes;
     // a chunk that holds the largest batch from any first column, or the smallest one where that does not fit
     srv->tc_chunk = std::min<long>(kServerTcChunk, std::max(kServerTcChunkMin, (max_batch_sequences + 127) / 64 * 64));
-    const size_t agg = (size_t)N * (srv->tc16 ? 16 : 32);
-    const bool room = ensure(ctx, srv->ohimg, img) == TN93G_OK;
-    // under a budget the larger chunk has to leave as much again for what batches grow (text, undecided lists)
-    if (ctx->budget && ctx->used + 2 * agg * srv->tc_chunk > ctx->budget) srv->tc_chunk = kServerTcChunkMin;
-    if (room && ensure(ctx, srv->tcagg, agg * srv->tc_chunk) != TN93G_OK) {
-      cudaGetLastError();
-      srv->tc_chunk = kServerTcChunkMin;
-    }
-    if (room && ensure(ctx, srv->tcagg, agg * srv->tc_chunk) == TN93G_OK &&
-        ensure(ctx, srv->tcerr, sizeof(unsigned long long)) == TN93G_OK) {
+    const bool room = ensure(ctx, srv->ohimg, img) == TN93G_OK && ensure(ctx, srv->tcerr, sizeof(unsigned long long)) == TN93G_OK;
+    if (room && ensure(ctx, srv->tcagg, server_records(srv, srv->tc_chunk), true) != TN93G_OK) srv->tc_chunk = kServerTcChunkMin;
+    if (room && ensure(ctx, srv->tcagg, server_records(srv, srv->tc_chunk)) == TN93G_OK) {
       srv->tc = true;
       srv->lin = weighted_mode(opts->mode);
       SV(tc_attr(ctx));
@@ -5057,17 +5061,26 @@ int tn93g_server_create(tn93g_ctx *ctx, tn93g_server **out, const uint8_t *codes
         SVC(cudaGetLastError());
       }
     } else {
-      for (DevBuf *b : {&srv->ohimg, &srv->tcagg, &srv->tcerr})
-        if (b->p) {
-          cudaFree(b->p);
-          ctx->used -= b->n;
-          b->p = nullptr;
-          b->n = 0;
-        }
+      for (DevBuf *b : {&srv->ohimg, &srv->tcagg, &srv->tcerr}) release(ctx, *b);
       ctx->err.clear();
     }
   }
+  // the events again as event_kernel reads them, where the pair stage takes it (pair_split) and there is room
+  if (srv->tc && !srv->lin && !rc.wplane && srv->ref_max_ev <= (uint32_t)kPackedMaxEvents && L * Np < (1l << 32)) {
+    const int r = ensure(ctx, srv->ev2, std::max<size_t>(srv->ev_cap, 1) * sizeof(uint2), true);
+    if (r != TN93G_ENOMEM) SV(r);
+  }
+  pa.ev_off = (const uint32_t *)srv->evoff.p;
+  pa.ev = (uint32_t *)srv->ev.p;
+  pa.ev2 = (uint2 *)srv->ev2.p;
+  pa.ev2_Npad = (uint32_t)Np;
+  pa.three = (uint8_t *)srv->three.p;
+  if (srv->ev_ref) {
+    events_kernel<<<(unsigned)((N + kWarps - 1) / kWarps), 256, 0, st>>>(pa);
+    SVC(cudaGetLastError());
+  }
   SVC(cudaStreamSynchronize(st));
+  ctx->servers.push_back(srv);
 #undef SV
 #undef SVC
   *out = srv;

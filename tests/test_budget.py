@@ -43,3 +43,20 @@ def test_run_without_room_for_event_offsets(n, L, ambiguous, path, megabytes):
         eng.free(s)
         eng.close()
     assert all(g == got[0] for g in got)
+
+
+@pytest.mark.parametrize("mode,servers,megabytes", [("resolve", 1, 86.0), ("average", 1, 86.0), ("resolve", 2, 210.3)])
+def test_server_without_room_for_offsets_and_larger_chunks(mode, servers, megabytes):
+    """One server, and two on one context of which the first has to give its extras back."""
+    from swifttn93_b200 import Fasta, Options, ResidentReference, synth
+
+    ref = Fasta(synth.to_fasta(_names(2000), _codes(2000, 3000, 0.1)))
+    queries = [Fasta(synth.to_fasta([f"q{k}_{i}" for i in range(n)], _codes(n, 3000, 0.1, k + 5)), expect_len=3000)
+               for k, n in enumerate((300, 200, 90))]
+    o, got = Options(threshold=1000.0, mode=mode, min_overlap=20), []
+    for budget in (0, megabytes):
+        eng = _engine(budget)
+        for res in [ResidentReference(eng, ref, o, 600, 4) for _ in range(servers)] * 2:
+            got.append([(b, s.json(ref.n, q.n, second_file=True)) for (b, s), q in zip(res.batch(queries), queries)])
+        eng.close()
+    assert all(g == got[0] for g in got)
