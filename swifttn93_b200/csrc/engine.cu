@@ -2421,7 +2421,14 @@ struct DevBuf {
   size_t n = 0;
 };
 
-constexpr int kBatchBufs = 64;
+// the buffers of tn93g_batch_run
+enum BatchBuf {
+  BB_CODES, BB_SEEN, BB_NN, BB_VARCOL, BB_PLANES, BB_CC, BB_CCT, BB_EVCOUNT, BB_EVOFF, BB_EV, BB_AGG, BB_SITE,
+  BB_NAMES, BB_NAMEOFF, BB_NAMELEN, BB_COUNTS, BB_DIST, BB_RQ, BB_RQN, BB_COUNTERS, BB_PDESC, BB_RDESC, BB_ROWDESC,
+  BB_TILES, BB_NEXT, BB_BLOCKS, BB_SBYTES, BB_SOFF, BB_SLINKS, BB_SSKIP, BB_SMAX, BB_RSUM, BB_RW, BB_HIST, BB_TOTAL,
+  BB_SCANTMP, BB_RED, BB_REDC, BB_FIRST, BB_FIRSTIDX, BB_OUT, BB_OH, BB_TCAGG, BB_TCDESC, BB_TCTILES, BB_TCERR,
+  BB_UND, BB_UNDN, BB_AMB, BB_SCANDESC, BB_PACKDESC, BB_TRDESC, BB_OHDESC, BB_BOFF, BB_EV2, BB_THREE, BB_SPLIT, BB_COUNT
+};
 constexpr int kMaxTcChunks = 48;         // row chunks of a band on the tensor-core count path
 // Pairs per chunk of the tensor-core path (count kernel, then pair kernel): 16 M pairs, 256 MB of 16-byte records.
 // Larger chunks amortise the persistent count kernel's pipeline fill and drain and the pair kernel's last wave
@@ -2476,7 +2483,7 @@ struct tn93g_ctx {
   double timings[8] = {0};
   long launches = 0;
   size_t dev_out_n = 0;
-  DevBuf bb[kBatchBufs];  // buffers of tn93g_batch_run (indexed by BatchBuf)
+  DevBuf bb[BB_COUNT];  // buffers of tn93g_batch_run (indexed by BatchBuf)
   int count_path = 1;  // clean-site counts: 0 popcounts on the CUDA cores, 1 tensor cores (tcgen05)
   int sms = 148;       // streaming multiprocessors of the device (persistent and grid-stride launches)
   DevBuf ohimg, tcagg;
@@ -2488,6 +2495,7 @@ struct tn93g_ctx {
   DevBuf und[2], undn, undwork, rdesc;
   double log_band = kLogBand, log_spread = kLogSpread;
   std::vector<tn93g_server *> servers;  // on this context
+  bool records_busy = false;  // a batch's pair stage has yet to read bb[BB_EV2] and bb[BB_TCAGG]
 };
 
 namespace {
@@ -2517,13 +2525,17 @@ void release(tn93g_ctx *ctx, DevBuf &b)
 void server_reclaim(tn93g_server *srv);
 
 // Gives back the memory that only saves time, for a call that has no room without it: a run's and the servers' event offsets
-// (the pair stage takes the fused kernel from then on, with the same results) and the servers' larger chunks. Kernels get
-// such a buffer's address from the context or the server at each launch, never from an earlier one. False when there was
-// nothing to give.
+// (the pair stage takes the fused kernel from then on, with the same results), the servers' larger chunks, and the records
+// that the last batch left. Kernels get such a buffer's address from the context or the server at each launch, never from an
+// earlier one. False when there was nothing to give.
 bool reclaim(tn93g_ctx *ctx)
 {
   const size_t before = ctx->used;
   release(ctx, ctx->ev2);
+  if (!ctx->records_busy) {
+    release(ctx, ctx->bb[BB_EV2]);
+    release(ctx, ctx->bb[BB_TCAGG]);
+  }
   for (tn93g_server *s : ctx->servers) server_reclaim(s);
   return ctx->used < before;
 }
@@ -5546,14 +5558,6 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
 // batched kernels over all alignments' rows. Each alignment's output equals its own tn93g_run byte for byte.
 namespace {
 
-enum BatchBuf {
-  BB_CODES, BB_SEEN, BB_NN, BB_VARCOL, BB_PLANES, BB_CC, BB_CCT, BB_EVCOUNT, BB_EVOFF, BB_EV, BB_AGG, BB_SITE,
-  BB_NAMES, BB_NAMEOFF, BB_NAMELEN, BB_COUNTS, BB_DIST, BB_RQ, BB_RQN, BB_COUNTERS, BB_PDESC, BB_RDESC, BB_ROWDESC,
-  BB_TILES, BB_NEXT, BB_BLOCKS, BB_SBYTES, BB_SOFF, BB_SLINKS, BB_SSKIP, BB_SMAX, BB_RSUM, BB_RW, BB_HIST, BB_TOTAL,
-  BB_SCANTMP, BB_RED, BB_REDC, BB_FIRST, BB_FIRSTIDX, BB_OUT, BB_OH, BB_TCAGG, BB_TCDESC, BB_TCTILES, BB_TCERR,
-  BB_UND, BB_UNDN, BB_AMB, BB_SCANDESC, BB_PACKDESC, BB_TRDESC, BB_OHDESC, BB_BOFF, BB_EV2, BB_THREE, BB_SPLIT, BB_COUNT
-};
-static_assert(BB_COUNT <= kBatchBufs, "batch buffer table");
 
 // Packing of a batch, one launch per step over all alignments: block b belongs to the alignment k with
 // off[k] <= b < off[k + 1] (off[] is the prefix sum of the alignments' block counts) and is its block b - off[k].
@@ -5695,9 +5699,9 @@ cudaError_t launch_pair_batch_t(int sms, bool wplane, bool gapmm, const PairArgs
 
 }  // namespace
 
-extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *alns, const tn93g_opts *opts,
-                               const int *rows_per_warp, int pair_blocks, tn93g_query_sink sink, void *user,
-                               tn93g_summary *sums)
+// records: alignments may take the records path, whose event offsets and wider records are taken where there is room
+static int batch_impl(tn93g_ctx *ctx, int K, const tn93g_alignment *alns, const tn93g_opts *opts, const int *rows_per_warp,
+                      int pair_blocks, tn93g_query_sink sink, void *user, tn93g_summary *sums, bool records)
 {
   if (!ctx || K <= 0 || !alns || !opts || !sums) return TN93G_EINVAL;
   for (int k = 0; k < K; k++) {
@@ -5903,7 +5907,8 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   // weighted operand image): all with variable columns on the tensor-core path but those with more than kPackedMaxEvents
   // events in a sequence, with an N plane under resolve (the batch makes no N word lists) or with a code matrix past 32-bit
   // offsets. 24 alignments of 50-2,000 x 900-3,000 in three modes: pair stage and replay 2.12 -> 0.93 ms. When its
-  // larger records do not fit, every alignment takes the fused kernel.
+  // larger records do not fit, or leave no room for what comes after them (tn93g_batch_run), every alignment takes the fused
+  // kernel.
   const bool use_tc = ctx->count_path == 1;
   std::vector<char> split(K, 0), lin(K, 0);
   std::vector<size_t> rec(K), ag_off(K + 1, 0);  // bytes of a pair's record; the alignments' records
@@ -5931,10 +5936,10 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
     if (nev >= (1ull << 32)) return TN93G_ETOOBIG;
     TRY(ensure(ctx, bb[BB_EV], std::max<size_t>(nev, 1) * sizeof(uint32_t)));
     if (may_split) {
-      TRY(ensure(ctx, bb[BB_EV2], std::max<size_t>(nev, 1) * sizeof(uint2)));
-      TRY(ensure(ctx, bb[BB_THREE], NR));
+      TRY(ensure(ctx, bb[BB_EV2], std::max<size_t>(nev, 1) * sizeof(uint2), true));
+      TRY(ensure(ctx, bb[BB_THREE], NR, true));
     }
-    if (use_tc) TRY(ensure(ctx, bb[BB_TCAGG], std::max<size_t>(ag_off[K], 16)));
+    if (use_tc) TRY(ensure(ctx, bb[BB_TCAGG], std::max<size_t>(ag_off[K], 16), may_split));
     return TN93G_OK;
   };
   // the pair stage's other large buffers come first, so that only the records path itself can be what does not fit
@@ -5947,15 +5952,9 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   }
   TRY(ensure(ctx, bb[BB_DIST], d_off[K] * sizeof(double)));
   TRY(ensure(ctx, bb[BB_RQ], q_off[K] * sizeof(unsigned long long)));
-  int planned = plan_events(use_tc);
-  if (use_tc && planned == TN93G_OK && ctx->budget) {  // under a budget, what comes after needs its share
-    size_t rest = (1 << 20) + NR * 512;                // lists and row arrays, then the operand images
-    for (int k = 0; k < K; k++)
-      rest += (size_t)(alns[k].n / 32 + 2) * ((RC[k].Lc + kTcStageK - 1) / kTcStageK) * kTcBlockBytes;
-    if (ctx->used + rest > ctx->budget) planned = TN93G_ENOMEM;
-  }
-  if (use_tc && planned != TN93G_OK && planned != TN93G_ETOOBIG) {
-    cudaGetLastError();
+  ctx->records_busy = true;
+  int planned = plan_events(use_tc && records);
+  if (use_tc && records && planned == TN93G_ENOMEM) {
     release(ctx, bb[BB_EV2]);
     release(ctx, bb[BB_TCAGG]);
     planned = plan_events(false);
@@ -6265,6 +6264,7 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
       CU(launch_pair(PD[k], (alns[k].n + kTile - 1) / kTile, alns[k].n, st));
       ctx->launches++;
     }
+  ctx->records_busy = false;  // what is launched from here on reads neither the records nor the offsets
   CU(cudaEventRecord(E[2], st));
   replay_batch_kernel<<<2 * ctx->sms, 256, 0, st>>>((const ReplayArgs *)bb[BB_RDESC].p, K);
   CU(cudaGetLastError());
@@ -6375,11 +6375,7 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
   bool any_emit = false;
   for (int k = 0; k < K; k++) any_emit |= RC[k].emit;
   if (any_emit && total) {
-    if (bb[BB_OUT].n < total && ensure(ctx, bb[BB_OUT], total + total / 4) != TN93G_OK) {
-      cudaGetLastError();
-      release(ctx, bb[BB_TCAGG]);  // the records are not read any more
-      TRY(ensure(ctx, bb[BB_OUT], total + total / 4));
-    }
+    if (bb[BB_OUT].n < total) TRY(ensure(ctx, bb[BB_OUT], total + total / 4));
     TRY(ensure_pinned(ctx, total));
     for (int k = 0; k < K; k++) RA[k].out = (char *)bb[BB_OUT].p;
     CU(cudaMemcpyAsync(bb[BB_ROWDESC].p, RA.data(), K * sizeof(RowArgs), cudaMemcpyHostToDevice, st));
@@ -6484,4 +6480,22 @@ extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *aln
       if (r) return TN93G_ESINK;
     }
   return TN93G_OK;
+}
+
+extern "C" int tn93g_batch_run(tn93g_ctx *ctx, int K, const tn93g_alignment *alns, const tn93g_opts *opts,
+                               const int *rows_per_warp, int pair_blocks, tn93g_query_sink sink, void *user,
+                               tn93g_summary *sums)
+{
+  if (!ctx) return TN93G_EINVAL;
+  int r = batch_impl(ctx, K, alns, opts, rows_per_warp, pair_blocks, sink, user, sums, true);
+  // no room for a later buffer beside the records path's (nothing has reached the sink by then): once more without it
+  if (r == TN93G_ENOMEM && ctx->records_busy) {
+    release(ctx, ctx->bb[BB_EV2]);
+    release(ctx, ctx->bb[BB_TCAGG]);
+    ctx->records_busy = false;
+    ctx->err.clear();
+    r = batch_impl(ctx, K, alns, opts, rows_per_warp, pair_blocks, sink, user, sums, false);
+  }
+  ctx->records_busy = false;
+  return r;
 }

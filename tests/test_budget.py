@@ -60,3 +60,21 @@ def test_server_without_room_for_offsets_and_larger_chunks(mode, servers, megaby
             got.append([(b, s.json(ref.n, q.n, second_file=True)) for (b, s), q in zip(res.batch(queries), queries)])
         eng.close()
     assert all(g == got[0] for g in got)
+
+
+def test_batch_whose_records_leave_no_room_for_what_follows():
+    """A batch of which every alignment runs again alone (a logarithm band of half a unit lists more pairs than the batch's
+    list holds): the larger records are given back for those runs."""
+    from swifttn93_b200 import HostAlignment, Options
+
+    shapes = ((50, 900), (700, 2500), (900, 1500), (1100, 2900), (333, 1111))
+    alns = [HostAlignment(_codes(n, L, 0.05, n), _names(n)) for n, L in shapes]
+    opts = [Options(threshold=1000.0, mode=m, resolve_fraction=0.05, min_overlap=20)
+            for m in ("resolve", "average", "resolve", "resolve", "gapmm")]
+    got = []
+    for budget in (0, 380.2):
+        eng = _engine(budget)
+        eng.set_log_band(0.5, 2.0**34)
+        got.append([(b, s.json(n)) for (b, s), (n, _) in zip(eng.batch_run(alns, opts), shapes)])
+        eng.close()
+    assert got[0] == got[1]
