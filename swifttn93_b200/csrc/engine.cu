@@ -2465,6 +2465,7 @@ struct tn93g_ctx {
   cudaStream_t copy_stream = nullptr;   // device->host copies of finished bands
   cudaStream_t write_stream = nullptr;  // text writers of finished bands (beside the next bands' kernels)
   cudaEvent_t evw0[2], evw1[2], evc0[2], evc1[2];
+  cudaEvent_t evrow[2];  // per band parity: its text is written
   cudaEvent_t evk[2][5];  // per band parity: start, after pair, after replay, after stats+sums+scan, stats on host
   cudaEvent_t evcnt[2][2 * kMaxTcChunks];  // per band parity: around each chunk's tensor-core count kernel
   DevBuf out2[2], total;
@@ -2495,6 +2496,7 @@ struct tn93g_ctx {
   DevBuf und[2], undn, undwork, rdesc;
   double log_band = kLogBand, log_spread = kLogSpread;
   std::vector<tn93g_server *> servers;  // on this context
+  bool bands_busy = false;    // a run is using its band buffers
   bool records_busy = false;  // a batch's pair stage has yet to read bb[BB_EV2] and bb[BB_TCAGG]
 };
 
@@ -2525,8 +2527,8 @@ void release(tn93g_ctx *ctx, DevBuf &b)
 void server_reclaim(tn93g_server *srv);
 
 // Gives back the memory that only saves time, for a call that has no room without it: a run's and the servers' event offsets
-// (the pair stage takes the fused kernel from then on, with the same results), the servers' larger chunks, and the records
-// that the last batch left. Kernels get such a buffer's address from the context or the server at each launch, never from an
+// (the pair stage takes the fused kernel from then on, with the same results), the servers' larger chunks, the records that
+// the last batch left, and the band and text buffers that the last run left. Kernels get such a buffer's address from the context or the server at each launch, never from an
 // earlier one. False when there was nothing to give.
 bool reclaim(tn93g_ctx *ctx)
 {
@@ -2536,6 +2538,9 @@ bool reclaim(tn93g_ctx *ctx)
     release(ctx, ctx->bb[BB_EV2]);
     release(ctx, ctx->bb[BB_TCAGG]);
   }
+  if (!ctx->bands_busy)
+    for (DevBuf *b : {&ctx->dist, &ctx->dcode, &ctx->tcagg, &ctx->rq, &ctx->und[0], &ctx->und[1], &ctx->out2[0], &ctx->out2[1]})
+      release(ctx, *b);
   for (tn93g_server *s : ctx->servers) server_reclaim(s);
   return ctx->used < before;
 }
@@ -2741,19 +2746,26 @@ int resolve_listed(tn93g_ctx *ctx, const ReplayArgs *d_descs, const unsigned lon
                    cudaStream_t st)
 {
   if (!n) return TN93G_OK;
-  TRY(ensure(ctx, ctx->undwork, (size_t)n * sizeof(UndEntry)));
+  unsigned piece = n;  // pairs at a time: all, or as many as there is room for
+  int r;
+  while ((r = ensure(ctx, ctx->undwork, (size_t)piece * sizeof(UndEntry))) == TN93G_ENOMEM && piece > 4096) piece = (piece + 1) / 2;
+  TRY(r);
   UndEntry *dw = (UndEntry *)ctx->undwork.p;
-  und_args_kernel<<<(unsigned)std::min<unsigned long>((n + kWarps - 1) / kWarps, 8ul * ctx->sms), 256, 0, st>>>(
-      d_descs, d_list, n, dw);
-  CU(cudaGetLastError());
-  std::vector<UndEntry> h(n);
-  CU(cudaMemcpyAsync(h.data(), dw, (size_t)n * sizeof(UndEntry), cudaMemcpyDeviceToHost, st));
-  CU(cudaStreamSynchronize(st));
-  host_logs(h);
-  CU(cudaMemcpyAsync(dw, h.data(), (size_t)n * sizeof(UndEntry), cudaMemcpyHostToDevice, st));
-  und_finish_kernel<<<(n + 255) / 256, 256, 0, st>>>(d_descs, dw, n);
-  CU(cudaGetLastError());
-  ctx->launches += 2;
+  std::vector<UndEntry> h;
+  for (size_t at = 0; at < n; at += piece) {
+    const unsigned m = (unsigned)std::min<size_t>(piece, n - at);
+    und_args_kernel<<<(unsigned)std::min<unsigned long>((m + kWarps - 1) / kWarps, 8ul * ctx->sms), 256, 0, st>>>(
+        d_descs, d_list + 2 * at, m, dw);
+    CU(cudaGetLastError());
+    h.resize(m);
+    CU(cudaMemcpyAsync(h.data(), dw, (size_t)m * sizeof(UndEntry), cudaMemcpyDeviceToHost, st));
+    CU(cudaStreamSynchronize(st));
+    host_logs(h);
+    CU(cudaMemcpyAsync(dw, h.data(), (size_t)m * sizeof(UndEntry), cudaMemcpyHostToDevice, st));
+    und_finish_kernel<<<(m + 255) / 256, 256, 0, st>>>(d_descs, dw, m);
+    CU(cudaGetLastError());
+    ctx->launches += 2;
+  }
   return TN93G_OK;
 }
 
@@ -3026,7 +3038,8 @@ int tn93g_create(tn93g_ctx **out, int device, size_t hbm_budget)
       if (cudaEventCreate(&e) != cudaSuccess) rc = TN93G_ECUDA;
     for (int q = 0; q < 2; q++) {
       if (cudaEventCreate(&ctx->evw0[q]) != cudaSuccess || cudaEventCreate(&ctx->evw1[q]) != cudaSuccess ||
-          cudaEventCreate(&ctx->evc0[q]) != cudaSuccess || cudaEventCreate(&ctx->evc1[q]) != cudaSuccess)
+          cudaEventCreate(&ctx->evc0[q]) != cudaSuccess || cudaEventCreate(&ctx->evc1[q]) != cudaSuccess ||
+          cudaEventCreateWithFlags(&ctx->evrow[q], cudaEventDisableTiming) != cudaSuccess)
         rc = TN93G_ECUDA;
       for (auto &e : ctx->evk[q])
         if (cudaEventCreate(&e) != cudaSuccess) rc = TN93G_ECUDA;
@@ -3079,7 +3092,7 @@ void tn93g_destroy(tn93g_ctx *ctx)
   for (int q = 0; q < 2; q++) {
     if (ctx->out2[q].p) cudaFree(ctx->out2[q].p);
     if (ctx->pin2[q]) cudaFreeHost(ctx->pin2[q]);
-    for (cudaEvent_t e : {ctx->evw0[q], ctx->evw1[q], ctx->evc0[q], ctx->evc1[q]})
+    for (cudaEvent_t e : {ctx->evw0[q], ctx->evw1[q], ctx->evc0[q], ctx->evc1[q], ctx->evrow[q]})
       if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->evk[q])
       if (e) cudaEventDestroy(e);
@@ -3510,6 +3523,11 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   rc.log_band = ctx->log_band;
   rc.log_spread = ctx->log_spread;
   rc.resolve_all = (flags & kRunResolveAll) != 0 || ctx->exact_sums;
+  struct Busy {  // (an exact-sums pass is a run inside a run)
+    bool &flag, was;
+    ~Busy() { flag = was; }
+  } busy = {ctx->bands_busy, ctx->bands_busy};
+  ctx->bands_busy = true;
   bool fault_pending = ctx->fault == TN93G_FAULT_SKIP_FILL;  // injected into the first count launch only
   ctx->fault = TN93G_FAULT_NONE;
   const bool hyphy = rc.emit && opts->format == TN93G_HYPHY;
@@ -3722,30 +3740,39 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
   // the copies run back to back), and taper at the end (half of what is left, down to 1/8), so that the first copy
   // starts early and the last one, which nothing overlaps, is short. When the first band shows that little is
   // reported, there is nothing to overlap and the rest runs as large bands (below).
-  std::vector<std::pair<long, long>> bands;
-  auto plan_bands = [&](long from, long target, long cap, bool ramps) {
-    long left = 0;
-    for (long r = from; r < upper; r++) left += rc.cross ? ncols : (N - r - 1);
-    for (long r0 = from; r0 < upper;) {
+  using Bands = std::vector<std::pair<long, long>>;
+  auto row_pairs = [&](long r) { return rc.cross ? ncols : N - r - 1; };
+  auto count_pairs = [&](long b, long e) {
+    long p = 0;
+    for (long r = b; r < e; r++) p += row_pairs(r);
+    return p;
+  };
+  // the rows from `from` on in bands of target pairs and at most cap pair slots; step: place in the ramp of the first one
+  auto plan_bands = [&](long from, long target, long cap, bool ramps, int step) {
+    Bands out;
+    long left = count_pairs(from, upper);
+    for (long r0 = from; r0 < upper; step++) {
       long tgt = target;
       if (ramps) {
-        const double ramp = std::pow(1.4, (double)bands.size()) / 16.0;
+        const double ramp = std::pow(1.4, (double)step) / 16.0;
         if (ramp < 1.0) tgt = std::max<long>(1, (long)((double)target * ramp));
         if (left < 2 * target) tgt = std::min(tgt, std::max(target / 8, left / 2));
       }
       long r = r0, pairs = 0;
       while (r < upper && (r == r0 || ((r - r0 + 1) * ncols <= cap && pairs < tgt && r - r0 < 65535l * kTile))) {
-        pairs += rc.cross ? ncols : (N - r - 1);
+        pairs += row_pairs(r);
         r++;
       }
-      bands.push_back({r0, r});
+      out.push_back({r0, r});
       left -= pairs;
       r0 = r;
     }
+    return out;
   };
-  constexpr long kBigSlots = 64l << 20;  // pair slots of a band that need not overlap a copy (512 MB of distances)
-  plan_bands(row_begin, (stream_text || rc.resolve_all) ? band_pairs : (1l << 62),
-             (stream_text || rc.resolve_all) ? (16l << 20) : kBigSlots, stream_text);
+  constexpr long kBigSlots = 64l << 20;    // pair slots of a band that need not overlap a copy (512 MB of distances)
+  constexpr long kSmallSlots = 16l << 20;  // of the other bands
+  Bands bands = (stream_text || rc.resolve_all) ? plan_bands(row_begin, band_pairs, kSmallSlots, stream_text, 0)
+                                                : plan_bands(row_begin, 1l << 62, kBigSlots, false, 0);
   const long maxseg = std::max<long>(1, (ncols + kSeg - 1) / kSeg);
   if (hyphy) {
     TRY(ensure(ctx, ctx->hy, (size_t)N * N * sizeof(double)));
@@ -3753,64 +3780,73 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     CU(cudaGetLastError());
     ctx->launches++;
   }
-  // per band parity (double-buffered): distances, segment statistics, row sums; the replay queue is per band. Sized for
-  // the largest of the bands from the first one on; called again, with nothing in flight, when the schedule changes.
   const int tc16 = 32 * L < 65536;  // the final x16 aggregates fit 16-bit lanes
   long band = 1, nseg = 1;
   size_t dslots = 1, stat_stride = 0;
-  std::vector<std::vector<std::pair<long, long>>> band_chunks;  // the tensor-core path's row chunks per band
+  std::vector<Bands> band_chunks;  // the tensor-core path's row chunks per band
   int nchunks[2] = {0, 0};
   unsigned und_cap_par[2] = {0, 0};  // grown per parity when a band lists more
   char *d_pstats = nullptr;          // the device's address of the statistics' staging
-  auto size_buffers = [&](size_t first) -> int {
-    band = 1;
-    for (size_t b = first; b < bands.size(); b++) band = std::max(band, bands[b].second - bands[b].first);
+  // the row chunks of the bands from `first` on, boundaries on the count kernel's 32-row tiles; returns the pair slots of the
+  // largest one
+  auto plan_chunks = [&](size_t first) {
+    band_chunks.resize(bands.size());
+    size_t slots = 1;
+    for (size_t b = first; b < bands.size(); b++) {
+      band_chunks[b].clear();
+      if (!use_tc) continue;
+      const long r0 = bands[b].first, r1 = bands[b].second;
+      static const long chunk_pairs = [] {
+        const char *e = getenv("TN93G_TC_CHUNK_PAIRS");  // tuning knob: pairs per count/pair chunk
+        return e && atol(e) > 0 ? atol(e) : kTcChunkPairs;
+      }();
+      const long target = std::max(chunk_pairs, (count_pairs(r0, r1) + kMaxTcChunks - 2) / (kMaxTcChunks - 1));
+      for (long c0 = r0; c0 < r1;) {
+        long c1 = c0, pairs = 0;
+        while (c1 < r1 && (c1 == c0 || pairs < target)) {
+          pairs += row_pairs(c1);
+          c1++;
+        }
+        c1 = std::min(r1, (c1 + kTcRows - 1) / kTcRows * kTcRows);
+        if ((int)band_chunks[b].size() == kMaxTcChunks - 1) c1 = r1;  // never more chunks than events
+        band_chunks[b].push_back({c0, c1});
+        slots = std::max(slots, (size_t)(c1 - c0) * ncols);
+        c0 = c1;
+      }
+    }
+    return slots;
+  };
+  auto max_rows = [](const Bands &v, size_t first) {
+    long n = 1;
+    for (size_t b = first; b < v.size(); b++) n = std::max(n, v[b].second - v[b].first);
+    return n;
+  };
+  auto und_entries = [&](size_t slots) {
+    return (unsigned)std::min<size_t>(rc.resolve_all ? slots : std::max<size_t>(4096, slots / 64), 0xFFFFFFF0u);
+  };
+  // per band parity (double-buffered): distances, segment statistics, row sums; the replay queue is per band
+  auto band_buffers = [&](long rows, size_t chunk_slots) {
+    const size_t slots = (size_t)rows * ncols, segs = (size_t)rows * maxseg, w = sizeof(unsigned long long);
+    const size_t und = (size_t)und_entries(slots) * 2 * w;
+    std::vector<std::pair<DevBuf *, size_t>> v = {{&ctx->dist, 2 * slots * w},       {&ctx->rq, slots * w},
+                                                  {&ctx->rbytes, 2 * segs * w},      {&ctx->roff, 2 * segs * w},
+                                                  {&ctx->rsum, 2 * (size_t)rows * 3 * w}, {&ctx->rw, 2 * (size_t)rows * 3 * w},
+                                                  {&ctx->rmax, 2 * segs * 3 * w},    {&ctx->rlinks, 2 * segs * w},
+                                                  {&ctx->rskip, 2 * segs * w},       {&ctx->und[0], und},
+                                                  {&ctx->und[1], und}};
+    if (rc.emit && !hyphy) v.push_back({&ctx->dcode, 2 * slots * sizeof(uint32_t)});
+    if (use_tc) v.push_back({&ctx->tcagg, chunk_slots * (tc16 ? 16 : 32)});
+    return v;
+  };
+  // Sizes them for the largest of the bands from the first one on; called again, with nothing in flight, when the schedule
+  // changes. spare: the caller can go on without.
+  auto size_buffers = [&](size_t first, bool spare) -> int {
+    const size_t chunk_slots = plan_chunks(first);
+    band = max_rows(bands, first);
     nseg = band * maxseg;
     dslots = (size_t)band * ncols;
-    TRY(ensure(ctx, ctx->dist, 2 * dslots * sizeof(double)));
-    if (rc.emit && !hyphy) TRY(ensure(ctx, ctx->dcode, 2 * dslots * sizeof(uint32_t)));
-    // chunk boundaries on the count kernel's 32-row tiles
-    band_chunks.assign(bands.size(), {});
-    size_t chunk_slots = 1;
-    if (use_tc) {
-      for (size_t b = first; b < bands.size(); b++) {
-        const long r0 = bands[b].first, r1 = bands[b].second;
-        long bp = 0;
-        for (long r = r0; r < r1; r++) bp += rc.cross ? ncols : (N - r - 1);
-        static const long chunk_pairs = [] {
-          const char *e = getenv("TN93G_TC_CHUNK_PAIRS");  // tuning knob: pairs per count/pair chunk
-          return e && atol(e) > 0 ? atol(e) : kTcChunkPairs;
-        }();
-        const long target = std::max(chunk_pairs, (bp + kMaxTcChunks - 2) / (kMaxTcChunks - 1));
-        for (long c0 = r0; c0 < r1;) {
-          long c1 = c0, pairs = 0;
-          while (c1 < r1 && (c1 == c0 || pairs < target)) {
-            pairs += rc.cross ? ncols : (N - c1 - 1);
-            c1++;
-          }
-          c1 = std::min(r1, (c1 + kTcRows - 1) / kTcRows * kTcRows);
-          if ((int)band_chunks[b].size() == kMaxTcChunks - 1) c1 = r1;  // never more chunks than events
-          band_chunks[b].push_back({c0, c1});
-          chunk_slots = std::max(chunk_slots, (size_t)(c1 - c0) * ncols);
-          c0 = c1;
-        }
-      }
-      TRY(ensure(ctx, ctx->tcagg, chunk_slots * (tc16 ? 16 : 32)));
-    }
-    TRY(ensure(ctx, ctx->rq, dslots * sizeof(unsigned long long)));
-    TRY(ensure(ctx, ctx->rbytes, 2 * nseg * sizeof(unsigned long long)));
-    TRY(ensure(ctx, ctx->roff, 2 * nseg * sizeof(unsigned long long)));
-    TRY(ensure(ctx, ctx->rsum, 2 * band * 3 * sizeof(double)));
-    TRY(ensure(ctx, ctx->rw, 2 * band * 3 * sizeof(double)));
-    TRY(ensure(ctx, ctx->rmax, 2 * nseg * 3 * sizeof(double)));
-    TRY(ensure(ctx, ctx->rlinks, 2 * nseg * sizeof(long long)));
-    TRY(ensure(ctx, ctx->rskip, 2 * nseg * sizeof(long long)));
-    const unsigned und_cap = (unsigned)std::min<size_t>(rc.resolve_all ? dslots : std::max<size_t>(4096, dslots / 64),
-                                                        0xFFFFFFF0u);
-    for (int q = 0; q < 2; q++) {
-      TRY(ensure(ctx, ctx->und[q], (size_t)und_cap * 2 * sizeof(unsigned long long)));
-      und_cap_par[q] = und_cap;
-    }
+    for (const auto &b : band_buffers(band, chunk_slots)) TRY(ensure(ctx, *b.first, b.second, spare));
+    for (unsigned &cap : und_cap_par) cap = und_entries(dslots);
     // pinned staging of a band's statistics: row sums and weights (3 each at most), total bytes, the band's histogram and
     // totals, its undecided count and the count kernel's error word
     stat_stride = (size_t)band * 6 * sizeof(double) + (3 + kBandWords) * sizeof(unsigned long long);
@@ -3818,7 +3854,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     CU(cudaHostGetDevicePointer((void **)&d_pstats, ctx->pstats, 0));
     return TN93G_OK;
   };
-  TRY(size_buffers(0));
+  TRY(size_buffers(0, false));
   TRY(ensure(ctx, ctx->rqn, sizeof(unsigned)));
   // the run's scalars: 4 counters, the 3 summary units' bounds (4 words each), the count kernel's error word
   TRY(ensure(ctx, ctx->counters, kRunScalars * sizeof(unsigned long long)));
@@ -3937,7 +3973,7 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     const long r0 = bands[bi].first, r1 = bands[bi].second, nr = r1 - r0;
     cudaEvent_t *K = ctx->evk[par];
     // this parity's distances, codes and row arrays are read by band bi - 2's text writer on the write stream
-    if (bi >= 2 && stream_text) CU(cudaStreamWaitEvent(st, ctx->evw1[par], 0));
+    if (bi >= 2 && stream_text) CU(cudaStreamWaitEvent(st, ctx->evrow[par], 0));
     CU(cudaEventRecord(K[0], st));
     CU(cudaMemsetAsync(ctx->rqn.p, 0, sizeof(unsigned), st));
     CU(cudaMemsetAsync((unsigned long long *)ctx->undn.p + par, 0, sizeof(unsigned long long), st));
@@ -4057,17 +4093,17 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
     CU(cudaEventRecord(K[2], st));
     return enqueue_rows(bi);
   };
-  // bands whose text is on its way to the host: parities, oldest first
-  int pend_par[2] = {0, 0}, pend_n = 0;
+  // texts on their way to the host: their buffers (out2, pin2), oldest first
+  int pend_buf[2] = {0, 0}, pend_n = 0, next_buf = 0;
   size_t pend_bytes[2] = {0, 0};
-  bool par_used[2] = {false, false};
-  // TN93G_TRACE=1: one stderr line per delivered band (device milliseconds from the run's first event: write
+  bool buf_used[2] = {false, false};
+  // TN93G_TRACE=1: one stderr line per delivered text (device milliseconds from the run's first event: write
   // start and end, copy start and end; host milliseconds when the copy was seen complete), for pipeline tuning
   static const bool trace = getenv("TN93G_TRACE") != nullptr;
   const auto host0 = std::chrono::steady_clock::now();
   int delivered = 0;
   auto deliver_oldest = [&]() -> int {
-    const int q = pend_par[0];
+    const int q = pend_buf[0];
     CU(cudaEventSynchronize(ctx->evc1[q]));
     CU(cudaEventElapsedTime(&ms, ctx->evw0[q], ctx->evw1[q]));
     ctx->timings[4] += ms;
@@ -4080,19 +4116,94 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
       CU(cudaEventElapsedTime(&c0, E[0], ctx->evc0[q]));
       CU(cudaEventElapsedTime(&c1, E[0], ctx->evc1[q]));
       const double h = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - host0).count();
-      fprintf(stderr, "tn93g trace: band %d bytes %zu write %.3f-%.3f copy %.3f-%.3f host %.3f\n", delivered++,
+      fprintf(stderr, "tn93g trace: text %d bytes %zu write %.3f-%.3f copy %.3f-%.3f host %.3f\n", delivered++,
               pend_bytes[q], w0, w1, c0, c1, h);
     }
-    pend_par[0] = pend_par[1];
+    pend_buf[0] = pend_buf[1];
     pend_n--;
     if (sink && sink(user, (const char *)ctx->pin2[q], pend_bytes[q])) return TN93G_ESINK;
     return TN93G_OK;
   };
-  auto band_pair_count = [&](int bi) -> long {
-    long p = 0;
-    for (long r = bands[bi].first; r < bands[bi].second; r++) p += rc.cross ? ncols : (N - r - 1);
-    return p;
+  // Text of band bi: its rows [ra, rb), the n bytes from byte `at` of the band's text on. It is written on the write stream,
+  // beside the next band's kernels, once the band's statistics are final (K[4]), then copied on the copy stream. The text
+  // that holds the same buffer pair goes to the sink first: its copy has then left the device buffer, the sink has taken the
+  // pinned buffer, and its events are free to record this one's. Meanwhile the copy engine works on the text in between.
+  auto send_text = [&](int bi, long ra, long rb, size_t at, size_t n) -> int {
+    const int q = next_buf;
+    for (;;) {
+      bool held = false;
+      for (int k = 0; k < pend_n; k++) held |= pend_buf[k] == q;
+      if (!held) break;
+      TRY(deliver_oldest());
+    }
+    TRY(ensure(ctx, ctx->out2[q], n));
+    TRY(ensure_pinned_at(ctx, ctx->pin2[q], ctx->pin2_n[q], n));
+    RowArgs RA = row_args(bi);
+    RA.r1 = RA.r0 + rb;
+    RA.r0 += ra;
+    RA.nrows = rb - ra;
+    RA.dist += (size_t)ra * ncols;
+    RA.dcode += (size_t)ra * ncols;
+    RA.seg_bytes += ra * maxseg;
+    RA.seg_off += ra * maxseg;
+    RA.out = (char *)((uintptr_t)ctx->out2[q].p - at);  // seg_off counts from the band's first byte
+    const cudaStream_t ws = ctx->write_stream;
+    CU(cudaStreamWaitEvent(ws, ctx->evk[bi & 1][4], 0));
+    if (buf_used[q]) CU(cudaStreamWaitEvent(ws, ctx->evc1[q], 0));
+    CU(cudaEventRecord(ctx->evw0[q], ws));
+    write_kernel<<<dim3((unsigned)((rb - ra + kWarps - 1) / kWarps), (unsigned)maxseg), 256, 0, ws>>>(RA);
+    CU(cudaGetLastError());
+    ctx->launches++;
+    CU(cudaEventRecord(ctx->evw1[q], ws));
+    CU(cudaStreamWaitEvent(ctx->copy_stream, ctx->evw1[q], 0));
+    CU(cudaEventRecord(ctx->evc0[q], ctx->copy_stream));
+    CU(cudaMemcpyAsync(ctx->pin2[q], ctx->out2[q].p, n, cudaMemcpyDeviceToHost, ctx->copy_stream));
+    CU(cudaEventRecord(ctx->evc1[q], ctx->copy_stream));
+    buf_used[q] = true;
+    pend_bytes[q] = n;
+    pend_buf[pend_n++] = q;
+    next_buf ^= 1;
+    return TN93G_OK;
   };
+  // The whole text of band bi, tot bytes: in pieces of whole rows where a band larger than the streaming ones reports much (a
+  // band of 64 M slots may have gigabytes, of which a piece is copied while the next is written), and where the buffers for
+  // more do not fit.
+  constexpr size_t kTextPiece = 64 << 20;
+  auto send_band = [&](int bi, size_t tot) -> int {
+    const long nr = bands[bi].second - bands[bi].first;
+    const bool large = count_pairs(bands[bi].first, bands[bi].second) > band_pairs + ncols;
+    size_t limit = large ? std::min(tot, kTextPiece) : tot;
+    std::vector<unsigned long long> off;  // where each row's text starts, when it is taken in pieces
+    for (long ra = 0; ra < nr;) {
+      long rb = nr;
+      size_t at = 0, n = tot;
+      if (limit < tot) {
+        if (off.empty()) {
+          off.resize(nr + 1);
+          CU(cudaMemcpy2DAsync(off.data(), sizeof off[0], row_args(bi).seg_off, maxseg * sizeof off[0], sizeof off[0], nr,
+                               cudaMemcpyDeviceToHost, ctx->write_stream));
+          CU(cudaStreamSynchronize(ctx->write_stream));
+          off[nr] = tot;
+        }
+        at = off[ra];
+        rb = std::max(ra + 1, (long)(std::upper_bound(off.begin() + ra, off.end(), at + limit) - off.begin()) - 1);
+        n = off[rb] - at;
+      }
+      if (n) {
+        const int r = send_text(bi, ra, rb, at, n);
+        if (r == TN93G_ENOMEM && rb - ra > 1) {
+          ctx->err.clear();
+          limit = n / 2;
+          continue;
+        }
+        TRY(r);
+      }
+      ra = rb;
+    }
+    CU(cudaEventRecord(ctx->evrow[bi & 1], ctx->write_stream));
+    return TN93G_OK;
+  };
+  size_t band_text = 0;  // bytes that the last finished band reported
   // statistics of band bi in row order, then its text: written on the compute stream (behind the next band's
   // kernels) and copied to the host on the copy stream
   auto finish = [&](int bi) -> int {
@@ -4167,11 +4278,12 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
         }
       }
     const unsigned long long tot = *h.total;
-    if (!(rc.emit && !hyphy && tot)) return TN93G_OK;
+    band_text = rc.emit && !hyphy ? tot : 0;
+    if (!band_text) return TN93G_OK;
     sum->output_bytes += tot;
-    RowArgs RA = row_args(bi);
-    const dim3 wgrid((unsigned)((nr + kWarps - 1) / kWarps), (unsigned)maxseg);
     if (to_device) {
+      RowArgs RA = row_args(bi);
+      const dim3 wgrid((unsigned)((nr + kWarps - 1) / kWarps), (unsigned)maxseg);
       TRY(ensure_keep(ctx, ctx->out, dev_off + tot, dev_off));
       RA.out = (char *)ctx->out.p + dev_off;
       CU(cudaEventRecord(ctx->evw0[0], st));
@@ -4185,68 +4297,76 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
       dev_off += tot;
       return TN93G_OK;
     }
-    // The band's text is written on the write stream, beside the next band's kernels, once its statistics are final
-    // (K[4]), then copied on the copy stream. The older band of this parity (or, when the bands between them wrote
-    // no text, an even older one) goes to the sink first: its copy has then left the device buffer, the sink has
-    // taken the pinned buffer, and its write and copy events are free to record this band's. Meanwhile the copy
-    // engine works on the band in between.
-    for (;;) {
-      bool held = false;
-      for (int q = 0; q < pend_n; q++) held |= pend_par[q] == par;
-      if (!held) break;
-      TRY(deliver_oldest());
-    }
-    const cudaStream_t ws = ctx->write_stream;
-    TRY(ensure(ctx, ctx->out2[par], tot));
-    TRY(ensure_pinned_at(ctx, ctx->pin2[par], ctx->pin2_n[par], tot));
-    RA.out = (char *)ctx->out2[par].p;
-    CU(cudaStreamWaitEvent(ws, K[4], 0));
-    if (par_used[par]) CU(cudaStreamWaitEvent(ws, ctx->evc1[par], 0));
-    CU(cudaEventRecord(ctx->evw0[par], ws));
-    write_kernel<<<wgrid, 256, 0, ws>>>(RA);
-    CU(cudaGetLastError());
-    ctx->launches++;
-    CU(cudaEventRecord(ctx->evw1[par], ws));
-    CU(cudaStreamWaitEvent(ctx->copy_stream, ctx->evw1[par], 0));
-    CU(cudaEventRecord(ctx->evc0[par], ctx->copy_stream));
-    CU(cudaMemcpyAsync(ctx->pin2[par], ctx->out2[par].p, tot, cudaMemcpyDeviceToHost, ctx->copy_stream));
-    CU(cudaEventRecord(ctx->evc1[par], ctx->copy_stream));
-    par_used[par] = true;
-    pend_bytes[par] = tot;
-    pend_par[pend_n++] = par;
-    return TN93G_OK;
+    return send_band(bi, tot);
   };
   // Band bi + 1's kernels are queued before band bi is finished, so the device computes while the host takes band
   // bi's statistics; texts reach the sink when their pinned buffer is needed again, or at the end (at most one band
   // per parity waits).
-  // A streamed run that reports few pairs (the first band gives less than 2 bytes of text a pair, so copying a band takes
-  // less than a sixth of computing it) has nothing to overlap: what is left after the second band runs as large bands,
-  // whose kernels fill the GPU (each kernel's last wave, the row sums' chains and the replays cost a band about as much
-  // whatever its size: 6,700 x 1,500 at -t 0.015 took 17 bands and 7.2 ms of device time, 4.9 ms so). If the larger
-  // buffers do not fit, the small bands go on.
+  // A streamed run whose first band reports few pairs (less than 2 bytes of text a pair, so copying a band takes less than a
+  // sixth of computing it) has nothing to overlap: what is left after the second runs as large bands, whose kernels fill the GPU (each
+  // kernel's last wave, the row sums' chains and the replays cost a band about as much whatever its size: 6,700 x 1,500 at
+  // -t 0.015 took 17 bands and 7.2 ms of device time, 4.9 ms so). The first rows may not be like the rest: the first large
+  // band takes a quarter of what is left, so that, where it reports much, the next one's kernels run under its copies, and
+  // what is not queued by then goes on in small bands (6,700 x 1,500, 100 unrelated rows and the rest linked: 8.5 ms, 9.6
+  // with the rest in one band, 9.7 in small bands; nothing linked: 3.88, 3.91 and 7.05). Less than four small bands' worth
+  // is one band: another would cost more than it could overlap (3,001 x 1,065: 1.36 and 1.49 ms, 4,000 x 1,500: 1.91 and
+  // 1.96). If the larger buffers do not fit, the small bands go on.
   const bool may_grow = stream_text && !rc.resolve_all && !forced_band;
+  auto few = [&](int bi) { return band_text < 2 * (size_t)count_pairs(bands[bi].first, bands[bi].second); };
+  // the rows from band 2 on in large bands, with buffers for them; where those do not fit the schedule stays as it was
+  bool large = false;
+  auto grow_bands = [&]() -> int {
+    const Bands small = bands;
+    const long from = small[2].first;
+    bool tried = false;
+    int r = TN93G_ENOMEM;
+    for (long cap = kBigSlots; cap > kSmallSlots && r == TN93G_ENOMEM; cap /= 2) {
+      bands.resize(2);
+      const long left = count_pairs(from, upper);
+      bands.push_back(plan_bands(from, left < 4 * band_pairs ? left + 1 : std::max(band_pairs, left / 4), cap, false, 0)[0]);
+      for (const auto &b : plan_bands(bands[2].second, left + 1, cap, false, 0)) bands.push_back(b);
+      const long rows = max_rows(bands, 2);
+      if (ctx->budget) {
+        // Room for the larger buffers, for texts, and for what a run may need later and needed with the small bands too:
+        // undecided lists of every pair, of these bands or of an exact-sums pass
+        size_t need = ctx->used + 2 * kTextPiece;
+        for (const auto &b : band_buffers(rows, plan_chunks(2))) need += b.second > b.first->n ? b.second - b.first->n : 0;
+        const long exact = max_rows(plan_bands(row_begin, band_pairs, kSmallSlots, false, 0), 0);
+        need += 4 * (size_t)std::max(rows, exact) * ncols * sizeof(unsigned long long);
+        if (need > ctx->budget) continue;
+      }
+      tried = true;
+      r = size_buffers(2, true);
+    }
+    large = r == TN93G_OK;
+    if (r == TN93G_ENOMEM) {
+      if (tried)  // what has grown makes room for the small bands' buffers again
+        for (const auto &b : band_buffers(1, 1)) release(ctx, *b.first);
+      bands = small;
+      r = size_buffers(2, false);
+    }
+    return r;
+  };
   int nb = (int)bands.size();
   for (int bi = 0; bi <= nb; bi++) {
     if (bi < nb) TRY(enqueue_compute(bi));
     if (bi >= 1) TRY(finish(bi - 1));
-    if (bi == 1 && may_grow && nb > 3 && sum->output_bytes < 2 * (size_t)band_pair_count(0)) {
+    if (bi == 1 && may_grow && nb > 3 && few(0)) {
       TRY(finish(1));
       while (pend_n) TRY(deliver_oldest());
-      const std::vector<std::pair<long, long>> small = bands;
-      bands.resize(2);
-      plan_bands(small[2].first, 1l << 62, kBigSlots, false);
-      const int grown = size_buffers(2);
-      if (grown == TN93G_ENOMEM) {
-        ctx->err.clear();
-        cudaGetLastError();
-        bands = small;
-        TRY(size_buffers(2));
-      } else {
-        TRY(grown);
-      }
+      TRY(grow_bands());
       nb = (int)bands.size();
       bi = 2;
       TRY(enqueue_compute(2));
+    } else if (large && bi >= 3 && bi + 1 < nb && !few(bi - 1)) {
+      large = false;
+      Bands next(bands.begin(), bands.begin() + bi + 1);
+      for (const auto &b : plan_bands(bands[bi].second, band_pairs, kSmallSlots, true, 99)) next.push_back(b);
+      if (max_rows(next, bi + 1) <= band) {
+        bands = next;
+        nb = (int)bands.size();
+        plan_chunks(bi + 1);
+      }
     }
   }
   while (pend_n) TRY(deliver_oldest());
