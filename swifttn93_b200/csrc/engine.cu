@@ -3660,13 +3660,16 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
       ctx->launches++;
     }
   }
-  evoff[0] = 0;
-  uint32_t max_ev = 0;
+  uint32_t max_ev = 0;  // null events add nothing to the packed sums
+  unsigned long long nev = 0;
   for (long i = 0; i < N; i++) {
-    const uint32_t n = use_ev ? pad_events(evc[i]) : 0;
-    evoff[i + 1] = evoff[i] + n;
-    max_ev = std::max(max_ev, n);
+    evoff[i] = (uint32_t)nev;
+    if (!use_ev) continue;
+    nev += pad_events(evc[i]);
+    max_ev = std::max(max_ev, evc[i]);
   }
+  if (nev >= (1ull << 32)) return TN93G_ETOOBIG;  // 32-bit offsets
+  evoff[N] = (uint32_t)nev;
   rc.packed = max_ev <= (uint32_t)kPackedMaxEvents;
   TRY(ensure(ctx, ctx->ev, std::max<size_t>(evoff[N], 1) * sizeof(uint32_t)));
   // The events again as event_kernel reads them, where the pair stage takes it (pair_split) and there is room: 8 bytes an
@@ -5102,13 +5105,14 @@ int tn93g_server_create(tn93g_ctx *ctx, tn93g_server **out, const uint8_t *codes
   std::vector<uint32_t> evc(N), evo(N + 1);
   SVC(cudaMemcpyAsync(evc.data(), srv->evcount.p, N * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   SVC(cudaStreamSynchronize(st));
-  evo[0] = 0;
   for (long i = 0; i < N; i++) {
-    evo[i + 1] = evo[i] + pad_events(evc[i]);
-    srv->ref_max_ev = std::max(srv->ref_max_ev, pad_events(evc[i]));
+    evo[i] = (uint32_t)srv->ev_ref;
+    srv->ev_ref += pad_events(evc[i]);
+    srv->ref_max_ev = std::max(srv->ref_max_ev, evc[i]);
   }
-  srv->ev_ref = evo[N];
   srv->ev_cap = srv->ev_ref + (size_t)max_batch_sequences * ((L + kEvPad - 1) / kEvPad * kEvPad);
+  if (srv->ev_cap >= (1ull << 32)) SV(TN93G_ETOOBIG);  // 32-bit offsets
+  evo[N] = (uint32_t)srv->ev_ref;
   SV(ensure(ctx, srv->ev, std::max<size_t>(srv->ev_cap, 1) * sizeof(uint32_t)));
   SVC(cudaMemcpyAsync(srv->evoff.p, evo.data(), (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
   // tables of the server's mode
@@ -5308,7 +5312,7 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
   uint32_t max_ev = srv->ref_max_ev;
   for (long k = 0; k < Q; k++) {
     evo[k + 1] = evo[k] + pad_events(evc[k]);
-    max_ev = std::max(max_ev, pad_events(evc[k]));
+    max_ev = std::max(max_ev, evc[k]);
   }
   rc.packed = max_ev <= (uint32_t)kPackedMaxEvents;
   CU(cudaMemcpyAsync((uint32_t *)srv->evoff.p + Nref, evo.data(), (Q + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice,
@@ -6041,9 +6045,9 @@ static int batch_impl(tn93g_ctx *ctx, int K, const tn93g_alignment *alns, const 
       const bool none = lin[k] && !three[k];  // no list: nothing reads one
       uint32_t max_ev = 0;
       for (long i = 0; i < alns[k].n; i++) {
-        const uint32_t n = none ? 0 : pad_events(evc[row_base[k] + i]);
+        const uint32_t n = none ? 0 : evc[row_base[k] + i];
         evo[evo_off[k] + i] = (uint32_t)nev;
-        nev += n;
+        nev += pad_events(n);
         max_ev = std::max(max_ev, n);
       }
       evo[evo_off[k] + alns[k].n] = (uint32_t)nev;
