@@ -2448,6 +2448,8 @@ struct tn93g_set {
   std::vector<long> counts, name_len;
 };
 
+constexpr int kUploadThreads = 4;  // upload_host's
+
 struct tn93g_ctx {
   int device = 0;
   size_t budget = 0, used = 0;
@@ -2477,8 +2479,8 @@ struct tn93g_ctx {
   std::string tab_key;   // what agg and site hold (run_impl; empty: nothing)
   void *hrun = nullptr;  // pinned block of a run's small transfers
   size_t hrun_n = 0;
-  void *upload_pin = nullptr;  // upload_host's pieces (two a thread) and the events of their copies
-  cudaEvent_t upload_ev[8] = {nullptr};
+  void *upload_pin = nullptr;  // upload_host's pieces (two a thread), and the events of their copies, made with the context
+  cudaEvent_t upload_ev[2 * kUploadThreads] = {nullptr};
   // device buffers of freed sets, kept for the next upload (repeated upload/free skips the allocator)
   std::vector<std::pair<void *, size_t>> set_pool;
   double timings[8] = {0};
@@ -2640,7 +2642,6 @@ struct HostSpan {
 // the link). From kUploadMin bytes on, up to kUploadThreads threads fill pinned buffers of the context instead, piece by
 // piece, and queue each piece's copy: 60 MB 3.4 -> 1.4 ms. The threads end with the call; where one cannot be started, or
 // the buffers cannot be allocated, the rest do its work.
-constexpr int kUploadThreads = 4;
 constexpr size_t kUploadPiece = 1 << 20;
 constexpr size_t kUploadMin = 4 << 20;
 
@@ -2678,8 +2679,6 @@ int upload_host(tn93g_ctx *ctx, const std::vector<HostSpan> &spans)
       ctx->upload_pin = nullptr;
       staged = false;
     }
-    for (int q = 0; staged && q < 2 * kUploadThreads; q++)
-      if (!ctx->upload_ev[q]) CU(cudaEventCreateWithFlags(&ctx->upload_ev[q], cudaEventDisableTiming));
   }
   if (!staged) {
     for (const HostSpan *h : pageable) CU(cudaMemcpyAsync(h->dst, h->src, h->n, cudaMemcpyHostToDevice, ctx->stream));
@@ -3046,6 +3045,8 @@ int tn93g_create(tn93g_ctx **out, int device, size_t hbm_budget)
       for (auto &e : ctx->evcnt[q])
         if (cudaEventCreate(&e) != cudaSuccess) rc = TN93G_ECUDA;
     }
+    for (auto &e : ctx->upload_ev)
+      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) rc = TN93G_ECUDA;
     if (cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking) != cudaSuccess) rc = TN93G_ECUDA;
     if (cudaStreamCreateWithFlags(&ctx->write_stream, cudaStreamNonBlocking) != cudaSuccess) rc = TN93G_ECUDA;
     if (const char *e = getenv("TN93G_COUNT")) ctx->count_path = strcmp(e, "popc") == 0 ? 0 : 1;
