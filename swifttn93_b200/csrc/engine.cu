@@ -2282,26 +2282,27 @@ cudaError_t launch_pair_t(const PairArgs &A, dim3 g, cudaStream_t st)
   return cudaGetLastError();
 }
 
-template <bool WPLANE, bool GAPMM, bool PACK>
+template <bool WPLANE, bool PACK>
 cudaError_t launch_event_t(const PairArgs &A, dim3 g, cudaStream_t st)
 {
   static PerDevice attr;
   const cudaError_t e = attr.once([] {
-    return cudaFuncSetAttribute(event_kernel<WPLANE, GAPMM, PACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(event_kernel<WPLANE, PACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)EvTile<WPLANE>::smem);
   });
   if (e != cudaSuccess) return e;
-  event_kernel<WPLANE, GAPMM, PACK><<<g, kEvThreads, EvTile<WPLANE>::smem, st>>>(A);
+  event_kernel<WPLANE, PACK><<<g, kEvThreads, EvTile<WPLANE>::smem, st>>>(A);
   return cudaGetLastError();
 }
 
 // Whether a pair launch takes the split form (event_kernel, then formula_kernel): with the tensor-core records, whose
 // slots hold the final aggregates, packed event sums (16-bit lanes), a code matrix that 32-bit offsets reach and, under
-// the N plane, the sequences' N words.
+// the N plane, the sequences' N words. (gapmm has weighted records, or takes the fused kernel: event_kernel does not know
+// sites where both have a gap.)
 bool pair_split(const PairArgs &A)
 {
   if (A.lin) return true;
-  return A.tcagg && A.ev2 && A.rc.packed && A.rc.Lc * A.rc.Npad < (1l << 32) && (!A.rc.wplane || A.wl_off);
+  return A.tcagg && A.ev2 && !A.rc.gapmm && A.rc.packed && A.rc.Lc * A.rc.Npad < (1l << 32) && (!A.rc.wplane || A.wl_off);
 }
 
 // Columns of a segment and rows of a warp in the formula kernel, for nrows x ncols pairs: a warp takes one segment of a few
@@ -2334,10 +2335,9 @@ cudaError_t launch_pair(const PairArgs &A, long ncolblocks, long nrows, cudaStre
     const long rows = A.rc.wplane ? EvTile<true>::rows : EvTile<false>::rows;
     const dim3 ge((unsigned)((jend - jbeg + kEvCols - 1) / kEvCols), (unsigned)((A.r1 - ibeg + rows - 1) / rows));
     const cudaError_t e = A.lin         ? cudaSuccess
-                          : A.rc.gapmm  ? launch_event_t<true, true, false>(A, ge, st)
-                          : A.rc.wplane ? launch_event_t<true, false, false>(A, ge, st)
-                          : A.tc16      ? launch_event_t<false, false, true>(A, ge, st)
-                                        : launch_event_t<false, false, false>(A, ge, st);
+                          : A.rc.wplane ? launch_event_t<true, false>(A, ge, st)
+                          : A.tc16      ? launch_event_t<false, true>(A, ge, st)
+                                        : launch_event_t<false, false>(A, ge, st);
     if (e != cudaSuccess) return e;
     const long jlo = std::max(A.cstart, A.tcncols ? A.tccolbase : A.colbase);
     int segw, rpw;
@@ -5782,16 +5782,16 @@ __global__ void gather_u64_kernel(const unsigned long long *src, const long *idx
   if (k < n) dst[k] = src[idx[k]];
 }
 
-template <bool WPLANE, bool GAPMM, bool PACK>
+template <bool WPLANE, bool PACK>
 cudaError_t launch_event_batch(const PairArgs *descs, const int4 *blocks, size_t n, cudaStream_t st)
 {
   static PerDevice attr;
   const cudaError_t e = attr.once([] {
-    return cudaFuncSetAttribute(event_batch_kernel<WPLANE, GAPMM, PACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(event_batch_kernel<WPLANE, PACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)EvTile<WPLANE>::smem);
   });
   if (e != cudaSuccess) return e;
-  event_batch_kernel<WPLANE, GAPMM, PACK><<<(unsigned)n, kEvThreads, EvTile<WPLANE>::smem, st>>>(descs, blocks);
+  event_batch_kernel<WPLANE, PACK><<<(unsigned)n, kEvThreads, EvTile<WPLANE>::smem, st>>>(descs, blocks);
   return cudaGetLastError();
 }
 
@@ -6374,8 +6374,8 @@ static int batch_impl(tn93g_ctx *ctx, int K, const tn93g_alignment *alns, const 
       const int4 *bl = (const int4 *)bb[BB_SPLIT].p + sb_at[c];
       const size_t n = sb_at[c + 1] - sb_at[c];
       if (!n) continue;
-      if (c == 0) CU((launch_event_batch<false, false, true>(dp, bl, n, st)));
-      if (c == 1) CU((launch_event_batch<false, false, false>(dp, bl, n, st)));
+      if (c == 0) CU((launch_event_batch<false, true>(dp, bl, n, st)));
+      if (c == 1) CU((launch_event_batch<false, false>(dp, bl, n, st)));
       if (c == 2) formula_batch_kernel<true, false><<<(unsigned)n, 256, 0, st>>>(dp, bl);
       if (c == 3) formula_batch_kernel<false, false><<<(unsigned)n, 256, 0, st>>>(dp, bl);
       if (c == 4) formula_batch_kernel<true, true><<<(unsigned)n, 256, 0, st>>>(dp, bl);

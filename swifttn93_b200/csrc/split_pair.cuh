@@ -6,8 +6,10 @@
 // One fused kernel (pair_kernel) holds the formula's registers through the event loads, whose latency then shows: it took
 // 1,920 instructions per 32 pairs (a third more for the certificate, which ran for one ambiguous lane in six) and issued
 // half of the time. Pair stage without the count kernel, per 22.4 M pairs of the 6,700 x 1,500 benchmark set: fused
-// 2.10 ms, split 1.36 ms under resolve; under gapmm 2.77 -> 2.16 ms; serving 38 M pairs, counts included, 6.2 -> 5.0 ms.
-// The fused kernel stays for the popcount path, sequences with more than 1,023 events and batches of alignments.
+// 2.10 ms, split 1.36 ms under resolve; serving 38 M pairs, counts included, 6.2 -> 5.0 ms.
+// The fused kernel stays for the popcount path, for sequences with more than 1,023 events, for the N plane where its words
+// are not listed (batches and servers), and where there is no room for the event offsets (pair_split).
+// Under average, gapmm and skip the records hold whole pairs and formula_kernel runs alone.
 //
 // Included by engine.cu inside its unnamed namespace.
 
@@ -202,7 +204,7 @@ __device__ __forceinline__ int next_item(int *counter)
 __device__ __forceinline__ int ev_slot(int x) { return (x & 1) * 32 + (x >> 1); }
 
 // tile (bx, by) of the columns from a.cstart and the rows from a.r0, by all threads of the block
-template <bool WPLANE, bool GAPMM, bool PACK>
+template <bool WPLANE, bool PACK>
 __device__ __forceinline__ void event_tile(const PairArgs &a, int bx, int by)
 {
   using T = EvTile<WPLANE>;
@@ -365,7 +367,7 @@ __device__ __forceinline__ void event_tile(const PairArgs &a, int bx, int by)
       if (WPLANE && valid) {
         // the row's N words against the column's clean bases and N sites, plus the column's share
         const uint32_t q0 = a.wl_off[i], q1 = a.wl_off[i + 1];
-        int nWW = 0, nGG = 0;
+        int nWW = 0;
         for (uint32_t q = q0; q < q1; q++) {
           const uint64_t *Pw = a.planes + (size_t)__ldg(a.wl + q) * rc.NP * Np;
           const uint64_t ni = __ldg(Pw + 3 * (size_t)Np + i);
@@ -375,13 +377,12 @@ __device__ __forceinline__ void event_tile(const PairArgs &a, int bx, int by)
           wc[h].l += popc(ni & lj);
           wc[h].t += popc(ni & hj & lj);
           nWW += popc(ni & __ldg(Pw + 3 * (size_t)Np + j));
-          if (GAPMM) nGG += popc(__ldg(Pw + 4 * (size_t)Np + i) & __ldg(Pw + 4 * (size_t)Np + j));
         }
         wb[3] = wc[h].t;
         wb[1] = wc[h].h - wc[h].t;
         wb[2] = wc[h].l - wc[h].t;
         wb[0] = wc[h].c - wb[1] - wb[2] - wb[3];
-        wb[4] = nWW - nGG;
+        wb[4] = nWW;
 #pragma unroll
         for (int b = 0; b < 5; b++) {
 #pragma unroll
@@ -466,10 +467,10 @@ __device__ __forceinline__ void event_tile(const PairArgs &a, int bx, int by)
   }
 }
 
-template <bool WPLANE, bool GAPMM, bool PACK>
+template <bool WPLANE, bool PACK>
 __global__ void __launch_bounds__(kEvThreads, 2) event_kernel(PairArgs a)
 {
-  event_tile<WPLANE, GAPMM, PACK>(a, blockIdx.x, blockIdx.y);
+  event_tile<WPLANE, PACK>(a, blockIdx.x, blockIdx.y);
 }
 
 // A batch of alignments: each block's (descriptor, bx, by, z). A descriptor's copy in shared memory, for all threads.
@@ -482,11 +483,11 @@ __device__ __forceinline__ const PairArgs &batch_args(const PairArgs *descs, int
   return *reinterpret_cast<const PairArgs *>(raw);
 }
 
-template <bool WPLANE, bool GAPMM, bool PACK>
+template <bool WPLANE, bool PACK>
 __global__ void __launch_bounds__(kEvThreads, 2) event_batch_kernel(const PairArgs *descs, const int4 *blocks)
 {
   const int4 b = blocks[blockIdx.x];
-  event_tile<WPLANE, GAPMM, PACK>(batch_args(descs, b.x), b.y, b.z);
+  event_tile<WPLANE, PACK>(batch_args(descs, b.x), b.y, b.z);
 }
 
 // Whether pair (i, j) has a contribution that is not a multiple of 1/16 in a run whose records hold everything else: the
