@@ -2312,18 +2312,18 @@ bool pair_split(const PairArgs &A)
 // SMs have two waves of warps (1,801 x 1,203 in bands of 0.2-0.4 M pairs: 0.10 -> 0.05 ms a band), and rows are added up
 // only past four waves, strips past one (a strip's row has few pairs, and its warp four atomics on its query's words: 32
 // columns x 30,000 rows 109 us with a row to a warp, 59 us with 8).
-void formula_shape(long nrows, long ncols, bool units, int &segw, int &rpw)
+void formula_shape(long nrows, long ncols, bool units, int sms, int &segw, int &rpw)
 {
   segw = units ? 32 : kSeg;
-  while (segw > 128 && nrows * ((ncols + segw - 1) / segw) < 148 * 48) segw /= 2;
+  while (segw > 128 && nrows * ((ncols + segw - 1) / segw) < sms * 48l) segw /= 2;
   const long nseg = (ncols + segw - 1) / segw;
-  rpw = (int)std::max<long>(1, std::min<long>(1024 / std::min<long>(segw, ncols), nrows * nseg / (148 * (units ? 24 : 128))));
+  rpw = (int)std::max<long>(1, std::min<long>(1024 / std::min<long>(segw, ncols), nrows * nseg / (sms * (units ? 24l : 128l))));
 }
 
 // The pair stage of rows [A.r0, A.r1) and the columns from A.cstart (32 ncolblocks of them). Fused kernel: 4 resident
 // blocks per SM (64 registers a thread) with the tensor-core counts and no N plane, 3 (80) with it, 2 with the popcount
 // loop, which needs the registers. TN93G_PAIR_BLOCKS=2|3|4 overrides.
-cudaError_t launch_pair(const PairArgs &A, long ncolblocks, long nrows, cudaStream_t st)
+cudaError_t launch_pair(const PairArgs &A, long ncolblocks, long nrows, int sms, cudaStream_t st)
 {
   static const int forced = [] {
     const char *e = getenv("TN93G_PAIR_BLOCKS");
@@ -2341,7 +2341,7 @@ cudaError_t launch_pair(const PairArgs &A, long ncolblocks, long nrows, cudaStre
     if (e != cudaSuccess) return e;
     const long jlo = std::max(A.cstart, A.tcncols ? A.tccolbase : A.colbase);
     int segw, rpw;
-    formula_shape(nrows, jend - jlo, A.ex.colunit != nullptr, segw, rpw);
+    formula_shape(nrows, jend - jlo, A.ex.colunit != nullptr, sms, segw, rpw);
     const long nseg = (jend - jlo + segw - 1) / segw;
     const dim3 gf((unsigned)((nrows + kWarps * rpw - 1) / (kWarps * rpw)), (unsigned)nseg);
     if (A.lin) {
@@ -4059,14 +4059,14 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
         const long cb0 = (ccs - colbase) / 32, cbs = (ncols + 31) / 32 - cb0;
         if (cbs > 0) {
           AC.cstart = colbase + cb0 * 32;
-          CU(launch_pair(AC, cbs, c1 - c0, st));
+          CU(launch_pair(AC, cbs, c1 - c0, ctx->sms, st));
           ctx->launches += pair_split(AC) && !AC.lin ? 2 : 1;
         }
       }
       nchunks[par] = (int)chunks.size();
     } else if (cblks > 0) {
       A.cstart = colbase + cblk0 * 32;
-      CU(launch_pair(A, cblks, nr, st));
+      CU(launch_pair(A, cblks, nr, ctx->sms, st));
       ctx->launches++;
       nchunks[par] = 0;
     } else {
@@ -4686,7 +4686,7 @@ int noalloc_run(const uint8_t *d_codes, long N, long L, const tn93g_opts *opts, 
   A.counters = counters;
   A.logt = (const LogTable *)(S + kNaLog);
   memset(&A.ex, 0, sizeof A.ex);  // raw distances only: no undecided list, no summary bounds
-  NA(launch_pair(A, (N + 31) / 32, N, st));
+  NA(launch_pair(A, (N + 31) / 32, N, 0 /* the fused kernel's grid does not use it */, st));
   unsigned nq = 0;
   NA(cudaMemcpyAsync(&nq, rqn, sizeof nq, cudaMemcpyDeviceToHost, st));
   NA(cudaStreamSynchronize(st));
@@ -5425,11 +5425,11 @@ int tn93g_server_batch(tn93g_server *srv, int nq, const tn93g_alignment *queries
         AC.tccolbase = c0;
         AC.cstart = c0;
         AC.cend = c1;  // the records past it are the next chunk's, not counted yet
-        CU(launch_pair(AC, (c1 - c0 + 31) / 32, Nref, st));
+        CU(launch_pair(AC, (c1 - c0 + 31) / 32, Nref, ctx->sms, st));
         ctx->launches += pair_split(AC) && !AC.lin ? 3 : 2;
       }
     } else {
-      CU(launch_pair(A, (Q + 31) / 32, Nref, st));
+      CU(launch_pair(A, (Q + 31) / 32, Nref, ctx->sms, st));
       ctx->launches++;
     }
     CU(cudaEventRecord(E[2], st));
@@ -6358,7 +6358,7 @@ static int batch_impl(tn93g_ctx *ctx, int K, const tn93g_alignment *alns, const 
             sb.push_back(make_int4(k, (int)(j0 / kEvCols), (int)(i0 / rows), 0));
       } else if (w16 == (c % 2 == 0) && (bool)lin[k] == (c >= 4)) {
         int segw, rpw;
-        formula_shape(N, N, false, segw, rpw);
+        formula_shape(N, N, false, ctx->sms, segw, rpw);
         for (long by = 0; by * segw < N - 1; by++)  // the segments of a row start at its first column
           for (long bx = 0; bx * kWarps * rpw < N - 1 - by * segw; bx++)
             sb.push_back(make_int4(k, (int)bx, (int)by, rpw << 11 | segw));
@@ -6386,7 +6386,7 @@ static int batch_impl(tn93g_ctx *ctx, int K, const tn93g_alignment *alns, const 
   }
   for (int k = 0; k < K; k++)
     if (!RC[k].W && alns[k].n > 1) {
-      CU(launch_pair(PD[k], (alns[k].n + kTile - 1) / kTile, alns[k].n, st));
+      CU(launch_pair(PD[k], (alns[k].n + kTile - 1) / kTile, alns[k].n, ctx->sms, st));
       ctx->launches++;
     }
   ctx->records_busy = false;  // what is launched from here on reads neither the records nor the offsets
