@@ -46,14 +46,17 @@ WORKLOAD = "hiv_bench 6700x1500, -t 1000 -g 0.05 -l 500 -f csv, -a resolve/avera
 
 
 # ncu figures of the pair stage behind the roofline line, 4,000-sequence prefix under -a resolve (one 16 M-pair chunk
-# holds all 7,998,000 pairs): DRAM bytes of its count_tc_persist_kernel + pair_kernel launches with the caches kept
-# between kernels (profiles/pair_stage_traffic_hiv_bench_n4000.md), the count kernel's tensor-pipe activity
-# (profiles/count_tc_kernel_hiv_bench_n4000.md) and the pair kernel's instructions and issue activity
-# (profiles/pair_kernel_hiv_bench_n4000.md)
-PAIR_STAGE_PROFILE = {"pairs": 7998000, "dram_bytes": 400.36e6, "tensor_pipe_active": 0.417,
-                      "pair_kernel_inst_per_pair": 467694944 * 32 / 7998000, "pair_kernel_issue_active": 0.555,
+# holds all 7,998,000 pairs): DRAM bytes of its count_tc_persist_kernel, event_kernel and formula_kernel launches with the
+# caches kept between kernels (profiles/pair_stage_traffic_hiv_bench_n4000.md), the count kernel's tensor-pipe activity
+# (profiles/count_tc_kernel_hiv_bench_n4000.md), and the other two's warp instructions per 32 pairs, issue activity and
+# FP64 pipe activity (profiles/event_formula_kernels_hiv_bench_n4000.md)
+PAIR_STAGE_PROFILE = {"pairs": 7998000, "dram_bytes": 517.91e6, "tensor_pipe_active": 0.528,
+                      "event_kernel": {"instructions_per_pair": 123696963 * 32 / 7998000, "issue_active": 0.593},
+                      "formula_kernel": {"instructions_per_pair": 201801758 * 32 / 7998000, "issue_active": 0.653,
+                                         "fp64_pipe_active": 0.531},
                       "files": ["profiles/pair_stage_traffic_hiv_bench_n4000.md",
-                                "profiles/count_tc_kernel_hiv_bench_n4000.md", "profiles/pair_kernel_hiv_bench_n4000.md"]}
+                                "profiles/count_tc_kernel_hiv_bench_n4000.md",
+                                "profiles/event_formula_kernels_hiv_bench_n4000.md"]}
 
 
 def peaks():
@@ -567,11 +570,11 @@ def main():
             d2h = nbytes
     e2e = pairs_step * ws / (float(np.mean(e2e_ms)) / 1e3) if e2e_ms else None
 
-    # ---- roofline of the dominant stage: the pair stage (count_tc_persist_kernel + pair_kernel)
+    # ---- roofline of the dominant stage: the pair stage (count_tc_persist_kernel, event_kernel, formula_kernel)
     # Algorithmic work (the clean-site count contraction): 16 x Lc INT8 one-hot MACs per pair, 25 x Lc when the
     # N/gap plane is active (gapmm here), 2 ops per MAC, against dense INT8 = 2 x the bf16 tensor peak. The count
-    # kernel is reported alone against the same peak on its 16 x Lc; the pair kernel (CUDA cores: sparse events,
-    # formula, certificate) is issue-bound and reported with its instructions per pair from the profile.
+    # kernel is reported alone against the same peak on its 16 x Lc; the other two (CUDA cores: sparse events; formula and
+    # certificate) saturate no pipe and are reported with their time together and the profile's figures.
     P = peaks()
     pairs_run = n * (n - 1) // 2
     per_mode = stage_by_mode
@@ -582,13 +585,13 @@ def main():
     peak_tc = 2 * P["bf16"]
     tc_work = sum(pairs_run * 16 * Lc * 2 for _ in MODES)
     tc_ms = sum(count_ms.values())
-    # DRAM bytes of one pair-stage launch (count_tc_persist_kernel + pair_kernel) from the ncu capture named below,
+    # DRAM bytes of one pair stage (its three kernels under -a resolve) from the ncu capture named below,
     # scaled by pairs; algorithmic bytes: the raw distance written once (8 B per pair) and the operands read once
     # (one-hot image 4 Lc B, bit planes 4 x 8 B per 64 columns, codes and transposed codes 2 Lc B per sequence)
     prof_pairs, prof_bytes = PAIR_STAGE_PROFILE["pairs"], PAIR_STAGE_PROFILE["dram_bytes"]
     traffic = prof_bytes * pairs_run / prof_pairs
     alg_bytes = 8 * pairs_run + n * (4 * Lc + 4 * 8 * ((Lc + 63) // 64) + 2 * Lc)
-    roof = {"kernel": "pair stage: count_tc_persist_kernel + pair_kernel", "bound": "tensor", "achieved": achieved,
+    roof = {"kernel": "pair stage: count_tc_persist_kernel + event_kernel + formula_kernel", "bound": "tensor", "achieved": achieved,
             "peak": peak_tc, "unit": "TFLOP/s", "frac": achieved / peak_tc, "traffic": traffic,
             "traffic_over_algorithmic": traffic / alg_bytes,
             "peak_note": f"dense INT8 ops = 2 x {P['src']} bf16 ({P['bf16']} TF/s)",
@@ -599,9 +602,9 @@ def main():
                                 "frac": (tc_work / (tc_ms / 1e3) / 1e12) / peak_tc if tc_ms else None,
                                 "ms_per_launch": {m: count_ms[m] for m in MODES},
                                 "tensor_pipe_active": PAIR_STAGE_PROFILE["tensor_pipe_active"]},
-            "pair_kernel": {"ms_per_launch": {m: pair_ms[m] - count_ms[m] for m in MODES}, "bound": "issue",
-                            "instructions_per_pair": PAIR_STAGE_PROFILE["pair_kernel_inst_per_pair"],
-                            "issue_active": PAIR_STAGE_PROFILE["pair_kernel_issue_active"]},
+            "event_and_formula_kernels": {"ms_per_pair_stage": {m: pair_ms[m] - count_ms[m] for m in MODES},
+                                          "bound": "latency", "event_kernel": PAIR_STAGE_PROFILE["event_kernel"],
+                                          "formula_kernel": PAIR_STAGE_PROFILE["formula_kernel"]},
             "profile": PAIR_STAGE_PROFILE["files"]}
 
     line = {"metric": METRIC, "value": value, "unit": "pairs/s", "n_gpus": ws, "steps": args.steps,

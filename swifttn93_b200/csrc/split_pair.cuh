@@ -1,10 +1,10 @@
 // split_pair.cuh -- the pair stage behind the tensor-core counts, as two kernels over the pairs' records:
 //   event_kernel    adds the sparse ambiguity events (and N-plane cross terms) to each pair's clean-site record and takes
-//                   tn93's -l, -g and site-order decisions; integers, about 490 instructions per 32 pairs;
-//   formula_kernel  the FP64 formula, its logarithms and the certificate; about 800 instructions per 32 pairs, 330 of
-//                   them FP64 (the FP64 pipe alone needs 0.4 ms per 22.4 M pairs).
+//                   tn93's -l, -g and site-order decisions; integers, 495 instructions per 32 pairs;
+//   formula_kernel  the FP64 formula, its logarithms and the certificate; 807 instructions per 32 pairs, the FP64 pipe
+//                   busy for half of its time (0.47 ms per 22.4 M pairs).
 // One fused kernel (pair_kernel) holds the formula's registers through the event loads, whose latency then shows: it took
-// 1,920 instructions per 32 pairs (a third more for the certificate, which ran for one ambiguous lane in six) and issued
+// 1,871 instructions per 32 pairs (a third more for the certificate, which ran for one ambiguous lane in six) and issued
 // half of the time. Pair stage without the count kernel, per 22.4 M pairs of the 6,700 x 1,500 benchmark set: fused
 // 2.10 ms, split 1.36 ms under resolve; serving 38 M pairs, counts included, 6.2 -> 5.0 ms.
 // The fused kernel stays for the popcount path, for sequences with more than 1,023 events, for the N plane where its words
