@@ -2535,6 +2535,7 @@ void server_reclaim(tn93g_server *srv);
 bool reclaim(tn93g_ctx *ctx)
 {
   const size_t before = ctx->used;
+  for (cudaStream_t s : {ctx->stream, ctx->write_stream, ctx->copy_stream}) cudaStreamSynchronize(s);
   release(ctx, ctx->ev2);
   if (!ctx->records_busy) {
     release(ctx, ctx->bb[BB_EV2]);
@@ -3145,6 +3146,7 @@ static int upload_set(tn93g_ctx *ctx, tn93g_set **out, const uint8_t *codes, cud
   std::vector<int32_t> nl(N);
   for (long i = 0; i < N; i++) nl[i] = (int32_t)name_len[i];
   auto fail = [&](cudaError_t e) {
+    cudaGetLastError();
     ctx->err = cudaGetErrorString(e);
     tn93g_free_set(ctx, s);
     return e == cudaErrorMemoryAllocation ? TN93G_ENOMEM : TN93G_ECUDA;
