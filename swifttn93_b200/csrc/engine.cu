@@ -4366,13 +4366,15 @@ static int run_impl(tn93g_ctx *ctx, const tn93g_set *set, long n1, const tn93g_o
       TRY(enqueue_compute(2));
     } else if (large && bi >= 3 && bi + 1 < nb && !few(bi - 1)) {
       large = false;
-      Bands next(bands.begin(), bands.begin() + bi + 1);
-      for (const auto &b : plan_bands(bands[bi].second, band_pairs, kSmallSlots, true, 99)) next.push_back(b);
-      if (max_rows(next, bi + 1) <= band) {
-        bands = next;
-        nb = (int)bands.size();
+      const Bands was = bands;
+      bands.resize(bi + 1);
+      for (const auto &b : plan_bands(was[bi].second, band_pairs, kSmallSlots, true, 99)) bands.push_back(b);
+      const size_t records = plan_chunks(bi + 1) * (tc16 ? 16 : 32);
+      if (max_rows(bands, bi + 1) > band || (use_tc && records > ctx->tcagg.n)) {  // (they fit the larger bands' buffers)
+        bands = was;
         plan_chunks(bi + 1);
       }
+      nb = (int)bands.size();
     }
   }
   while (pend_n) TRY(deliver_oldest());
